@@ -76,13 +76,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait on phase `parity`.  Returns false (and records `code`) when
 // the time limit passes or another thread already recorded an error.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  uint64_t t0 = globaltimer();
-  for (uint32_t i = 1;; ++i) {
+  uint64_t t0 = 0;  // the timer is read only once the wait is long
+  for (uint32_t i = 0;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 63u) == 0) {
+    if ((i & 63u) == 63u) {
       if (dev_error_set()) return false;
-      if (globaltimer() - t0 > kWaitLimitNs) {
+      if (t0 == 0) {
+        t0 = globaltimer();
+      } else if (globaltimer() - t0 > kWaitLimitNs) {
         dev_error(code);
         return false;
       }
