@@ -46,8 +46,6 @@ struct Consts {
   int nmod;
   int H;                       // scaled operands stay below 2^H in 2-norm
   int p[kMaxMod];
-  float invp_f[kMaxMod];
-  double invp_d[kMaxMod];
   uint32_t wlo[kMaxMod], whi[kMaxMod];  // bytes of 2^(8t) mod p, t = 0..3, 4..7
   uint32_t off[kMaxMod];                // p - (2^62 mod p): undoes the +2^62 offset
   uint32_t offh[kMaxMod];               // off + floor(p/2): symmetric residues
@@ -57,6 +55,7 @@ struct Consts {
   // bits of w from 2^csplit up (exact double, <= 41 significant bits), w2
   // the rest rounded to double; P = P1 + P2 the same way
   double w1[kMaxMod], w2[kMaxMod];
+  double s1, s2;  // -4096 sum w1, -4096 sum w2: where the sums over 4096 + r start
   double P1d, P2d, Pd, invPd;
 };
 
@@ -129,17 +128,15 @@ static bool make_consts(int n, Consts* c) {
   for (int i = 0; i < n; ++i) P *= (u128)m[i];
   // budget: ||A'_i||_2 ||B'_j||_2 <= 2^(2H) (1+tiny) < P/2
   c->H = (int)std::floor((log2P(n) - 1.0) / 2.0) - 1;
-  // split point of the CRT weights: sum_l r_l w1_l < 4080 P < 2^(bits(P)+12)
-  // must be an integer multiple of 2^csplit below 2^(53+csplit)
+  // split point of the CRT weights: sum_l (4096 + r_l) w1_l < 16 * 4352 P <
+  // 2^(bits(P)+17) must be an integer multiple of 2^csplit below 2^(53+csplit)
   int bitsP = 0;
   for (u128 t = P; t; t >>= 1) ++bitsP;
-  const int csplit = std::max(0, bitsP + 12 - 53);
+  const int csplit = std::max(0, bitsP + 17 - 53);
   const u128 low = csplit ? (((u128)1 << csplit) - 1) : 0;
   for (int i = 0; i < n; ++i) {
     const int p = m[i];
     c->p[i] = p;
-    c->invp_f[i] = std::nextafter(1.0f / (float)p, 0.0f);  // <= 1/p (see k_oz_residues)
-    c->invp_d[i] = 1.0 / (double)p;
     uint32_t lo = 0, hi = 0;
     for (int t = 0; t < 8; ++t) {
       uint64_t w = 1;
@@ -158,8 +155,10 @@ static bool make_consts(int n, Consts* c) {
     const u128 Mi = P / (u128)p;
     const int inv = inv_mod((int)(Mi % (u128)p), p);
     const u128 w = mulmod(Mi, (u128)inv, P);
-    c->w1[i] = std::ldexp((double)(uint64_t)(w >> csplit), csplit);  // < 2^41 units: exact
+    c->w1[i] = std::ldexp((double)(uint64_t)(w >> csplit), csplit);  // < 2^36 units: exact
     c->w2[i] = (double)(w & low);
+    c->s1 -= 4096.0 * c->w1[i];  // exact: multiples of 2^csplit below 2^(53+csplit)
+    c->s2 -= 4096.0 * c->w2[i];
   }
   c->P1d = std::ldexp((double)(uint64_t)(P >> csplit), csplit);
   c->P2d = (double)(P & low);
@@ -466,7 +465,7 @@ struct GemmP {
   int uplo;
   long diag;
   int p[kMaxMod];
-  double invp[kMaxMod];
+  uint32_t bias[kMaxMod], magic[kMaxMod];  // of the epilogue's mod p
 };
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
@@ -525,6 +524,64 @@ __device__ __forceinline__ bool oz_tile(const GemmP& p, int t, int& mod, int& m0
   if (p.uplo == XKB_LOWER && (long)(m0 + BM - 1) + p.diag < (long)n0) return false;
   if (p.uplo == XKB_UPPER && (long)m0 + p.diag > (long)(n0 + BN - 1)) return false;
   return true;
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+      "%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Epilogue of one warp: its 32 TMEM lanes (rows) x 256 columns of an
+// accumulator -> mod p -> uint8 plane R[column / 16][row][column % 16] (blocks
+// of 16 columns: a lane's 16 bytes lie beside its neighbours', here and when
+// the CRT reads them), 32 columns per lane at a time; drained() is called
+// once every column is in registers.  The residue by integers: u = acc + bias is non-negative (bias:
+// the multiple of p from 2^31 on; |acc| < 2^31 - 2^24 for p < 256, and for
+// p = 256 wrapping is exact), q = umulhi(u, ceil(2^32 / p)) is floor(u / p)
+// or one more, so r = u - q p or that plus p.  (By FP64 -- two conversions
+// and a floor per element, a byte store per element -- the epilogue took
+// longer than the MMAs below K of about 1500.)
+template <class F>
+__device__ __forceinline__ void oz_epilogue(const GemmP& p, int mod, int row, int n0,
+                                            uint32_t tbase, F drained) {
+  const uint32_t pm = (uint32_t)p.p[mod], bias = p.bias[mod], magic = p.magic[mod];
+  uint8_t* dst = p.R + (size_t)mod * (size_t)p.Mpad * (size_t)p.Npad +
+                 (size_t)n0 * (size_t)p.Mpad + (size_t)row * 16;
+  const size_t blk = (size_t)p.Mpad * 16;  // bytes of a block of 16 columns
+#pragma unroll 1
+  for (int c = 0; c < 256 / 32; ++c) {
+    uint32_t v[32];
+    tmem_ld32(v, tbase + (uint32_t)(c * 32));
+    if (c == 256 / 32 - 1) {
+      tc_fence_before();
+      __syncwarp();
+      drained();
+    }
+    uint32_t w[8];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) {
+      const uint32_t u = v[e] + bias;
+      const uint32_t r = u - __umulhi(u, magic) * pm;
+      v[e] = min(r, r + pm);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      w[e] = __byte_perm(__byte_perm(v[4 * e], v[4 * e + 1], 0x0040),
+                         __byte_perm(v[4 * e + 2], v[4 * e + 3], 0x0040), 0x5410);
+    // streaming stores: the planes are read once, by the CRT kernel; they
+    // should not evict the operand panels from L2
+    __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0], w[1], w[2], w[3]));
+    __stcs(reinterpret_cast<uint4*>(dst + blk), make_uint4(w[4], w[5], w[6], w[7]));
+    dst += 2 * blk;
+  }
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -638,38 +695,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN);
-      const int pm = p.p[mod];
-      const double ip = p.invp[mod];
-      uint8_t* plane = p.R + (size_t)mod * (size_t)p.Mpad * (size_t)p.Npad;
-      for (int c = 0; c < BN / 16; ++c) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-            "%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-              "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tbase + (uint32_t)(c * 16)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c == BN / 16 - 1) {
-          // every column of buffer b is in registers: hand it back to the MMA warp
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acce[b]);
-        }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int acc = (int)v[e];
-          const int qq = (int)floor((double)acc * ip);
-          int r = acc - qq * pm;
-          if (r < 0) r += pm;
-          else if (r >= pm) r -= pm;
-          const size_t col = (size_t)(n0 + c * 16 + e);
-          // streaming store: the residue planes are read once, by the CRT
-          // kernel; they should not evict the operand panels from L2
-          __stcs(plane + col * (size_t)p.Mpad + (size_t)row, (unsigned char)r);
-        }
-      }
+      oz_epilogue(p, mod, row, n0, tbase, [&] {
+        if (lane == 0) mbar_arrive(&acce[b]);
+      });
       ++tl;
     }
   }
@@ -716,12 +744,6 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(
-                   cluster_addr),
-               "r"(bytes)
                : "memory");
 }
 __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m, int x, int y,
@@ -788,7 +810,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S2; ++s) {
-      mbar_init(&full[s], 2);  // one arrive.expect_tx per CTA of the pair
+      mbar_init(&full[s], 1);  // the even CTA expects the bytes of both CTAs' loads
       mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -827,9 +849,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             ok = false;
             break;
           }
-          // the even CTA's stage barrier: arrive through its cluster address,
-          // the pair-form TMA names it with the peer bit cleared
-          mbar_expect_tx_cluster(mapa_rank(smem_u32(&full[s]), 0), 2 * H_STAGE);
+          // the even CTA's stage barrier (the pair-form TMA names it with the
+          // peer bit cleared) counts the four halves.  The odd CTA signals it
+          // by its bytes only: a remote arrive per stage held its producer
+          // back for longer than the stage's MMAs
+          if (rank == 0) mbar_expect_tx(&full[s], 4 * H_STAGE);
           const uint32_t fe = smem_u32(&full[s]) & kPeerMask;
           tma_load_3d_pair(sA + s * H_STAGE, &tA, kb * BKB, m0 + 128 * (int)rank, mod, fe);
           tma_load_3d_pair(sB + s * H_STAGE, &tB, kb * BKB, n0 + 128 * (int)rank, mod, fe);
@@ -885,36 +909,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tc_fence_after();
       const int row = m0 + 128 * (int)rank + q * 32 + lane;
       const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN2);
-      const int pm = p.p[mod];
-      const double ip = p.invp[mod];
-      uint8_t* plane = p.R + (size_t)mod * (size_t)p.Mpad * (size_t)p.Npad;
-      for (int c = 0; c < BN2 / 16; ++c) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-            "%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-              "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tbase + (uint32_t)(c * 16)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c == BN2 / 16 - 1) {
-          // every column of buffer b is in registers: release it to the even CTA
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(b ? ae1 : ae0);
-        }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int acc = (int)v[e];
-          const int qq = (int)floor((double)acc * ip);
-          int r = acc - qq * pm;
-          if (r < 0) r += pm;
-          else if (r >= pm) r -= pm;
-          const size_t col = (size_t)(n0 + c * 16 + e);
-          __stcs(plane + col * (size_t)p.Mpad + (size_t)row, (unsigned char)r);
-        }
-      }
+      oz_epilogue(p, mod, row, n0, tbase, [&] {
+        if (lane == 0) mbar_arrive_cluster(b ? ae1 : ae0);
+      });
       ++tl;
     }
   }
@@ -931,7 +928,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 }
 
 // ---------------------------------------------------------------------------
-// 4. CRT reconstruction + scaling + alpha/beta, 4 consecutive rows per thread.
+// 4. CRT reconstruction + scaling + alpha/beta, 16 columns of one row per thread.
 struct CrtP {
   int M, N;
   const uint8_t* R;
@@ -950,31 +947,22 @@ struct CrtP {
 
 // Recombination on the FP64 pipe.  S = sum_l r_l w_l < 4080 P; the shifts
 // keep |C'| <= P/8, so the wanted value is S - qP with q = round(S / P).
-// With w = w1 + w2 (w1: multiples of 2^csplit, <= 41 significant bits):
-//  - S1 = sum r_l w1_l is exact (8-bit x 41-bit products, multiples of
-//    2^csplit, sum below 2^(53+csplit));
-//  - q = rint(S1 / P) is exact: S2 / P < 2^-28 and S / P lies within 1/8 of
+// r_l enters as the double 4096 + r_l, one byte permutation (an int -> double
+// conversion per residue would take longer than the sums), and the sums start
+// at -4096 sum_l w_l.
+// With w = w1 + w2 (w1: multiples of 2^csplit, <= 36 significant bits):
+//  - S1 = sum r_l w1_l is exact (13-bit x 36-bit products, multiples of
+//    2^csplit, every partial sum below 2^(53+csplit));
+//  - q = rint(S1 / P) is exact: S2 / P < 2^-23 and S / P lies within 1/8 of
 //    an integer (q < 2^12);
-//  - S1 - q P1 is exact (a 53-bit product, the difference a multiple of
-//    2^csplit below 2^(42+csplit));
-//  - S2 - q P2 carries absolute errors of order 2^(csplit-37) plus the
-//    rounding of w2 (2^43 at 16 moduli), far below the 2^(2H-61) sqrt(K)
+//  - S1 - q P1 is exact (a 48-bit product, the difference a multiple of
+//    2^csplit below 2^(38+csplit));
+//  - S2 - q P2 carries absolute errors of order 2^(csplit-36) (2^54 at 16
+//    moduli), 2^-67 of the largest result and far below the 2^(2H-61) sqrt(K)
 //    already left by rounding the scaled operands to integers.
 // 2 FP64 FMAs per modulus and element (a 128-bit integer sum would take 4
-// 64-bit integer multiply-adds): the kernel runs on the FP64 pipe, which
-// nothing else here uses.
-template <int NM>
-__device__ __forceinline__ double crt_value(const uint32_t (&r)[NM], const Consts& c) {
-  double s1 = 0.0, s2 = 0.0;
-#pragma unroll
-  for (int m = 0; m < NM; ++m) {
-    const double rv = (double)r[m];
-    s1 = fma(rv, c.w1[m], s1);
-    s2 = fma(rv, c.w2[m], s2);
-  }
-  const double q = rint(s1 * c.invPd);
-  return fma(-q, c.P1d, s1) + fma(-q, c.P2d, s2);
-}
+// 64-bit integer multiply-adds).  The weights are constant loads, not operands
+// of an FP64 FMA, so each is used for eight elements at once.
 
 // x * 2^e for the shift range used here (|e| <= 2000), exact unless the
 // result under/overflows
@@ -988,75 +976,102 @@ __device__ __forceinline__ double scale2(double x, int e) {
   return x * pow2(e1) * pow2(e2);
 }
 
-// The four rows of a thread are reconstructed unconditionally (rows past M
-// reuse the last row's shift and are not stored), so their independent
-// integer chains interleave; the stores are predicated afterwards.
-template <int NM>
-__device__ __forceinline__ void crt_quad(const CrtP& p, const Consts& c, int H, long i0, int j,
-                                         double (&y)[4]) {
+// A warp takes 16 rows x 16 columns: lane l row l / 2 and columns 8 (l % 2)
+// .. + 7, so that each plane is read 256 contiguous bytes at a time and C's
+// columns 128.
+constexpr int kCrtRows = 16, kCrtCols = 16 * 8;  // of a block of eight warps
+
+// The eight columns j0 + e of this thread: pre(i, j, e) for each (the loads of
+// what f combines, issued together and before any store), then
+// f(i, j, e, value); columns outside C or the triangle mask are left out.
+template <int NM, class G, class F>
+__device__ __forceinline__ void crt_cols(const CrtP& p, const Consts& c, int H, G pre, F f) {
   const size_t plane = (size_t)p.Mpad * (size_t)p.Npad;
-  uint32_t words[NM];
+  const int lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * kCrtRows, i = i0 + (lane >> 1);
+  const int jw = blockIdx.y * kCrtCols + (int)(threadIdx.x >> 5) * 16;  // the warp's columns
+  const int j0 = jw + 8 * (lane & 1);
+  const bool mask = p.uplo != XKB_FULL;
+  // a block of 16 rows x 16 columns wholly outside the triangle
+  if (p.uplo == XKB_LOWER && (long)i0 + kCrtRows - 1 + p.diag < (long)jw) return;
+  if (p.uplo == XKB_UPPER && (long)i0 + p.diag > (long)jw + 15) return;
+  if (i >= p.M || j0 >= p.N) return;
+  uint2 words[NM];
+  const uint8_t* src = p.R + (size_t)jw * (size_t)p.Mpad + (size_t)i * 16 + (size_t)(8 * (lane & 1));
 #pragma unroll
   for (int m = 0; m < NM; ++m)
-    words[m] = *reinterpret_cast<const uint32_t*>(p.R + (size_t)m * plane + (size_t)j * p.Mpad + i0);
-  const int nuj = shift_of(p.nu[j], H);
+    words[m] = __ldcs(reinterpret_cast<const uint2*>(src + (size_t)m * plane));
+  const int last = p.N - j0;  // columns of this thread inside C
+  const bool whole = !mask && jw + 16 <= p.N;  // the warp's
+  auto in = [&](int e) {
+    if (whole) return true;
+    if (e >= last) return false;
+    if (!mask) return true;
+    return p.uplo == XKB_LOWER ? (long)i + p.diag >= (long)(j0 + e)
+                               : (long)i + p.diag <= (long)(j0 + e);
+  };
+  double s1[8], s2[8];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    uint32_t r[NM];
+  for (int e = 0; e < 8; ++e) {
+    s1[e] = c.s1;
+    s2[e] = c.s2;
+  }
 #pragma unroll
-    for (int m = 0; m < NM; ++m) r[m] = __byte_perm(words[m], 0u, 0x4440 + v);
-    const int mui = shift_of(p.mu[min(i0 + v, (long)p.M - 1)], H);
-    if (mui == kShiftNonFinite || nuj == kShiftNonFinite) y[v] = __longlong_as_double(0x7ff8000000000000ll);
-    else y[v] = scale2(crt_value<NM>(r, c), -(mui + nuj));
+  for (int m = 0; m < NM; ++m) {
+    const double w1 = c.w1[m], w2 = c.w2[m];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      // bytes 40 B0 r 00: the high word of the double 4096 + r
+      const uint32_t hi = __byte_perm(e < 4 ? words[m].x : words[m].y, 0x40B00000u,
+                                      0x7604 + ((e & 3) << 4));
+      const double rv = __hiloint2double((int)hi, 0);
+      s1[e] = fma(rv, w1, s1[e]);
+      s2[e] = fma(rv, w2, s2[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (in(e)) pre(i, j0 + e, e);
+  const int mui = shift_of(p.mu[i], H);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    if (!in(e)) continue;
+    const double q = rint(s1[e] * c.invPd);
+    const double v = fma(-q, c.P1d, s1[e]) + fma(-q, c.P2d, s2[e]);
+    const int nuj = shift_of(p.nu[j0 + e], H);
+    f(i, j0 + e, e, (mui == kShiftNonFinite || nuj == kShiftNonFinite)
+                        ? __longlong_as_double(0x7ff8000000000000ll)
+                        : scale2(v, -(mui + nuj)));
   }
 }
 
 template <int NM>
 __device__ __forceinline__ void crt_body(const CrtP& p, const Consts& c, int H) {
-  const long iq = (long)blockIdx.x * blockDim.x + threadIdx.x;  // row quad
-  const long i0 = iq * 4;
-  if (i0 >= p.M) return;
-  for (int j = blockIdx.y; j < p.N; j += gridDim.y) {
-    double y[4];
-    crt_quad<NM>(p, c, H, i0, j, y);
-    const size_t idx0 = (size_t)i0 + (size_t)j * p.ldc;
-    if (!p.cplx) {
-      const bool full = i0 + 3 < p.M && p.uplo == XKB_FULL &&
-                        (reinterpret_cast<uintptr_t>(p.C + idx0) & 15) == 0;
-      if (full) {  // two 16-byte loads / stores for the quad
-        double2* cp2 = reinterpret_cast<double2*>(p.C + idx0);
-        double2 o0 = make_double2(p.ar * y[0], p.ar * y[1]);
-        double2 o1 = make_double2(p.ar * y[2], p.ar * y[3]);
-        if (p.br != 0.0) {
-          const double2 c0 = cp2[0], c1 = cp2[1];
-          o0.x = fma(p.br, c0.x, o0.x);
-          o0.y = fma(p.br, c0.y, o0.y);
-          o1.x = fma(p.br, c1.x, o1.x);
-          o1.y = fma(p.br, c1.y, o1.y);
-        }
-        cp2[0] = o0;
-        cp2[1] = o1;
-        continue;
-      }
-    }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const long i = i0 + v;
-      if (i >= p.M) break;
-      if (p.uplo == XKB_LOWER && i + p.diag < j) continue;
-      if (p.uplo == XKB_UPPER && i + p.diag > j) continue;
-      const size_t idx = (size_t)i + (size_t)j * p.ldc;
-      if (!p.cplx) {
-        double out = p.ar * y[v];
-        if (p.br != 0.0) out = fma(p.br, p.C[idx], out);
-        p.C[idx] = out;
-      } else {
-        // complex: the first pass wrote Re(AB) into p.other[i + j*M]; this
-        // pass reconstructs Im(AB) and writes the (Re, Im) pairs of C
-        const double xr = p.other[(size_t)i + (size_t)j * p.M], xi = y[v];
-        double vr = p.ar * xr - p.ai * xi;
-        double vi = p.ar * xi + p.ai * xr;
-        if (p.br != 0.0 || p.bi != 0.0) {
+  const bool beta = p.br != 0.0 || p.bi != 0.0;
+  if (!p.cplx) {
+    double cr[8];
+    crt_cols<NM>(
+        p, c, H,
+        [&](int i, int j, int e) {
+          if (beta) cr[e] = p.C[(size_t)i + (size_t)j * p.ldc];
+        },
+        [&](int i, int j, int e, double y) {
+          double out = p.ar * y;
+          if (beta) out = fma(p.br, cr[e], out);
+          p.C[(size_t)i + (size_t)j * p.ldc] = out;
+        });
+    return;
+  }
+  // complex: the first pass wrote Re(AB) into p.other[i + j*M]; this pass
+  // reconstructs Im(AB) and writes the (Re, Im) pairs of C
+  double xr[8];
+  crt_cols<NM>(
+      p, c, H, [&](int i, int j, int e) { xr[e] = p.other[(size_t)i + (size_t)j * p.M]; },
+      [&](int i, int j, int e, double y) {
+        const size_t idx = (size_t)i + (size_t)j * p.ldc;
+        double vr = p.ar * xr[e] - p.ai * y;
+        double vi = p.ar * y + p.ai * xr[e];
+        if (beta) {
           const double cr = p.C[2 * idx], ci = p.C[2 * idx + 1];
           vr += p.br * cr - p.bi * ci;
           vi += p.br * ci + p.bi * cr;
@@ -1064,30 +1079,16 @@ __device__ __forceinline__ void crt_body(const CrtP& p, const Consts& c, int H) 
         if (p.herm_diag && i + p.diag == j) vi = 0.0;
         p.C[2 * idx] = vr;
         p.C[2 * idx + 1] = vi;
-      }
-    }
-  }
+      });
 }
 
 // Complex first pass: Re(op(A)op(B)) (unscaled by alpha) into a scratch M x N.
 template <int NM>
 __device__ __forceinline__ void crt_store_body(const CrtP& p, const Consts& c, int H,
                                                double* out) {
-  const long iq = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long i0 = iq * 4;
-  if (i0 >= p.M) return;
-  for (int j = blockIdx.y; j < p.N; j += gridDim.y) {
-    double y[4];
-    crt_quad<NM>(p, c, H, i0, j, y);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const long i = i0 + v;
-      if (i >= p.M) break;
-      if (p.uplo == XKB_LOWER && i + p.diag < j) continue;
-      if (p.uplo == XKB_UPPER && i + p.diag > j) continue;
-      out[(size_t)i + (size_t)j * p.M] = y[v];
-    }
-  }
+  crt_cols<NM>(
+      p, c, H, [](int, int, int) {},
+      [&](int i, int j, int, double y) { out[(size_t)i + (size_t)j * p.M] = y; });
 }
 
 // CRT kernels.  A fixed count: one instance per count.  A count chosen on the
@@ -1095,24 +1096,24 @@ __device__ __forceinline__ void crt_store_body(const CrtP& p, const Consts& c, i
 // holding both reconstructions, each block taking the one sel->n names.  A
 // call the pick sent to the plain kernel (sel->n == 0) writes nothing here.
 template <int NM>
-__global__ void __launch_bounds__(256, 4) k_oz_crt(const CrtP p, const Consts c) {
+__global__ void __launch_bounds__(256, 3) k_oz_crt(const CrtP p, const Consts c) {
   const OzSel s = *p.sel;
   if (s.n != NM) return;
   crt_body<NM>(p, c, s.H);
 }
 template <int NM>
-__global__ void __launch_bounds__(256, 4) k_oz_crt_store(const CrtP p, const Consts c, double* out) {
+__global__ void __launch_bounds__(256, 3) k_oz_crt_store(const CrtP p, const Consts c, double* out) {
   const OzSel s = *p.sel;
   if (s.n != NM) return;
   crt_store_body<NM>(p, c, s.H, out);
 }
-__global__ void __launch_bounds__(256, 4) k_oz_crt_15_16(const CrtP p, const Consts c15,
+__global__ void __launch_bounds__(256, 3) k_oz_crt_15_16(const CrtP p, const Consts c15,
                                                          const Consts c16) {
   const OzSel s = *p.sel;
   if (s.n == 15) crt_body<15>(p, c15, s.H);
   else if (s.n == 16) crt_body<16>(p, c16, s.H);
 }
-__global__ void __launch_bounds__(256, 4) k_oz_crt_store_15_16(const CrtP p, const Consts c15,
+__global__ void __launch_bounds__(256, 3) k_oz_crt_store_15_16(const CrtP p, const Consts c15,
                                                                const Consts c16, double* out) {
   const OzSel s = *p.sel;
   if (s.n == 15) crt_store_body<15>(p, c15, s.H, out);
@@ -1125,9 +1126,11 @@ static void crt_launch(dim3 g, cudaStream_t st, const CrtP& cp, const Consts& c,
   else k_oz_crt<NM><<<g, 256, 0, st>>>(cp, c);
 }
 // lo == hi: that count; (lo, hi) == (15, 16): the count the device chose.
-static int launch_crt(dim3 g, cudaStream_t st, const CrtP& cp, const Consts* lo,
+static int launch_crt(cudaStream_t st, const CrtP& cp, const Consts* lo,
                       const Consts* hi, double* store) {
   if (!lo || !hi) return XKB_EINVAL;
+  const dim3 g((unsigned)((cp.M + kCrtRows - 1) / kCrtRows),
+               (unsigned)((cp.N + kCrtCols - 1) / kCrtCols));
   const long long tv = evlog_kern_begin(st, store ? "k_oz_crt_store" : "k_oz_crt");
   if (lo->nmod != hi->nmod) {
     if (lo->nmod != 15 || hi->nmod != 16) return XKB_EINVAL;
@@ -1315,7 +1318,9 @@ static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_r
   p.diag = diag;
   for (int m = 0; m < c->nmod; ++m) {
     p.p[m] = c->p[m];
-    p.invp[m] = c->invp_d[m];
+    p.magic[m] = c->magic[m];
+    p.bias[m] = (uint32_t)(((1ull << 31) + (uint64_t)c->p[m] - 1) / (uint64_t)c->p[m]) *
+                (uint32_t)c->p[m];
   }
   const long total2 = (Mpad % BM2 == 0 && Npad % BN2 == 0)
                          ? (Mpad / BM2) * (Npad / BN2) * (long)c->nmod : 0;
@@ -1547,7 +1552,6 @@ extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* strea
   cp.uplo = a->uplo;
   cp.herm_diag = a->herm_diag;
   cp.diag = a->diag;
-  const dim3 cg((unsigned)(((M + 3) / 4 + 255) / 256), (unsigned)std::min(N, 65535));
   trace_mark(slot, 1, st);
   if (err == XKB_OK) {
     err = same ? launch_gemm(Ap, Arows, Ap, Arows, Mpad, Npad, Kpad, pl.chi, sel, R, a->uplo,
@@ -1557,16 +1561,16 @@ extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* strea
     if (!err) {
       if (!cplx) {
         trace_mark(slot, 2, st);
-        err = launch_crt(cg, st, cp, pl.clo, pl.chi, nullptr);
+        err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
       } else {
-        err = launch_crt(cg, st, cp, pl.clo, pl.chi, re);
+        err = launch_crt(st, cp, pl.clo, pl.chi, re);
         if (!err)
           err = launch_gemm(Ap, Mpad, Bp + szB, Npad, Mpad, Npad, Kpad, pl.chi, sel, R, a->uplo,
                             a->diag, st);
         trace_mark(slot, 2, st);
         if (!err) {
           cp.other = re;
-          err = launch_crt(cg, st, cp, pl.clo, pl.chi, nullptr);
+          err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
         }
       }
     }
@@ -1699,8 +1703,7 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
         cp.ar = a->alpha[0];
         cp.br = a->beta[0];
         cp.uplo = XKB_FULL;
-        const dim3 cg((unsigned)(((M + 3) / 4 + 255) / 256), (unsigned)std::min<long>(nw, 65535));
-        err = launch_crt(cg, st, cp, c, c, nullptr);
+        err = launch_crt(st, cp, c, c, nullptr);
       }
     }
     done(q);  // recorded on every path: waiters never hang on an error
@@ -1870,8 +1873,7 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
         cp.ar = a->alpha[0];
         cp.br = a->beta[0];
         cp.uplo = XKB_FULL;
-        const dim3 cg((unsigned)(((cp.M + 3) / 4 + 255) / 256), (unsigned)std::min<long>(cp.N, 65535));
-        err = launch_crt(cg, st, cp, c, c, nullptr);
+        err = launch_crt(st, cp, c, c, nullptr);
       }
     }
     done(k);  // recorded on every path: waiters never hang on an error
@@ -2126,8 +2128,7 @@ extern "C" int xkb_cuda_ozaki_gemm_noalloc(const xkb_gemm_args* a, int nmod, voi
     cp.br = a->beta[0];
     cp.uplo = a->uplo;
     cp.diag = a->diag;
-    const dim3 cg((unsigned)(((M + 3) / 4 + 255) / 256), (unsigned)N);
-    err = launch_crt(cg, st, cp, pl.clo, pl.chi, nullptr);
+    err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
   }
   trace_mark(slot, 3, st);
   return err;
