@@ -33,6 +33,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "xkb_dev.cuh"
@@ -40,7 +41,9 @@
 namespace xkb {
 namespace oz {
 
-constexpr int kMaxMod = 16;
+constexpr int kMaxMod = 16;  // moduli of a real product
+constexpr int kMaxC = 17;    // moduli of a complex product (two planes each)
+constexpr int kMaxPl = 2 * kMaxC;  // residue planes of an operand
 
 struct Consts {
   int nmod;
@@ -168,6 +171,118 @@ static bool make_consts(int n, Consts* c) {
 }
 
 // ---------------------------------------------------------------------------
+// Complex products.  Modulo an odd p whose prime factors are all 1 mod 4, -1
+// has a square root j, and a + ib -> (a + jb, a - jb) maps the complex
+// integers mod p onto pairs of integers mod p with the product taken entry by
+// entry.  So a complex contraction costs TWO real INT8 products per modulus
+// (four with the operands concatenated as [Re | Im]), and the residues of its
+// real and imaginary parts are (c+ + c-) / 2 and (c+ - c-) / (2j).  The factors
+// 1/2 and 1/(2j) go into the CRT weights.  These moduli are smaller (the
+// seventeen largest such pairwise coprime ones from 241 down), so a call of n
+// real moduli's budget H takes n + 1 of them: 16 for n = 15, 17 for n = 16.
+constexpr int kCMod[kMaxC] = {241, 233, 229, 221, 205, 197, 193, 181, 173,
+                              157, 149, 137, 113, 109, 101, 97,  89};
+
+struct CResConsts {  // of the residue kernel
+  int p[kMaxC], half[kMaxC];
+  uint32_t wlo[kMaxC], whi[kMaxC];  // bytes of 2^(8t) mod p
+  uint32_t jlo[kMaxC], jhi[kMaxC];  // bytes of j 2^(8t) mod p
+  uint32_t off[kMaxC], offj[kMaxC];  // undo the +2^62 offset of Re (plus half) and of Im
+  uint32_t cp[kMaxC];                // a multiple of p above j Im's largest sum
+  uint32_t magic[kMaxC];
+};
+struct CCrtConsts {  // of the recombination with n moduli, weights split as in Consts
+  double w1[kMaxC], w2[kMaxC];  // real part: times c+ + c-
+  double v1[kMaxC], v2[kMaxC];  // imaginary part: times c+ - c-
+  double s1, s2;                // -8192 sum w1, -8192 sum w2
+  double P1d, P2d, invPd;
+};
+struct CCrtTab {
+  CCrtConsts c[kMaxC + 1];  // by moduli count
+};
+
+static double log2Pc(int n) {
+  double s = 0;
+  for (int i = 0; i < n; ++i) s += std::log2((double)kCMod[i]);
+  return s;
+}
+
+static uint32_t pack_weights(uint64_t f, int p, int t0) {
+  uint32_t r = 0;
+  for (int t = t0; t < t0 + 4; ++t) {
+    uint64_t w = f % (uint64_t)p;
+    for (int q = 0; q < 8 * t; ++q) w = (w * 2) % (uint64_t)p;
+    r |= (uint32_t)w << (8 * (t - t0));
+  }
+  return r;
+}
+
+static int sqrt_minus_one(int p) {
+  for (int j = 1; j < p; ++j)
+    if ((j * j) % p == p - 1) return j;
+  return 0;
+}
+
+static const CResConsts& cres_consts() {
+  static const CResConsts c = [] {
+    CResConsts r;
+    for (int i = 0; i < kMaxC; ++i) {
+      const int p = kCMod[i], j = sqrt_minus_one(p);
+      uint64_t t62 = 1;
+      for (int q = 0; q < 62; ++q) t62 = (t62 * 2) % (uint64_t)p;
+      r.p[i] = p;
+      r.half[i] = p / 2;
+      r.wlo[i] = pack_weights(1, p, 0);
+      r.whi[i] = pack_weights(1, p, 4);
+      r.jlo[i] = pack_weights((uint64_t)j, p, 0);
+      r.jhi[i] = pack_weights((uint64_t)j, p, 4);
+      r.off[i] = (uint32_t)((uint64_t)p - t62) + (uint32_t)(p / 2);
+      r.offj[i] = (uint32_t)((uint64_t)p - (t62 * (uint64_t)j) % (uint64_t)p);
+      r.cp[i] = (uint32_t)(((1 << 20) + p - 1) / p * p);
+      r.magic[i] = (uint32_t)(((1ull << 32) + (uint64_t)p - 1) / (uint64_t)p);
+    }
+    return r;
+  }();
+  return c;
+}
+
+static const CCrtTab& ccrt_tab() {
+  static const CCrtTab tab = [] {
+    CCrtTab t;
+    std::memset(&t, 0, sizeof(t));
+    for (int n = 2; n <= kMaxC; ++n) {
+      CCrtConsts& c = t.c[n];
+      u128 P = 1;
+      for (int i = 0; i < n; ++i) P *= (u128)kCMod[i];
+      // sum_l (8192 + c+ + c-) w1 < 17 * 8702 P < 2^(bits(P)+18)
+      int bitsP = 0;
+      for (u128 q = P; q; q >>= 1) ++bitsP;
+      const int cs = std::max(0, bitsP + 18 - 53);
+      const u128 low = cs ? (((u128)1 << cs) - 1) : 0;
+      for (int i = 0; i < n; ++i) {
+        const int p = kCMod[i], j = sqrt_minus_one(p);
+        const u128 Mi = P / (u128)p;
+        const int im = inv_mod((int)(Mi % (u128)p), p);
+        const int fr = (int)((long)im * inv_mod(2, p) % p);
+        const int fi = (int)((long)im * inv_mod(2 * j % p, p) % p);
+        const u128 w = Mi * (u128)fr, v = Mi * (u128)fi;  // below P
+        c.w1[i] = std::ldexp((double)(uint64_t)(w >> cs), cs);
+        c.w2[i] = (double)(w & low);
+        c.v1[i] = std::ldexp((double)(uint64_t)(v >> cs), cs);
+        c.v2[i] = (double)(v & low);
+        c.s1 -= 8192.0 * c.w1[i];
+        c.s2 -= 8192.0 * c.w2[i];
+      }
+      c.P1d = std::ldexp((double)(uint64_t)(P >> cs), cs);
+      c.P2d = (double)(P & low);
+      c.invPd = 1.0 / (double)P;
+    }
+    return t;
+  }();
+  return tab;
+}
+
+// ---------------------------------------------------------------------------
 // 1. scaling exponents and the moduli count.  View the operand as L "rows"
 //    of length K, element (l,k) at X[l*sl + k*sk] (one of sl, sk is 1).
 //    Partial sums over k-chunks go to part[chunk][l] = (sum of squares,
@@ -178,24 +293,40 @@ constexpr int kNormChunk = 512;
 // every later kernel of the call: n moduli (0: the plain FP64 kernel runs
 // instead), H the exponent budget of the scaled operands for that count.
 struct OzSel {
-  int n, H, fallback, pad;
+  int n, H, fallback;
+  int np;  // moduli actually multiplied: n, or a complex product's larger count
 };
 
 // Counters over all contractions of the process (xkb_ozaki_counts).
 static __device__ unsigned long long g_oz_calls, g_oz_mod_sum, g_oz_fallbacks;
 static __device__ int g_oz_last = -1;
 
-template <bool KC>  // KC: k contiguous (sk == 1)
-__global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const double* X, long ld, int cplx,
+// Exponent of the lowest set bit of a float that is not 0.
+__device__ __forceinline__ int lsb_exp(float x) {
+  const int b = __float_as_int(x), e = (b >> 23) & 0xff, m = b & 0x7fffff;
+  return e ? e - 150 + __ffs(m | 0x800000) - 1 : -150 + __ffs(m);
+}
+
+// KC: k contiguous (sk == 1).  Single-precision operands (exact products, see
+// k_oz_pick): the third sum is the lowest bit of the row's entries instead.
+template <bool KC, class E>
+__global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const E* X, long ld, int cplx,
                                                   double4* part) {
+  constexpr bool EXACT = sizeof(E) == 4;
   // block: 32 rows x 8 lanes along k (KC: warp-cooperative along k instead)
   const int chunk = blockIdx.y;
   const int k0 = chunk * kNormChunk, k1 = min(K, k0 + kNormChunk);
-  double ss = 0.0, mx = 0.0, s1 = 0.0, nz = 0.0;
-  auto acc = [&](double v) {
+  double ss = 0.0, mx = 0.0, s1 = EXACT ? 1.0e6 : 0.0, nz = 0.0;
+  auto merge = [](double a, double b) { return EXACT ? fmin(a, b) : a + b; };
+  auto acc = [&](E x) {
+    const double v = (double)x;
     ss = fma(v, v, ss);
     mx = fmax(mx, fabs(v));
-    s1 += fabs(v);
+    if constexpr (EXACT) {
+      if (x != 0.0f) s1 = fmin(s1, (double)lsb_exp(x));
+    } else {
+      s1 += fabs(v);
+    }
     nz += (v != 0.0) ? 1.0 : 0.0;
   };
   if constexpr (KC) {
@@ -216,7 +347,7 @@ __global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const double* X, 
     for (int o = 16; o; o >>= 1) {
       ss += __shfl_xor_sync(0xffffffffu, ss, o);
       mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s1 = merge(s1, __shfl_xor_sync(0xffffffffu, s1, o));
       nz += __shfl_xor_sync(0xffffffffu, nz, o);
     }
     if (lane == 0 && l < L) part[(size_t)chunk * L + l] = make_double4(ss, mx, s1, nz);
@@ -242,7 +373,7 @@ __global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const double* X, 
       for (int i = 1; i < 8; ++i) {
         t.x += red[i][tl].x;
         t.y = fmax(t.y, red[i][tl].y);
-        t.z += red[i][tl].z;
+        t.z = merge(t.z, red[i][tl].z);
         t.w += red[i][tl].w;
       }
       part[(size_t)chunk * L + l] = t;
@@ -270,23 +401,30 @@ __device__ __forceinline__ int shift_of(int code, int H) {
 // rho = sqrt(nnz) ||x||_2 / ||x||_1 (1 for entries of one magnitude, up to
 // sqrt(nnz) for one dominant entry), whose maximum over the rows goes to
 // *rmax (a non-negative float compared as its bits).
+// exact (single precision): the code is the exponent of the row's lowest bit
+// instead, and *rmax the largest log2 of the 2-norm of a row scaled to
+// integers by it (infinite when a row holds Inf / NaN).
 __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* code,
-                          unsigned* rmax) {
+                          unsigned* rmax, int exact) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   float rho = 0.0f;
   if (l < L) {
-    double ss = 0.0, mx = 0.0, s1 = 0.0, nz = 0.0;
+    double ss = 0.0, mx = 0.0, s1 = exact ? 1.0e6 : 0.0, nz = 0.0;
     for (int c = 0; c < nchunks; ++c) {  // fixed order: deterministic
       const double4 v = part[(size_t)c * L + l];
       ss += v.x;
       mx = fmax(mx, v.y);
-      s1 += v.z;
+      s1 = exact ? fmin(s1, v.z) : s1 + v.z;
       nz += v.w;
     }
     if (!isfinite(mx) || isnan(ss)) {
       code[l] = kShiftNonFinite;
+      if (exact) rho = __int_as_float(0x7f800000);
     } else if (mx == 0.0) {
       code[l] = kCodeZero;
+    } else if (exact) {
+      code[l] = (int)s1;
+      rho = (float)(log2(fmax(sqrt(ss), mx)) - s1 + 1e-3);  // >= 0: the row has a bit at s1
     } else {
       // bound on the row 2-norm (the sum of squares may overflow for huge entries)
       double nrm = isfinite(ss) ? sqrt(ss) : mx * sqrt((double)K);
@@ -314,14 +452,32 @@ __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* c
 // FP64 rounding; if the largest count cannot, the call runs the plain FP64
 // kernel instead (fallback = 1), or, where that is not allowed, the largest
 // count.  fixed > 0: that count, no data rule.
+// Exact products (single-precision operands): the operands are scaled to
+// integers without rounding, so the product is the exact one whenever
+// ||a'_i|| ||b'_j|| < P/4 for all rows and columns: the smallest count for
+// which it is; else the plain kernel.
 struct PickP {
-  int fixed, lo, hi, allow_fallback;
-  int H[kMaxMod + 1];  // exponent budget per count
+  int fixed, lo, hi, allow_fallback, exact;
+  int H[kMaxMod + 1];        // exponent budget per count
+  int np[kMaxMod + 1];       // moduli multiplied per count
+  float lim[kMaxC + 1];      // exact: log2 of P/4 per moduli multiplied
 };
 
 __global__ void k_oz_pick(const unsigned* rmax, OzSel* sel, const PickP q) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int n = q.fixed, fb = 0;
+  if (q.exact) {
+    const float ra = __uint_as_float(rmax[0]), rb = __uint_as_float(rmax[1]);
+    n = 0;
+#pragma unroll
+    for (int c = kMaxC; c >= 2; --c)
+      if (c >= q.lo && c <= q.hi && ra < 61.5f && rb < 61.5f && ra + rb <= q.lim[c]) n = c;
+    sel->n = n;
+    sel->H = 0;  // the codes are the shifts
+    sel->fallback = n == 0;
+    sel->np = n;
+    return;
+  }
   if (n <= 0) {
     const double ra = fmax(1.0, (double)__uint_as_float(rmax[0]));
     const double rb = fmax(1.0, (double)__uint_as_float(rmax[1]));
@@ -338,7 +494,11 @@ __global__ void k_oz_pick(const unsigned* rmax, OzSel* sel, const PickP q) {
   sel->n = n;
   sel->H = n ? q.H[n] : 0;
   sel->fallback = fb;
-  sel->pad = 0;
+  int np = 0;
+#pragma unroll
+  for (int c = kMaxMod; c >= 2; --c)
+    if (c == n) np = q.np[c];
+  sel->np = np;
   atomicAdd(&g_oz_calls, 1ull);
   atomicAdd(&g_oz_mod_sum, (unsigned long long)n);
   if (fb) atomicAdd(&g_oz_fallbacks, 1ull);
@@ -377,13 +537,12 @@ __device__ __forceinline__ void res_planes(const Consts& c, const uint32_t (&lo)
   }
 }
 
-template <bool KC, int NM>
-__global__ void __launch_bounds__(256) k_oz_residues(int L, int K, const double* X, long ld,
-                                                      long estride, long eoff, double esign,
+template <bool KC, int NM, class E>
+__global__ void __launch_bounds__(256) k_oz_residues(int L, int K, const E* X, long ld,
                                                       const int* code, const OzSel* sel,
                                                       const Consts c, int8_t* planes, long Lpad,
-                                                      long Kpad, long kofs) {
-  // X element (l,k) = esign * X[eoff + estride*(KC ? k + l*ld : l + k*ld)];
+                                                      long Kpad) {
+  // X element (l,k) = X[KC ? k + l*ld : l + k*ld];
   // planes 0 .. sel->n - 1 are written (NM: the most the call may use)
   const int nm = sel->n, H = sel->H;
   if (nm == 0) return;  // the plain kernel computes this call
@@ -400,7 +559,7 @@ __global__ void __launch_bounds__(256) k_oz_residues(int L, int K, const double*
       v[q] = 0.0;
       if (l < L && k < K) {
         const size_t idx = KC ? (size_t)k + (size_t)l * ld : (size_t)l + (size_t)k * ld;
-        v[q] = esign * X[eoff + estride * idx];
+        v[q] = (double)X[idx];
       }
     }
 #pragma unroll
@@ -429,7 +588,7 @@ __global__ void __launch_bounds__(256) k_oz_residues(int L, int K, const double*
       lo[v] = (uint32_t)u;
       hi[v] = (uint32_t)(u >> 32);
     }
-    int8_t* dst = planes + (size_t)l * Kpad + kofs + k0 + kq;
+    int8_t* dst = planes + (size_t)l * Kpad + k0 + kq;
     // p_0 = 256: the two's complement low byte (the offset 2^62 is 0 mod 256)
     *reinterpret_cast<uint32_t*>(dst) =
         __byte_perm(__byte_perm(lo[0], lo[1], 0x0040), __byte_perm(lo[2], lo[3], 0x0040), 0x5410);
@@ -439,6 +598,81 @@ __global__ void __launch_bounds__(256) k_oz_residues(int L, int K, const double*
     else if (NM > 2 && nm == NM - 1)
       res_planes<(NM > 2 ? NM - 1 : NM)>(c, lo, hi, dst, plane, NM - 1);
     else res_planes<NM>(c, lo, hi, dst, plane, nm);
+  }
+}
+
+// Residue planes of a complex operand: planes 2m and 2m + 1 hold a + jb and
+// a - jb mod p_m of every element a + ib (sign = -1: of its conjugate); element
+// (l, k) = X[2 (KC ? k + l ld : l + k ld)].  The grid covers Lpad x Kpad.
+template <bool KC, class E>
+__global__ void __launch_bounds__(256) k_oz_residues_c(int L, int K, const E* X, long ld,
+                                                        double sign, const int* code,
+                                                        const OzSel* sel, const CResConsts c,
+                                                        int8_t* planes, long Lpad, long Kpad) {
+  using E2 = typename std::conditional<sizeof(E) == 4, float2, double2>::type;
+  const int nm = sel->np, H = sel->H;
+  if (nm == 0) return;
+  __shared__ double tr[64][33], ti[64][33];
+  const int l0 = blockIdx.x * 64, k0 = blockIdx.y * 32;
+  {
+    E2 v[8];  // all loads of a thread in flight before the shared stores
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = threadIdx.x + q * 256;
+      const int l = l0 + (KC ? e >> 5 : e & 63), k = k0 + (KC ? e & 31 : e >> 6);
+      v[q].x = v[q].y = (E)0;
+      if (l < L && k < K) {
+        const size_t idx = KC ? (size_t)k + (size_t)l * ld : (size_t)l + (size_t)k * ld;
+        v[q].x = X[2 * idx];
+        v[q].y = X[2 * idx + 1];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = threadIdx.x + q * 256;
+      tr[KC ? e >> 5 : e & 63][KC ? e & 31 : e >> 6] = (double)v[q].x;
+      ti[KC ? e >> 5 : e & 63][KC ? e & 31 : e >> 6] = sign * (double)v[q].y;
+    }
+  }
+  __syncthreads();
+  const size_t plane = (size_t)Lpad * (size_t)Kpad;
+#pragma unroll 1
+  for (int it = threadIdx.x; it < 64 * 8; it += 256) {
+    const int ll = it >> 3, kq = (it & 7) * 4;
+    const int l = l0 + ll;
+    const int s = (l < L) ? shift_of(code[l], H) : 0;
+    const double sc = (s == kShiftNonFinite) ? 0.0 : pow2(s / 2) * pow2(s - s / 2);
+    uint32_t rl[4], rh[4], il[4], ih[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {  // offset values a + 2^62, b + 2^62
+      const unsigned long long u =
+          (unsigned long long)llrint(tr[ll][kq + v] * sc) + (1ull << 62);
+      const unsigned long long w =
+          (unsigned long long)llrint(ti[ll][kq + v] * sc) + (1ull << 62);
+      rl[v] = (uint32_t)u, rh[v] = (uint32_t)(u >> 32);
+      il[v] = (uint32_t)w, ih[v] = (uint32_t)(w >> 32);
+    }
+    int8_t* dst = planes + (size_t)l * Kpad + k0 + kq;
+#pragma unroll
+    for (int m = 0; m < kMaxC; ++m) {
+      if (m >= nm) break;
+      const uint32_t p = (uint32_t)c.p[m], h = (uint32_t)c.half[m], mg = c.magic[m];
+      uint32_t rp[4], rm[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        // sums of bytes times 2^(8t) mod p: below 2^22 with the offsets, so
+        // umulhi by ceil(2^32 / p) is the exact quotient
+        const uint32_t sa = __dp4a(rh[v], c.whi[m], __dp4a(rl[v], c.wlo[m], c.off[m]));
+        const uint32_t sj = __dp4a(ih[v], c.jhi[m], __dp4a(il[v], c.jlo[m], c.offj[m]));
+        const uint32_t a = sa + sj, b = sa + (c.cp[m] - sj);
+        rp[v] = a - __umulhi(a, mg) * p - h;
+        rm[v] = b - __umulhi(b, mg) * p - h;
+      }
+      *reinterpret_cast<uint32_t*>(dst + (size_t)(2 * m) * plane) = __byte_perm(
+          __byte_perm(rp[0], rp[1], 0x0040), __byte_perm(rp[2], rp[3], 0x0040), 0x5410);
+      *reinterpret_cast<uint32_t*>(dst + (size_t)(2 * m + 1) * plane) = __byte_perm(
+          __byte_perm(rm[0], rm[1], 0x0040), __byte_perm(rm[2], rm[3], 0x0040), 0x5410);
+    }
   }
 }
 
@@ -458,14 +692,16 @@ constexpr int kEpiWarps = 4;
 
 struct GemmP {
   int tiles_m, tiles_n, kblocks, nmod;  // nmod: planes of the operand buffers (the most used)
-  const OzSel* sel;                     // moduli multiplied: sel->n (<= nmod)
+  const OzSel* sel;                     // planes multiplied: mult sel->np (<= nmod)
+  int mult;                             // planes per modulus: 1, complex 2
+  int bxor;  // plane z of op(A) meets plane z ^ bxor of op(B) (1: B is A's conjugate)
   int group;  // raster: M tiles per group (tiles in flight share A / B panels in L2)
   uint8_t* R;
   long Mpad, Npad;
   int uplo;
   long diag;
-  int p[kMaxMod];
-  uint32_t bias[kMaxMod], magic[kMaxMod];  // of the epilogue's mod p
+  int p[kMaxPl];
+  uint32_t bias[kMaxPl], magic[kMaxPl];  // of the epilogue's mod p
 };
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
@@ -598,7 +834,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t* acce = accf + 2;   // [2] accumulator drained
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
 
-  const int total = p.tiles_m * p.tiles_n * min(p.sel->n, p.nmod);
+  const int total = p.tiles_m * p.tiles_n * min(p.sel->np * p.mult, p.nmod);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -642,7 +878,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           mbar_expect_tx(&full[s], A_STAGE + B_STAGE);
           tma_load_3d(sA + s * A_STAGE, &tA, kb * BKB, m0, mod, &full[s]);
-          tma_load_3d(sB + s * B_STAGE, &tB, kb * BKB, n0, mod, &full[s]);
+          tma_load_3d(sB + s * B_STAGE, &tB, kb * BKB, n0, mod ^ p.bxor, &full[s]);
         }
       }
     }
@@ -806,7 +1042,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   const uint32_t rank = cluster_rank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int total = p.tiles_m * p.tiles_n * min(p.sel->n, p.nmod);
+  const int total = p.tiles_m * p.tiles_n * min(p.sel->np * p.mult, p.nmod);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S2; ++s) {
@@ -856,7 +1092,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           if (rank == 0) mbar_expect_tx(&full[s], 4 * H_STAGE);
           const uint32_t fe = smem_u32(&full[s]) & kPeerMask;
           tma_load_3d_pair(sA + s * H_STAGE, &tA, kb * BKB, m0 + 128 * (int)rank, mod, fe);
-          tma_load_3d_pair(sB + s * H_STAGE, &tB, kb * BKB, n0 + 128 * (int)rank, mod, fe);
+          tma_load_3d_pair(sB + s * H_STAGE, &tB, kb * BKB, n0 + 128 * (int)rank, mod ^ p.bxor,
+                           fe);
         }
       }
     }
@@ -936,11 +1173,9 @@ struct CrtP {
   const int* mu;     // row codes of op(A) (k_oz_stat)
   const int* nu;     // column codes of op(B)
   const OzSel* sel;  // the call's moduli count and exponent budget
-  double* C;         // interleaved complex when cplx: writes part `part` (0 re, 1 im)
+  void* C;
   long ldc;
-  int cplx, part;
   double ar, ai, br, bi;  // real: ar, br used
-  const double* other;    // complex: the other part's integer result, see host
   int uplo, herm_diag;
   long diag;
 };
@@ -1045,102 +1280,176 @@ __device__ __forceinline__ void crt_cols(const CrtP& p, const Consts& c, int H, 
   }
 }
 
-template <int NM>
+template <int NM, class E>
 __device__ __forceinline__ void crt_body(const CrtP& p, const Consts& c, int H) {
-  const bool beta = p.br != 0.0 || p.bi != 0.0;
-  if (!p.cplx) {
-    double cr[8];
-    crt_cols<NM>(
-        p, c, H,
-        [&](int i, int j, int e) {
-          if (beta) cr[e] = p.C[(size_t)i + (size_t)j * p.ldc];
-        },
-        [&](int i, int j, int e, double y) {
-          double out = p.ar * y;
-          if (beta) out = fma(p.br, cr[e], out);
-          p.C[(size_t)i + (size_t)j * p.ldc] = out;
-        });
-    return;
-  }
-  // complex: the first pass wrote Re(AB) into p.other[i + j*M]; this pass
-  // reconstructs Im(AB) and writes the (Re, Im) pairs of C
-  double xr[8];
+  const bool beta = p.br != 0.0;
+  E* C = static_cast<E*>(p.C);
+  double cr[8];
   crt_cols<NM>(
-      p, c, H, [&](int i, int j, int e) { xr[e] = p.other[(size_t)i + (size_t)j * p.M]; },
+      p, c, H,
+      [&](int i, int j, int e) {
+        if (beta) cr[e] = (double)C[(size_t)i + (size_t)j * p.ldc];
+      },
       [&](int i, int j, int e, double y) {
-        const size_t idx = (size_t)i + (size_t)j * p.ldc;
-        double vr = p.ar * xr[e] - p.ai * y;
-        double vi = p.ar * y + p.ai * xr[e];
-        if (beta) {
-          const double cr = p.C[2 * idx], ci = p.C[2 * idx + 1];
-          vr += p.br * cr - p.bi * ci;
-          vi += p.br * ci + p.bi * cr;
-        }
-        if (p.herm_diag && i + p.diag == j) vi = 0.0;
-        p.C[2 * idx] = vr;
-        p.C[2 * idx + 1] = vi;
+        double out = p.ar * y;
+        if (beta) out = fma(p.br, cr[e], out);
+        C[(size_t)i + (size_t)j * p.ldc] = (E)out;
       });
 }
 
-// Complex first pass: Re(op(A)op(B)) (unscaled by alpha) into a scratch M x N.
-template <int NM>
-__device__ __forceinline__ void crt_store_body(const CrtP& p, const Consts& c, int H,
-                                               double* out) {
-  crt_cols<NM>(
-      p, c, H, [](int, int, int) {},
-      [&](int i, int j, int, double y) { out[(size_t)i + (size_t)j * p.M] = y; });
+// Complex recombination: a warp takes 8 rows x 16 columns, a lane row l / 4
+// and the four columns 4 (l % 4) .. + 3; both parts of an element come from
+// the planes 2m (c+) and 2m + 1 (c-) in one pass.  c+ and c- enter as 4096 + r
+// (see above): their sum, offset by 8192, meets the real part's weights, their
+// difference the imaginary part's.  Same bounds as the real form: the real
+// part's partial sums stay below 17 * 8702 P < 2^(53+csplit), |q| < 2^14, and
+// |C'| <= P/4 leaves q = rint(S1 / P) exact.
+constexpr int kCrtRowsC = 8;
+
+template <int NM, class E>
+__device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, int H) {
+  const size_t plane = (size_t)p.Mpad * (size_t)p.Npad;
+  const int lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * kCrtRowsC, i = i0 + (lane >> 2);
+  const int jw = blockIdx.y * kCrtCols + (int)(threadIdx.x >> 5) * 16;
+  const int j0 = jw + 4 * (lane & 3);
+  if (p.uplo == XKB_LOWER && (long)i0 + kCrtRowsC - 1 + p.diag < (long)jw) return;
+  if (p.uplo == XKB_UPPER && (long)i0 + p.diag > (long)jw + 15) return;
+  if (i >= p.M || j0 >= p.N) return;
+  uint32_t wp[NM], wm[NM];
+  const uint8_t* src = p.R + (size_t)jw * (size_t)p.Mpad + (size_t)i * 16 + (size_t)(4 * (lane & 3));
+#pragma unroll
+  for (int m = 0; m < NM; ++m) {
+    wp[m] = __ldcs(reinterpret_cast<const uint32_t*>(src + (size_t)(2 * m) * plane));
+    wm[m] = __ldcs(reinterpret_cast<const uint32_t*>(src + (size_t)(2 * m + 1) * plane));
+  }
+  double r1[4], r2[4], x1[4], x2[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    r1[e] = c.s1;
+    r2[e] = c.s2;
+    x1[e] = x2[e] = 0.0;
+  }
+#pragma unroll
+  for (int m = 0; m < NM; ++m) {
+    const double w1 = c.w1[m], w2 = c.w2[m], v1 = c.v1[m], v2 = c.v2[m];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const double a =
+          __hiloint2double((int)__byte_perm(wp[m], 0x40B00000u, 0x7604 + (e << 4)), 0);
+      const double b =
+          __hiloint2double((int)__byte_perm(wm[m], 0x40B00000u, 0x7604 + (e << 4)), 0);
+      const double su = a + b, di = a - b;
+      r1[e] = fma(su, w1, r1[e]);
+      r2[e] = fma(su, w2, r2[e]);
+      x1[e] = fma(di, v1, x1[e]);
+      x2[e] = fma(di, v2, x2[e]);
+    }
+  }
+  const bool beta = p.br != 0.0 || p.bi != 0.0;
+  const bool mask = p.uplo != XKB_FULL;
+  E* C = static_cast<E*>(p.C);
+  auto in = [&](int e) {
+    if (j0 + e >= p.N) return false;
+    if (!mask) return true;
+    return p.uplo == XKB_LOWER ? (long)i + p.diag >= (long)(j0 + e)
+                               : (long)i + p.diag <= (long)(j0 + e);
+  };
+  double cr[4], ci[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    cr[e] = ci[e] = 0.0;
+    if (beta && in(e)) {
+      const size_t idx = (size_t)i + (size_t)(j0 + e) * p.ldc;
+      cr[e] = (double)C[2 * idx];
+      ci[e] = (double)C[2 * idx + 1];
+    }
+  }
+  const int mui = shift_of(p.mu[i], H);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (!in(e)) continue;
+    const int nuj = shift_of(p.nu[j0 + e], H);
+    const double qr = rint(r1[e] * c.invPd), qi = rint(x1[e] * c.invPd);
+    double xr = fma(-qr, c.P1d, r1[e]) + fma(-qr, c.P2d, r2[e]);
+    double xi = fma(-qi, c.P1d, x1[e]) + fma(-qi, c.P2d, x2[e]);
+    if (mui == kShiftNonFinite || nuj == kShiftNonFinite) {
+      xr = xi = __longlong_as_double(0x7ff8000000000000ll);
+    } else {
+      xr = scale2(xr, -(mui + nuj));
+      xi = scale2(xi, -(mui + nuj));
+    }
+    double vr = p.ar * xr - p.ai * xi;
+    double vi = p.ar * xi + p.ai * xr;
+    if (beta) {
+      vr += p.br * cr[e] - p.bi * ci[e];
+      vi += p.br * ci[e] + p.bi * cr[e];
+    }
+    if (p.herm_diag && (long)i + p.diag == (long)(j0 + e)) vi = 0.0;
+    const size_t idx = (size_t)i + (size_t)(j0 + e) * p.ldc;
+    C[2 * idx] = (E)vr;
+    C[2 * idx + 1] = (E)vi;
+  }
 }
 
 // CRT kernels.  A fixed count: one instance per count.  A count chosen on the
 // device between 15 and 16 (the data rule's range, k_oz_pick): one kernel
-// holding both reconstructions, each block taking the one sel->n names.  A
-// call the pick sent to the plain kernel (sel->n == 0) writes nothing here.
+// holding both reconstructions, each block taking the one sel->n names; the
+// single-precision and complex kernels hold every count a call may come to.
+// A call the pick sent to the plain kernel (sel->n == 0) writes nothing here.
 template <int NM>
 __global__ void __launch_bounds__(256, 3) k_oz_crt(const CrtP p, const Consts c) {
   const OzSel s = *p.sel;
   if (s.n != NM) return;
-  crt_body<NM>(p, c, s.H);
-}
-template <int NM>
-__global__ void __launch_bounds__(256, 3) k_oz_crt_store(const CrtP p, const Consts c, double* out) {
-  const OzSel s = *p.sel;
-  if (s.n != NM) return;
-  crt_store_body<NM>(p, c, s.H, out);
+  crt_body<NM, double>(p, c, s.H);
 }
 __global__ void __launch_bounds__(256, 3) k_oz_crt_15_16(const CrtP p, const Consts c15,
                                                          const Consts c16) {
   const OzSel s = *p.sel;
-  if (s.n == 15) crt_body<15>(p, c15, s.H);
-  else if (s.n == 16) crt_body<16>(p, c16, s.H);
-}
-__global__ void __launch_bounds__(256, 3) k_oz_crt_store_15_16(const CrtP p, const Consts c15,
-                                                               const Consts c16, double* out) {
-  const OzSel s = *p.sel;
-  if (s.n == 15) crt_store_body<15>(p, c15, s.H, out);
-  else if (s.n == 16) crt_store_body<16>(p, c16, s.H, out);
+  if (s.n == 15) crt_body<15, double>(p, c15, s.H);
+  else if (s.n == 16) crt_body<16, double>(p, c16, s.H);
 }
 
+constexpr int kExactLo = 8, kExactLoC = 9;  // fewest moduli of an exact product
+struct CrtTabS {
+  Consts c[kMaxMod - kExactLo + 1];
+};
 template <int NM>
-static void crt_launch(dim3 g, cudaStream_t st, const CrtP& cp, const Consts& c, double* store) {
-  if (store) k_oz_crt_store<NM><<<g, 256, 0, st>>>(cp, c, store);
-  else k_oz_crt<NM><<<g, 256, 0, st>>>(cp, c);
+__device__ __forceinline__ void crt_any_s(const CrtP& p, const CrtTabS& t, const OzSel& s) {
+  if (s.np == NM) crt_body<NM, float>(p, t.c[NM - kExactLo], s.H);
+  else if constexpr (NM < kMaxMod) crt_any_s<NM + 1>(p, t, s);
 }
+__global__ void __launch_bounds__(256, 3) k_oz_crt_s(const CrtP p,
+                                                     const __grid_constant__ CrtTabS t) {
+  const OzSel s = *p.sel;
+  if (s.np >= kExactLo) crt_any_s<kExactLo>(p, t, s);
+}
+template <int NM, class E>
+__device__ __forceinline__ void crt_any_c(const CrtP& p, const CCrtTab& t, const OzSel& s) {
+  if (s.np == NM) crt_body_c<NM, E>(p, t.c[NM], s.H);
+  else if constexpr (NM < kMaxC) crt_any_c<NM + 1, E>(p, t, s);
+}
+template <class E>
+__global__ void __launch_bounds__(256, 2) k_oz_crt_c(const CrtP p,
+                                                     const __grid_constant__ CCrtTab t) {
+  const OzSel s = *p.sel;
+  if (s.np >= 2) crt_any_c<2, E>(p, t, s);
+}
+
 // lo == hi: that count; (lo, hi) == (15, 16): the count the device chose.
-static int launch_crt(cudaStream_t st, const CrtP& cp, const Consts* lo,
-                      const Consts* hi, double* store) {
+static int launch_crt(cudaStream_t st, const CrtP& cp, const Consts* lo, const Consts* hi) {
   if (!lo || !hi) return XKB_EINVAL;
   const dim3 g((unsigned)((cp.M + kCrtRows - 1) / kCrtRows),
                (unsigned)((cp.N + kCrtCols - 1) / kCrtCols));
-  const long long tv = evlog_kern_begin(st, store ? "k_oz_crt_store" : "k_oz_crt");
+  const long long tv = evlog_kern_begin(st, "k_oz_crt");
   if (lo->nmod != hi->nmod) {
     if (lo->nmod != 15 || hi->nmod != 16) return XKB_EINVAL;
-    if (store) k_oz_crt_store_15_16<<<g, 256, 0, st>>>(cp, *lo, *hi, store);
-    else k_oz_crt_15_16<<<g, 256, 0, st>>>(cp, *lo, *hi);
+    k_oz_crt_15_16<<<g, 256, 0, st>>>(cp, *lo, *hi);
   } else {
     switch (hi->nmod) {
 #define XKB_CRT_CASE(NM) \
   case NM:               \
-    crt_launch<NM>(g, st, cp, *hi, store); break;
+    k_oz_crt<NM><<<g, 256, 0, st>>>(cp, *hi); break;
       XKB_CRT_CASE(2) XKB_CRT_CASE(3) XKB_CRT_CASE(4) XKB_CRT_CASE(5) XKB_CRT_CASE(6)
       XKB_CRT_CASE(7) XKB_CRT_CASE(8) XKB_CRT_CASE(9) XKB_CRT_CASE(10) XKB_CRT_CASE(11)
       XKB_CRT_CASE(12) XKB_CRT_CASE(13) XKB_CRT_CASE(14) XKB_CRT_CASE(15) XKB_CRT_CASE(16)
@@ -1171,14 +1480,13 @@ static const Consts* consts_for(int n) {
 }
 
 // Operand descriptor: an L x K "row" view (rows of op(A), or columns of
-// op(B)) of a real matrix, or of one part of a complex one.
+// op(B)) of a matrix.
 struct View {
-  const double* X;  // base (double units)
-  long ld;          // leading dimension in elements (complex: complex elements)
-  bool kc;          // k contiguous
-  long estride;     // 1 real, 2 complex
-  long eoff;        // 0 real part, 1 imaginary part
-  double sign;
+  const void* X;
+  long ld;    // leading dimension in elements
+  bool kc;    // k contiguous
+  int dtype;  // XKB_S .. XKB_Z
+  bool conj;
 };
 
 // Device words of one call: the moduli selection and the two concentration
@@ -1215,24 +1523,40 @@ static bool plan_moduli(int nmod, long K, ModPlan* pl) {
 
 // Row statistics of an L x K operand view: codes (k_oz_stat) and the
 // concentration maximum into *rmax.
-static int launch_norm(const View& v, int L, int K, int cplx, double4* part, int* code,
-                       unsigned* rmax, cudaStream_t st) {
-  const int nch = (K + kNormChunk - 1) / kNormChunk;
+template <class E>
+static void norm_kernel(const View& v, int L, int K, int cplx, double4* part, cudaStream_t st) {
+  const unsigned nch = (unsigned)((K + kNormChunk - 1) / kNormChunk);
+  const E* X = static_cast<const E*>(v.X);
+  if (v.kc)
+    k_oz_norm<true, E><<<dim3((unsigned)((L + 7) / 8), nch), 256, 0, st>>>(L, K, X, v.ld, cplx,
+                                                                           part);
+  else
+    k_oz_norm<false, E><<<dim3((unsigned)((L + 31) / 32), nch), 256, 0, st>>>(L, K, X, v.ld, cplx,
+                                                                              part);
+}
+static int launch_norm(const View& v, int L, int K, double4* part, int* code, unsigned* rmax,
+                       cudaStream_t st) {
+  const int cplx = v.dtype == XKB_C || v.dtype == XKB_Z;
+  const int exact = v.dtype == XKB_S || v.dtype == XKB_C;
   const long long tv = evlog_kern_begin(st, "k_oz_norm+k_oz_stat");
-  if (v.kc) {
-    dim3 g((unsigned)((L + 7) / 8), (unsigned)nch);
-    k_oz_norm<true><<<g, 256, 0, st>>>(L, K, v.X, v.ld, cplx, part);
-  } else {
-    dim3 g((unsigned)((L + 31) / 32), (unsigned)nch);
-    k_oz_norm<false><<<g, 256, 0, st>>>(L, K, v.X, v.ld, cplx, part);
-  }
-  k_oz_stat<<<(unsigned)((L + 255) / 256), 256, 0, st>>>(L, K, nch, part, code, rmax);
+  if (exact) norm_kernel<float>(v, L, K, cplx, part, st);
+  else norm_kernel<double>(v, L, K, cplx, part, st);
+  k_oz_stat<<<(unsigned)((L + 255) / 256), 256, 0, st>>>(
+      L, K, (K + kNormChunk - 1) / kNormChunk, part, code, rmax, exact);
   evlog_kern_end(tv, st);
   count_launch(2);
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
 }
 
-static int launch_pick(CallWords* w, const ModPlan& pl, bool allow_fallback, cudaStream_t st) {
+// Smallest complex moduli count whose P/4 holds |C'| <= 2^(2H).
+static int cplx_count(int H) {
+  for (int n = 2; n < kMaxC; ++n)
+    if (log2Pc(n) - 2.0 >= 2.0 * H) return n;
+  return kMaxC;
+}
+
+static int launch_pick(CallWords* w, const ModPlan& pl, bool allow_fallback, cudaStream_t st,
+                       bool cplx = false, bool exact = false) {
   PickP q;
   std::memset(&q, 0, sizeof(q));
   q.fixed = pl.fixed ? pl.hi : 0;
@@ -1243,6 +1567,13 @@ static int launch_pick(CallWords* w, const ModPlan& pl, bool allow_fallback, cud
     const Consts* c = consts_for(n);
     if (!c) return XKB_EINVAL;
     q.H[n] = c->H;
+    q.np[n] = cplx ? cplx_count(c->H) : n;
+  }
+  if (exact) {
+    q.exact = 1;
+    q.lo = cplx ? kExactLoC : kExactLo;
+    q.hi = cplx ? kMaxC : kMaxMod;
+    for (int n = 2; n <= q.hi; ++n) q.lim[n] = (float)((cplx ? log2Pc(n) : log2P(n)) - 2.01);
   }
   const long long tv = evlog_kern_begin(st, "k_oz_pick");
   k_oz_pick<<<1, 32, 0, st>>>(w->rmax, &w->sel, q);
@@ -1253,34 +1584,67 @@ static int launch_pick(CallWords* w, const ModPlan& pl, bool allow_fallback, cud
 
 // Residue planes 0 .. sel->n - 1 of an operand view (c: the constants of the
 // plan's largest count; the per-modulus constants are those of every count).
-static int launch_res(const View& v, int L, int K, const int* code, const OzSel* sel,
-                      const Consts* c, int8_t* planes, long Lpad, long Kpad, long kofs,
-                      cudaStream_t st, long grid_rows = 0) {
-  // grid covers Lpad (or grid_rows, for a block of rows of larger planes:
-  // planes stay Lpad rows apart) x (K rounded to 64); kofs places the block
-  // at column kofs; rows from L to the grid's end are written as zeros
-  dim3 g((unsigned)((grid_rows ? grid_rows : Lpad) / 64), (unsigned)(rup((size_t)K, 64) / 64));
-#define XKB_RES_CASE(NM)                                                                     \
-  case NM:                                                                                   \
-    if (v.kc)                                                                                \
-      k_oz_residues<true, NM><<<g, 256, 0, st>>>(L, K, v.X, v.ld, v.estride, v.eoff, v.sign, \
-                                                 code, sel, *c, planes, Lpad, Kpad, kofs);   \
-    else                                                                                     \
-      k_oz_residues<false, NM><<<g, 256, 0, st>>>(L, K, v.X, v.ld, v.estride, v.eoff,       \
-                                                  v.sign, code, sel, *c, planes, Lpad, Kpad, \
-                                                  kofs);                                     \
-    break;
-  if (c->nmod < 2 || c->nmod > kMaxMod) return XKB_EINVAL;
-  const long long tv = evlog_kern_begin(st, "k_oz_residues");
-  switch (c->nmod) {
-    XKB_RES_CASE(2) XKB_RES_CASE(3) XKB_RES_CASE(4) XKB_RES_CASE(5) XKB_RES_CASE(6)
-    XKB_RES_CASE(7) XKB_RES_CASE(8) XKB_RES_CASE(9) XKB_RES_CASE(10) XKB_RES_CASE(11)
-    XKB_RES_CASE(12) XKB_RES_CASE(13) XKB_RES_CASE(14) XKB_RES_CASE(15) XKB_RES_CASE(16)
-    default: break;
-  }
+template <class E>
+static int res_real(const View& v, int L, int K, const int* code, const OzSel* sel,
+                    const Consts* c, int8_t* planes, long Lpad, long Kpad, long rows,
+                    cudaStream_t st) {
+  const dim3 g((unsigned)(rows / 64), (unsigned)(rup((size_t)K, 64) / 64));
+  const E* X = static_cast<const E*>(v.X);
+  const auto go = [&](auto nm) {
+    constexpr int NM = decltype(nm)::value;
+    if (v.kc)
+      k_oz_residues<true, NM, E><<<g, 256, 0, st>>>(L, K, X, v.ld, code, sel, *c, planes, Lpad,
+                                                    Kpad);
+    else
+      k_oz_residues<false, NM, E><<<g, 256, 0, st>>>(L, K, X, v.ld, code, sel, *c, planes, Lpad,
+                                                     Kpad);
+  };
+  if constexpr (sizeof(E) == 4) {  // exact products plan for every count
+    go(std::integral_constant<int, kMaxMod>());
+    return XKB_OK;
+  } else {
+    switch (c->nmod) {
+#define XKB_RES_CASE(NM) \
+  case NM: go(std::integral_constant<int, NM>()); return XKB_OK;
+      XKB_RES_CASE(2) XKB_RES_CASE(3) XKB_RES_CASE(4) XKB_RES_CASE(5) XKB_RES_CASE(6)
+      XKB_RES_CASE(7) XKB_RES_CASE(8) XKB_RES_CASE(9) XKB_RES_CASE(10) XKB_RES_CASE(11)
+      XKB_RES_CASE(12) XKB_RES_CASE(13) XKB_RES_CASE(14) XKB_RES_CASE(15) XKB_RES_CASE(16)
 #undef XKB_RES_CASE
+      default: return XKB_EINVAL;
+    }
+  }
+}
+template <class E>
+static void res_cplx(const View& v, int L, int K, const int* code, const OzSel* sel,
+                     int8_t* planes, long Lpad, long Kpad, cudaStream_t st) {
+  const dim3 g((unsigned)(Lpad / 64), (unsigned)(Kpad / 32));
+  const E* X = static_cast<const E*>(v.X);
+  const double sign = v.conj ? -1.0 : 1.0;
+  if (v.kc)
+    k_oz_residues_c<true, E><<<g, 256, 0, st>>>(L, K, X, v.ld, sign, code, sel, cres_consts(),
+                                                planes, Lpad, Kpad);
+  else
+    k_oz_residues_c<false, E><<<g, 256, 0, st>>>(L, K, X, v.ld, sign, code, sel, cres_consts(),
+                                                 planes, Lpad, Kpad);
+}
+static int launch_res(const View& v, int L, int K, const int* code, const OzSel* sel,
+                      const Consts* c, int8_t* planes, long Lpad, long Kpad, cudaStream_t st,
+                      long grid_rows = 0) {
+  // grid covers Lpad (or grid_rows, for a block of rows of larger planes:
+  // planes stay Lpad rows apart) x (K rounded to 64; complex: Kpad); rows
+  // from L to the grid's end are written as zeros
+  const long rows = grid_rows ? grid_rows : Lpad;
+  const long long tv = evlog_kern_begin(st, "k_oz_residues");
+  int e = XKB_OK;
+  switch (v.dtype) {
+    case XKB_S: e = res_real<float>(v, L, K, code, sel, c, planes, Lpad, Kpad, rows, st); break;
+    case XKB_D: e = res_real<double>(v, L, K, code, sel, c, planes, Lpad, Kpad, rows, st); break;
+    case XKB_C: res_cplx<float>(v, L, K, code, sel, planes, Lpad, Kpad, st); break;
+    default: res_cplx<double>(v, L, K, code, sel, planes, Lpad, Kpad, st); break;
+  }
   evlog_kern_end(tv, st);
   count_launch();
+  if (e) return e;
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
 }
 
@@ -1294,20 +1658,25 @@ static bool encode_planes(CUtensorMap* m, const int8_t* base, long Kpad, long Lp
 // Npad; equal when one buffer serves both operands).  a_stride / b_stride
 // (0: the same): rows between consecutive planes, when Ap / Bp point at a
 // block of rows of larger planes.
+// c: the plan's largest count; null: a complex product, 2 kMaxC planes
+// (bxor: see GemmP).
 static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_rows, long Mpad,
                        long Npad, long Kpad, const Consts* c, const OzSel* sel, uint8_t* R,
                        int uplo, long diag, cudaStream_t st, long a_stride = 0,
-                       long b_stride = 0) {
+                       long b_stride = 0, int bxor = 0) {
   CUtensorMap tA, tB;
+  const int npl = c ? c->nmod : 2 * kMaxC;
   if (a_rows < Mpad || b_rows < Npad) return XKB_EINVAL;
-  if (!encode_planes(&tA, Ap, Kpad, a_rows, c->nmod, BM, a_stride)) return XKB_EINVAL;
-  if (!encode_planes(&tB, Bp, Kpad, b_rows, c->nmod, BN, b_stride)) return XKB_EINVAL;
+  if (!encode_planes(&tA, Ap, Kpad, a_rows, npl, BM, a_stride)) return XKB_EINVAL;
+  if (!encode_planes(&tB, Bp, Kpad, b_rows, npl, BN, b_stride)) return XKB_EINVAL;
   GemmP p;
   std::memset(&p, 0, sizeof(p));
+  p.mult = c ? 1 : 2;
+  p.bxor = bxor;
   p.tiles_m = (int)(Mpad / BM);
   p.tiles_n = (int)(Npad / BN);
   p.kblocks = (int)(Kpad / BKB);
-  p.nmod = c->nmod;
+  p.nmod = npl;
   p.sel = sel;
   // raster group (tuning table oz_group_m, default 8 M tiles)
   p.group = std::max(1, std::min(p.tiles_m, (int)tune("oz_group_m", 8.0)));
@@ -1316,18 +1685,18 @@ static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_r
   p.Npad = Npad;
   p.uplo = uplo;
   p.diag = diag;
-  for (int m = 0; m < c->nmod; ++m) {
-    p.p[m] = c->p[m];
-    p.magic[m] = c->magic[m];
-    p.bias[m] = (uint32_t)(((1ull << 31) + (uint64_t)c->p[m] - 1) / (uint64_t)c->p[m]) *
-                (uint32_t)c->p[m];
+  for (int m = 0; m < npl; ++m) {
+    const uint32_t q = (uint32_t)(c ? c->p[m] : kCMod[m / 2]);
+    p.p[m] = (int)q;
+    p.magic[m] = (uint32_t)(((1ull << 32) + q - 1) / q);
+    p.bias[m] = (uint32_t)(((1ull << 31) + q - 1) / q) * q;
   }
   const long total2 = (Mpad % BM2 == 0 && Npad % BN2 == 0)
-                         ? (Mpad / BM2) * (Npad / BN2) * (long)c->nmod : 0;
+                         ? (Mpad / BM2) * (Npad / BN2) * (long)npl : 0;
   if (total2 > 0 && tune("oz_2cta", 0.0) != 0.0 && sm_count() >= 2) {
     // CTA pairs: 256 x 256 tiles, each CTA loading 128-row halves of A and B
     CUtensorMap tB2;
-    if (!encode_planes(&tB2, Bp, Kpad, b_rows, c->nmod, 128, b_stride)) return XKB_EINVAL;
+    if (!encode_planes(&tB2, Bp, Kpad, b_rows, npl, 128, b_stride)) return XKB_EINVAL;
     p.tiles_m = (int)(Mpad / BM2);
     p.tiles_n = (int)(Npad / BN2);
     p.group = std::max(1, std::min(p.tiles_m, (int)tune("oz_group_m", 8.0)));
@@ -1368,7 +1737,7 @@ static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_r
       return XKB_ECUDA;
     attr = true;
   }
-  const long total = (long)p.tiles_m * p.tiles_n * c->nmod;
+  const long total = (long)p.tiles_m * p.tiles_n * npl;
   const unsigned grid = (unsigned)std::min<long>(total, sm_count());  // persistent
   const long long tv = evlog_kern_begin(st, "k_oz_gemm");
   k_oz_gemm<<<grid, kGemmThreads, smem, st>>>(tA, tB, p);
@@ -1426,52 +1795,46 @@ extern "C" int xkb_ozaki_counts(unsigned long long* out, int* last, int reset) {
 // least the tuning table's count for K's band); operands whose spread 16
 // moduli cannot carry to FP64 accuracy are computed by the plain FP64
 // kernel instead, launched here and predicated on the device's choice.
+// Single precision (S, C): the exact product or the plain kernel.
 // Scratch (stream-ordered, from the pool): residue planes of op(A) and
 // op(B) for the largest count the call may use (nmod x Mpad x Kpad,
-// nmod x Npad x Kpad int8), residue planes of C (nmod x Mpad x Npad uint8),
-// row codes, norm partials and the call's device words.
-extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* stream) {
-  if (!a || (a->dtype != XKB_D && a->dtype != XKB_Z)) return XKB_EINVAL;
-  if (a->M < 0 || a->N < 0 || a->K < 0) return XKB_EINVAL;
-  if (a->M == 0 || a->N == 0) return XKB_OK;
-  const bool cplx = a->dtype == XKB_Z;
+// nmod x Npad x Kpad int8; complex 34 planes), residue planes of C (as many
+// Mpad x Npad uint8), row codes, norm partials and the call's device words.
+static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
+  const bool cplx = a->dtype == XKB_Z || a->dtype == XKB_C;
+  const bool exact = a->dtype == XKB_S || a->dtype == XKB_C;
   const long Keff = cplx ? 2L * a->K : (long)a->K;
-  if (a->K == 0 || (a->alpha[0] == 0.0 && a->alpha[1] == 0.0))
-    return xkb_cuda_gemm(a, stream);
   if (Keff > 131072) return XKB_ERANGE;
   ModPlan pl;
-  if (!plan_moduli(nmod, Keff, &pl)) return XKB_ERANGE;
-  const int nmax = pl.hi;
-  cudaStream_t st = resolve_stream(stream);
+  if (!plan_moduli(exact ? kMaxMod : nmod, Keff, &pl)) return XKB_ERANGE;
+  const int nmax = cplx ? kMaxPl : pl.hi;  // planes
+  const Consts* c = cplx ? nullptr : pl.chi;
   const int M = a->M, N = a->N, K = a->K;
-  // complex operands are laid out [Re | pad | Im | pad] along k, each block
-  // starting on a 64-column boundary (aligned 4-byte stores in the residue
-  // kernel); the zero pads contribute nothing to the products
-  const long kofs2 = (long)rup(K, 64);
-  const long Kpad = cplx ? (long)rup(2 * kofs2, BKB) : (long)rup(K, BKB);
+  const long Kpad = (long)rup(K, BKB);
   const long Mpad = (long)rup(M, BM2), Npad = (long)rup(N, BN);  // BM2: CTA-pair tiles
   const bool akc = a->opA != XKB_OP_N, bkc = a->opB == XKB_OP_N;
-  // C = A A^T (or A^T A): op(B)^T's rows are op(A)'s rows, one residue buffer
-  // serves both operands; it then holds max(Mpad, Npad) rows per plane
-  const bool same = (a->A == a->B) && (a->lda == a->ldb) && (akc == bkc) && !cplx && M == N;
+  const bool cA = a->opA == XKB_OP_C, cB = a->opB == XKB_OP_C;
+  // C = A A^T or A A^H (or A^T A, A^H A): op(B)^T's rows are op(A)'s rows or,
+  // complex, their conjugates (whose planes are op(A)'s, each pair swapped),
+  // so one residue buffer serves both operands; it then holds
+  // max(Mpad, Npad) rows per plane
+  const bool same = (a->A == a->B) && (a->lda == a->ldb) && (akc == bkc) && M == N;
+  const int bxor = cplx && same && cA != cB ? 1 : 0;
   const long Arows = same ? std::max(Mpad, Npad) : Mpad;
-  const size_t szA = (size_t)nmax * Arows * Kpad, szB = (size_t)nmax * Npad * Kpad;
+  const size_t szA = (size_t)nmax * Arows * Kpad, szB = same ? 0 : (size_t)nmax * Npad * Kpad;
   const size_t szR = (size_t)nmax * Mpad * Npad;
-  const int nch = (int)((Keff + kNormChunk - 1) / kNormChunk);
+  const int nch = (K + kNormChunk - 1) / kNormChunk;
   const size_t szPart = 256 + sizeof(double4) * (size_t)nch * (size_t)std::max(M, N) * 2;
-  const size_t szRe = cplx ? sizeof(double) * (size_t)M * N : 0;
   int8_t *Ap = nullptr, *Bp = nullptr;
   uint8_t* R = nullptr;
   int *mu = nullptr, *nu = nullptr;
   unsigned char* pw = nullptr;  // CallWords, then the norm partials from byte 256
-  double* re = nullptr;
   auto alloc = [&](void** p, size_t n) {
     return cudaMallocAsync(p, std::max<size_t>(n, 256), st) == cudaSuccess;
   };
-  bool ok = alloc((void**)&Ap, szA) && alloc((void**)&Bp, cplx ? 2 * szB : szB) &&
+  bool ok = alloc((void**)&Ap, szA) && (same || alloc((void**)&Bp, szB)) &&
             alloc((void**)&R, szR) && alloc((void**)&mu, sizeof(int) * M) &&
-            alloc((void**)&nu, sizeof(int) * N) && alloc((void**)&pw, szPart) &&
-            (!cplx || alloc((void**)&re, szRe));
+            alloc((void**)&nu, sizeof(int) * N) && alloc((void**)&pw, szPart);
   int err = ok ? XKB_OK : XKB_ENOMEM;
   if (!ok) cudaGetLastError();
   CallWords* w = reinterpret_cast<CallWords*>(pw);
@@ -1482,102 +1845,73 @@ extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* strea
   //                else     -> A is K x M, row i = A[k + i*lda] (k contiguous)
   // columns of op(B): opB == N -> B is K x N, col j = B[k + j*ldb] (k contig.)
   //                   else     -> B is N x K, col j = B[j + k*ldb]
-  const double* Ad = static_cast<const double*>(a->A);
-  const double* Bd = static_cast<const double*>(a->B);
-  const double sa = (a->opA == XKB_OP_C) ? -1.0 : 1.0;  // conj: negate Im
-  const double sb = (a->opB == XKB_OP_C) ? -1.0 : 1.0;
-  const int slot = trace_begin("ozaki_gemm", a->dtype, M, N, K, pl.fixed ? nmax : 0, st);
-  if (err == XKB_OK) {
-    // scaling: complex rows use the norm over (re, im) = the concatenated row
-    View va{Ad, a->lda, akc, 1, 0, 1.0}, vb{Bd, a->ldb, bkc, 1, 0, 1.0};
-    if (cudaMemsetAsync(w, 0, sizeof(CallWords), st) != cudaSuccess) err = XKB_ECUDA;
-    if (!err) err = launch_norm(va, M, K, cplx, part, mu, &w->rmax[0], st);
-    if (!err)
-      err = launch_norm(vb, N, K, cplx, part + (size_t)nch * std::max(M, N), nu, &w->rmax[1], st);
-    if (!err) err = launch_pick(w, pl, !pl.fixed, st);
+  // (complex: the norm of a row is over its real and imaginary parts)
+  const View va{a->A, a->lda, akc, a->dtype, cA}, vb{a->B, a->ldb, bkc, a->dtype, cB};
+  const int slot = trace_begin("ozaki_gemm", a->dtype, M, N, K, pl.fixed ? pl.hi : 0, st);
+  if (!err && cudaMemsetAsync(w, 0, sizeof(CallWords), st) != cudaSuccess) err = XKB_ECUDA;
+  if (!err) err = launch_norm(va, M, K, part, mu, &w->rmax[0], st);
+  if (!err)
+    err = launch_norm(vb, N, K, part + (size_t)nch * std::max(M, N), nu, &w->rmax[1], st);
+  if (!err) err = launch_pick(w, pl, !pl.fixed, st, cplx, exact);
+  if (!err) err = launch_res(va, M, K, mu, sel, pl.chi, Ap, Arows, Kpad, st);
+  if (!err && !same) err = launch_res(vb, N, K, nu, sel, pl.chi, Bp, Npad, Kpad, st);
+  if (!err && !cplx && Kpad > (long)rup(K, 64)) {
+    // zero the k padding beyond the last 64-column block
+    const size_t kz = rup(K, 64);
+    if (cudaMemset2DAsync(Ap + kz, Kpad, 0, Kpad - kz, (size_t)nmax * Arows, st) != cudaSuccess ||
+        (!same &&
+         cudaMemset2DAsync(Bp + kz, Kpad, 0, Kpad - kz, (size_t)nmax * Npad, st) != cudaSuccess))
+      err = XKB_ECUDA;
   }
-  if (err == XKB_OK) {
-    if (!cplx) {
-      View va{Ad, a->lda, akc, 1, 0, 1.0}, vb{Bd, a->ldb, bkc, 1, 0, 1.0};
-      err = launch_res(va, M, K, mu, sel, pl.chi, Ap, Arows, Kpad, 0, st);
-      if (!err && !same) err = launch_res(vb, N, K, nu, sel, pl.chi, Bp, Npad, Kpad, 0, st);
-      if (!err && Kpad > (long)rup(K, 64)) {
-        // zero the k padding beyond the last 64-column block
-        const size_t kz = rup(K, 64);
-        err = cudaMemset2DAsync(Ap + kz, Kpad, 0, Kpad - kz, (size_t)nmax * Arows, st) == cudaSuccess
-                  ? XKB_OK : XKB_ECUDA;
-        if (!err && !same)
-          err = cudaMemset2DAsync(Bp + kz, Kpad, 0, Kpad - kz, (size_t)nmax * Npad, st) == cudaSuccess
-                    ? XKB_OK : XKB_ECUDA;
-      }
-    } else {
-      // A' = [Re op(A) | Im op(A)] (K' = 2K);  B1 = [Re op(B); -Im op(B)],
-      // B2 = [Im op(B); Re op(B)]:  Re(AB) = A' B1,  Im(AB) = A' B2.
-      View ar{Ad, a->lda, akc, 2, 0, 1.0}, ai{Ad, a->lda, akc, 2, 1, sa};
-      View br{Bd, a->ldb, bkc, 2, 0, 1.0}, bi{Bd, a->ldb, bkc, 2, 1, sb};
-      View bin{Bd, a->ldb, bkc, 2, 1, -sb};
-      int8_t* B1 = Bp;
-      int8_t* B2 = Bp + szB;
-      err = launch_res(ar, M, K, mu, sel, pl.chi, Ap, Mpad, Kpad, 0, st);
-      if (!err) err = launch_res(ai, M, K, mu, sel, pl.chi, Ap, Mpad, Kpad, kofs2, st);
-      if (!err) err = launch_res(br, N, K, nu, sel, pl.chi, B1, Npad, Kpad, 0, st);
-      if (!err) err = launch_res(bin, N, K, nu, sel, pl.chi, B1, Npad, Kpad, kofs2, st);
-      if (!err) err = launch_res(bi, N, K, nu, sel, pl.chi, B2, Npad, Kpad, 0, st);
-      if (!err) err = launch_res(br, N, K, nu, sel, pl.chi, B2, Npad, Kpad, kofs2, st);
-      if (!err && Kpad > 2 * kofs2) {
-        const size_t kz = 2 * (size_t)kofs2;
-        if (cudaMemset2DAsync(Ap + kz, Kpad, 0, Kpad - kz, (size_t)nmax * Mpad, st) != cudaSuccess ||
-            cudaMemset2DAsync(Bp + kz, Kpad, 0, Kpad - kz, (size_t)2 * nmax * Npad, st) != cudaSuccess)
-          err = XKB_ECUDA;
-      }
-    }
-  }
-  CrtP cp;
-  std::memset(&cp, 0, sizeof(cp));
-  cp.M = M;
-  cp.N = N;
-  cp.R = R;
-  cp.Mpad = Mpad;
-  cp.Npad = Npad;
-  cp.mu = mu;
-  cp.nu = nu;
-  cp.sel = sel;
-  cp.C = static_cast<double*>(a->C);
-  cp.ldc = a->ldc;
-  cp.cplx = cplx;
-  cp.ar = a->alpha[0];
-  cp.ai = cplx ? a->alpha[1] : 0.0;
-  cp.br = a->beta[0];
-  cp.bi = cplx ? a->beta[1] : 0.0;
-  cp.uplo = a->uplo;
-  cp.herm_diag = a->herm_diag;
-  cp.diag = a->diag;
   trace_mark(slot, 1, st);
-  if (err == XKB_OK) {
-    err = same ? launch_gemm(Ap, Arows, Ap, Arows, Mpad, Npad, Kpad, pl.chi, sel, R, a->uplo,
-                             a->diag, st)
-               : launch_gemm(Ap, Mpad, Bp, Npad, Mpad, Npad, Kpad, pl.chi, sel, R, a->uplo,
-                             a->diag, st);
-    if (!err) {
-      if (!cplx) {
-        trace_mark(slot, 2, st);
-        err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
+  if (!err)
+    err = launch_gemm(Ap, Arows, same ? Ap : Bp, same ? Arows : Npad, Mpad, Npad, Kpad, c, sel, R,
+                      a->uplo, a->diag, st, 0, 0, bxor);
+  trace_mark(slot, 2, st);
+  if (!err) {
+    CrtP cp;
+    std::memset(&cp, 0, sizeof(cp));
+    cp.M = M;
+    cp.N = N;
+    cp.R = R;
+    cp.Mpad = Mpad;
+    cp.Npad = Npad;
+    cp.mu = mu;
+    cp.nu = nu;
+    cp.sel = sel;
+    cp.C = a->C;
+    cp.ldc = a->ldc;
+    cp.ar = a->alpha[0];
+    cp.ai = cplx ? a->alpha[1] : 0.0;
+    cp.br = a->beta[0];
+    cp.bi = cplx ? a->beta[1] : 0.0;
+    cp.uplo = a->uplo;
+    cp.herm_diag = a->herm_diag;
+    cp.diag = a->diag;
+    if (a->dtype == XKB_D) {
+      err = launch_crt(st, cp, pl.clo, pl.chi);
+    } else {
+      const long long tv = evlog_kern_begin(st, "k_oz_crt");
+      const unsigned gy = (unsigned)((N + kCrtCols - 1) / kCrtCols);
+      const unsigned gr = (unsigned)((M + kCrtRows - 1) / kCrtRows);
+      const unsigned gc = (unsigned)((M + kCrtRowsC - 1) / kCrtRowsC);
+      if (a->dtype == XKB_S) {
+        CrtTabS t;
+        for (int n = kExactLo; n <= kMaxMod; ++n) t.c[n - kExactLo] = *consts_for(n);
+        k_oz_crt_s<<<dim3(gr, gy), 256, 0, st>>>(cp, t);
+      } else if (a->dtype == XKB_C) {
+        k_oz_crt_c<float><<<dim3(gc, gy), 256, 0, st>>>(cp, ccrt_tab());
       } else {
-        err = launch_crt(st, cp, pl.clo, pl.chi, re);
-        if (!err)
-          err = launch_gemm(Ap, Mpad, Bp + szB, Npad, Mpad, Npad, Kpad, pl.chi, sel, R, a->uplo,
-                            a->diag, st);
-        trace_mark(slot, 2, st);
-        if (!err) {
-          cp.other = re;
-          err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
-        }
+        k_oz_crt_c<double><<<dim3(gc, gy), 256, 0, st>>>(cp, ccrt_tab());
       }
+      evlog_kern_end(tv, st);
+      count_launch();
+      if (cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
     }
-    // the data rule may have sent the call to the plain FP64 kernel
-    if (!err && !pl.fixed) err = gemm_if(a, &w->sel.fallback, st);
-    if (!err && cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
   }
+  // the device may have sent the call to the plain FP64 kernel
+  if (!err && (exact || !pl.fixed)) err = gemm_if(a, &w->sel.fallback, st);
+  if (!err && cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
   trace_mark(slot, 3, st);
   if (Ap) cudaFreeAsync(Ap, st);
   if (Bp) cudaFreeAsync(Bp, st);
@@ -1585,9 +1919,39 @@ extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* strea
   if (mu) cudaFreeAsync(mu, st);
   if (nu) cudaFreeAsync(nu, st);
   if (pw) cudaFreeAsync(pw, st);
-  if (re) cudaFreeAsync(re, st);
   return err;
 }
+
+extern "C" int xkb_cuda_ozaki_gemm(const xkb_gemm_args* a, int nmod, void* stream) {
+  if (!a || (a->dtype != XKB_D && a->dtype != XKB_Z)) return XKB_EINVAL;
+  if (a->M < 0 || a->N < 0 || a->K < 0) return XKB_EINVAL;
+  if (a->M == 0 || a->N == 0) return XKB_OK;
+  if (a->K == 0 || (a->alpha[0] == 0.0 && a->alpha[1] == 0.0))
+    return xkb_cuda_gemm(a, stream);
+  return oz_run(a, nmod, resolve_stream(stream));
+}
+
+namespace xkb {
+// The exact form of a large single-precision product (S, C): FP64 work would
+// leave the INT8 tensor cores idle.  Whether the operands allow it is decided
+// on the device (k_oz_pick), else the plain kernel runs within the same call.
+// XKB_ERANGE: not taken for this shape, XKB_ENOMEM: no scratch; the caller
+// then runs the plain kernel.  Taken from M N K = 3.4e9 on (C: a quarter of
+// it).  Measured (B200, us, plain -> exact): S 1024^3 76 -> 108, 1500^3 214 ->
+// 184, 2048^3 527 -> 270, 4096^3 3978 -> 1042 (error against 64 bits 2.53e-8,
+// the final rounding, on both); C 1024^3 258 -> 209, 2048^3 1976 -> 489.
+int gemm_exact(const xkb_gemm_args* a, cudaStream_t st) {
+  const bool cplx = a->dtype == XKB_C;
+  const double mn = std::min(a->M, a->N);
+  if (tune("gemm_exact", 1.0) == 0.0 || mn < 512 || a->K < 512 ||
+      (double)a->M * a->N * a->K * (cplx ? 4.0 : 1.0) < tune("gemm_exact_min", 3.4e9))
+    return XKB_ERANGE;
+  const double planes = cplx ? kMaxPl : kMaxMod;
+  if (planes * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N) > 17.2e9)
+    return XKB_ERANGE;  // at most 16 GiB of scratch
+  return oz_run(a, 0, st);
+}
+}  // namespace xkb
 
 // ===========================================================================
 // Column-panel form of the real contraction, for callers that move op(B)
@@ -1659,11 +2023,11 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
   const double* Bd = static_cast<const double*>(a->B);
   const int slot = trace_begin("ozaki_panels", a->dtype, M, a->N, K, nmod, st);
   if (!err) {
-    View va{Ad, a->lda, akc, 1, 0, 1.0};
+    View va{Ad, a->lda, akc, XKB_D, false};
     if (cudaMemsetAsync(w, 0, sizeof(CallWords), st) != cudaSuccess) err = XKB_ECUDA;
-    if (!err) err = launch_norm(va, M, K, 0, part, mu, &w->rmax[0], st);
+    if (!err) err = launch_norm(va, M, K, part, mu, &w->rmax[0], st);
     if (!err) err = launch_pick(w, pl, false, st);
-    if (!err) err = launch_res(va, M, K, mu, sel, c, Ap, Mpad, Kpad, 0, st);
+    if (!err) err = launch_res(va, M, K, mu, sel, c, Ap, Mpad, Kpad, st);
     if (!err && Kpad > (long)rup(K, 64)) {
       const size_t kz = rup(K, 64);
       if (cudaMemset2DAsync(Ap + kz, Kpad, 0, Kpad - kz, (size_t)nmod * Mpad, st) != cudaSuccess)
@@ -1677,9 +2041,9 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
     const long npad = (long)rup((size_t)nw, BN);
     if (!err) {
       // columns n0.. of op(B): opB == N -> B[k + j ldb]; else B[j + k ldb]
-      View vb{bkc ? Bd + n0 * a->ldb : Bd + n0, a->ldb, bkc, 1, 0, 1.0};
-      err = launch_norm(vb, (int)nw, K, 0, part, nu + n0, &w->rmax[1], st);
-      if (!err) err = launch_res(vb, (int)nw, K, nu + n0, sel, c, Bp, npad, Kpad, 0, st);
+      View vb{bkc ? Bd + n0 * a->ldb : Bd + n0, a->ldb, bkc, XKB_D, false};
+      err = launch_norm(vb, (int)nw, K, part, nu + n0, &w->rmax[1], st);
+      if (!err) err = launch_res(vb, (int)nw, K, nu + n0, sel, c, Bp, npad, Kpad, st);
       if (!err && Kpad > (long)rup(K, 64)) {
         const size_t kz = rup(K, 64);
         if (cudaMemset2DAsync(Bp + kz, Kpad, 0, Kpad - kz, (size_t)nmod * npad, st) != cudaSuccess)
@@ -1703,7 +2067,7 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
         cp.ar = a->alpha[0];
         cp.br = a->beta[0];
         cp.uplo = XKB_FULL;
-        err = launch_crt(st, cp, c, c, nullptr);
+        err = launch_crt(st, cp, c, c);
       }
     }
     done(q);  // recorded on every path: waiters never hang on an error
@@ -1827,11 +2191,11 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
       c1 = cb[cn];
       if (!err) {
         // rows r0.. of op(A): opA == N -> A[i + k lda]; else A[k + i lda]
-        View va{akc ? Ad + r0 * a->lda : Ad + r0, a->lda, akc, 1, 0, 1.0};
+        View va{akc ? Ad + r0 * a->lda : Ad + r0, a->lda, akc, XKB_D, false};
         const int L = (int)(r1 - r0);
-        err = launch_norm(va, L, K, 0, part, mu + r0, &w->rmax[0], st);
+        err = launch_norm(va, L, K, part, mu + r0, &w->rmax[0], st);
         if (!err)
-          err = launch_res(va, L, K, mu + r0, sel, c, Ap + r0 * Kpad, Mpad, Kpad, 0, st,
+          err = launch_res(va, L, K, mu + r0, sel, c, Ap + r0 * Kpad, Mpad, Kpad, st,
                            (long)rup((size_t)L, 64));
       }
       ++ra;
@@ -1844,11 +2208,11 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
       c1 = cb[j + 1];
       if (!err) {
         // columns c0.. of op(B): opB == N -> B[k + j ldb]; else B[j + k ldb]
-        View vb{bkc ? Bd + c0 * a->ldb : Bd + c0, a->ldb, bkc, 1, 0, 1.0};
+        View vb{bkc ? Bd + c0 * a->ldb : Bd + c0, a->ldb, bkc, XKB_D, false};
         const int L = (int)(c1 - c0);
-        err = launch_norm(vb, L, K, 0, part, nu + c0, &w->rmax[1], st);
+        err = launch_norm(vb, L, K, part, nu + c0, &w->rmax[1], st);
         if (!err)
-          err = launch_res(vb, L, K, nu + c0, sel, c, Bp + c0 * Kpad, Npad, Kpad, 0, st,
+          err = launch_res(vb, L, K, nu + c0, sel, c, Bp + c0 * Kpad, Npad, Kpad, st,
                            (long)rup((size_t)L, 64));
       }
       ++cn;
@@ -1873,7 +2237,7 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
         cp.ar = a->alpha[0];
         cp.br = a->beta[0];
         cp.uplo = XKB_FULL;
-        err = launch_crt(st, cp, c, c, nullptr);
+        err = launch_crt(st, cp, c, c);
       }
     }
     done(k);  // recorded on every path: waiters never hang on an error
@@ -1990,14 +2354,14 @@ static unsigned long long current_ctx_id() {
 template <int NM>
 static bool load_nm_kernels() {
   cudaFuncAttributes fa;
-  return cudaFuncGetAttributes(&fa, k_oz_residues<true, NM>) == cudaSuccess &&
-         cudaFuncGetAttributes(&fa, k_oz_residues<false, NM>) == cudaSuccess &&
+  return cudaFuncGetAttributes(&fa, k_oz_residues<true, NM, double>) == cudaSuccess &&
+         cudaFuncGetAttributes(&fa, k_oz_residues<false, NM, double>) == cudaSuccess &&
          cudaFuncGetAttributes(&fa, k_oz_crt<NM>) == cudaSuccess;
 }
 static bool load_noalloc_kernels() {
   cudaFuncAttributes fa;
-  bool ok = cudaFuncGetAttributes(&fa, k_oz_norm<true>) == cudaSuccess &&
-            cudaFuncGetAttributes(&fa, k_oz_norm<false>) == cudaSuccess &&
+  bool ok = cudaFuncGetAttributes(&fa, k_oz_norm<true, double>) == cudaSuccess &&
+            cudaFuncGetAttributes(&fa, k_oz_norm<false, double>) == cudaSuccess &&
             cudaFuncGetAttributes(&fa, k_oz_stat) == cudaSuccess &&
             cudaFuncGetAttributes(&fa, k_oz_pick) == cudaSuccess &&
             cudaFuncGetAttributes(&fa, k_oz_crt_15_16) == cudaSuccess &&
@@ -2090,13 +2454,13 @@ extern "C" int xkb_cuda_ozaki_gemm_noalloc(const xkb_gemm_args* a, int nmod, voi
   const double* Ad = static_cast<const double*>(a->A);
   const double* Bd = static_cast<const double*>(a->B);
   const int slot = trace_begin("ozaki_noalloc", a->dtype, M, N, K, pl.fixed ? nmod : 0, st);
-  View va{Ad, a->lda, akc, 1, 0, 1.0}, vb{Bd, a->ldb, bkc, 1, 0, 1.0};
+  View va{Ad, a->lda, akc, XKB_D, false}, vb{Bd, a->ldb, bkc, XKB_D, false};
   if (cudaMemsetAsync(w, 0, sizeof(CallWords), st) != cudaSuccess) err = XKB_ECUDA;
-  if (!err) err = launch_norm(va, M, K, 0, part, mu, &w->rmax[0], st);
-  if (!err) err = launch_norm(vb, N, K, 0, part + kNoAllocRows, nu, &w->rmax[1], st);
+  if (!err) err = launch_norm(va, M, K, part, mu, &w->rmax[0], st);
+  if (!err) err = launch_norm(vb, N, K, part + kNoAllocRows, nu, &w->rmax[1], st);
   if (!err) err = launch_pick(w, pl, false, st);
-  if (!err) err = launch_res(va, M, K, mu, sel, c, Ap, Arows, Kpad, 0, st);
-  if (!err && !same) err = launch_res(vb, N, K, nu, sel, c, Bp, Npad, Kpad, 0, st);
+  if (!err) err = launch_res(va, M, K, mu, sel, c, Ap, Arows, Kpad, st);
+  if (!err && !same) err = launch_res(vb, N, K, nu, sel, c, Bp, Npad, Kpad, st);
   if (!err && Kpad > (long)rup(K, 64)) {
     const size_t kz = rup(K, 64);
     if (cudaMemset2DAsync(Ap + kz, Kpad, 0, Kpad - kz, (size_t)nmod * Arows, st) != cudaSuccess ||
@@ -2122,13 +2486,13 @@ extern "C" int xkb_cuda_ozaki_gemm_noalloc(const xkb_gemm_args* a, int nmod, voi
     cp.mu = mu;
     cp.nu = nu;
     cp.sel = sel;
-    cp.C = static_cast<double*>(a->C);
+    cp.C = a->C;
     cp.ldc = a->ldc;
     cp.ar = a->alpha[0];
     cp.br = a->beta[0];
     cp.uplo = a->uplo;
     cp.diag = a->diag;
-    err = launch_crt(st, cp, pl.clo, pl.chi, nullptr);
+    err = launch_crt(st, cp, pl.clo, pl.chi);
   }
   trace_mark(slot, 3, st);
   return err;

@@ -171,6 +171,9 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
 // xkb_cuda_gemm whose kernel runs only where the device word *run_if is
 // non-zero (gemm_dmma.cu): the plain fallback of a data-chosen Ozaki call.
 int gemm_if(const xkb_gemm_args* a, const int* run_if, cudaStream_t st);
+// A large single-precision product by exact INT8 arithmetic (ozaki.cu);
+// XKB_ERANGE / XKB_ENOMEM: not taken, nothing was launched.
+int gemm_exact(const xkb_gemm_args* a, cudaStream_t st);
 double tune(const char* key, double dflt);   // tuning table (runtime_cuda.cu)
 int tune_band(const char* prefix, long K);
 int sm_count();
