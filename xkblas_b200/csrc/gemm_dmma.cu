@@ -163,6 +163,10 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
     return run_if ? XKB_EINVAL
                   : xkb_cuda_scale(a->dtype, a->M, a->N, a->beta, a->C, a->ldc, a->uplo,
                                    a->herm_diag, a->diag, st);
+  if (!run_if && (a->dtype == XKB_S || a->dtype == XKB_C)) {
+    const int e = gemm_exact(a, st);
+    if (e != XKB_ERANGE && e != XKB_ENOMEM) return e;
+  }
   const int slot = trace_begin(run_if ? "dmma_fallback" : "dmma_gemm", a->dtype, a->M, a->N,
                                a->K, 0, st);
   trace_mark(slot, 1, st);

@@ -58,7 +58,6 @@ struct Consts {
   // bits of w from 2^csplit up (exact double, <= 41 significant bits), w2
   // the rest rounded to double; P = P1 + P2 the same way
   double w1[kMaxMod], w2[kMaxMod];
-  double s1, s2;  // -4096 sum w1, -4096 sum w2: where the sums over 4096 + r start
   double P1d, P2d, Pd, invPd;
 };
 
@@ -131,11 +130,11 @@ static bool make_consts(int n, Consts* c) {
   for (int i = 0; i < n; ++i) P *= (u128)m[i];
   // budget: ||A'_i||_2 ||B'_j||_2 <= 2^(2H) (1+tiny) < P/2
   c->H = (int)std::floor((log2P(n) - 1.0) / 2.0) - 1;
-  // split point of the CRT weights: sum_l (4096 + r_l) w1_l < 16 * 4352 P <
-  // 2^(bits(P)+17) must be an integer multiple of 2^csplit below 2^(53+csplit)
+  // split point of the CRT weights: sum_l r_l w1_l < 4080 P < 2^(bits(P)+12)
+  // must be an integer multiple of 2^csplit below 2^(53+csplit)
   int bitsP = 0;
   for (u128 t = P; t; t >>= 1) ++bitsP;
-  const int csplit = std::max(0, bitsP + 17 - 53);
+  const int csplit = std::max(0, bitsP + 12 - 53);
   const u128 low = csplit ? (((u128)1 << csplit) - 1) : 0;
   for (int i = 0; i < n; ++i) {
     const int p = m[i];
@@ -158,10 +157,8 @@ static bool make_consts(int n, Consts* c) {
     const u128 Mi = P / (u128)p;
     const int inv = inv_mod((int)(Mi % (u128)p), p);
     const u128 w = mulmod(Mi, (u128)inv, P);
-    c->w1[i] = std::ldexp((double)(uint64_t)(w >> csplit), csplit);  // < 2^36 units: exact
+    c->w1[i] = std::ldexp((double)(uint64_t)(w >> csplit), csplit);  // < 2^41 units: exact
     c->w2[i] = (double)(w & low);
-    c->s1 -= 4096.0 * c->w1[i];  // exact: multiples of 2^csplit below 2^(53+csplit)
-    c->s2 -= 4096.0 * c->w2[i];
   }
   c->P1d = std::ldexp((double)(uint64_t)(P >> csplit), csplit);
   c->P2d = (double)(P & low);
@@ -194,7 +191,6 @@ struct CResConsts {  // of the residue kernel
 struct CCrtConsts {  // of the recombination with n moduli, weights split as in Consts
   double w1[kMaxC], w2[kMaxC];  // real part: times c+ + c-
   double v1[kMaxC], v2[kMaxC];  // imaginary part: times c+ - c-
-  double s1, s2;                // -8192 sum w1, -8192 sum w2
   double P1d, P2d, invPd;
 };
 struct CCrtTab {
@@ -254,10 +250,10 @@ static const CCrtTab& ccrt_tab() {
       CCrtConsts& c = t.c[n];
       u128 P = 1;
       for (int i = 0; i < n; ++i) P *= (u128)kCMod[i];
-      // sum_l (8192 + c+ + c-) w1 < 17 * 8702 P < 2^(bits(P)+18)
+      // sum_l (c+ + c-) w1 < 17 * 510 P < 2^(bits(P)+14)
       int bitsP = 0;
       for (u128 q = P; q; q >>= 1) ++bitsP;
-      const int cs = std::max(0, bitsP + 18 - 53);
+      const int cs = std::max(0, bitsP + 14 - 53);
       const u128 low = cs ? (((u128)1 << cs) - 1) : 0;
       for (int i = 0; i < n; ++i) {
         const int p = kCMod[i], j = sqrt_minus_one(p);
@@ -270,8 +266,6 @@ static const CCrtTab& ccrt_tab() {
         c.w2[i] = (double)(w & low);
         c.v1[i] = std::ldexp((double)(uint64_t)(v >> cs), cs);
         c.v2[i] = (double)(v & low);
-        c.s1 -= 8192.0 * c.w1[i];
-        c.s2 -= 8192.0 * c.w2[i];
       }
       c.P1d = std::ldexp((double)(uint64_t)(P >> cs), cs);
       c.P2d = (double)(P & low);
@@ -401,9 +395,9 @@ __device__ __forceinline__ int shift_of(int code, int H) {
 // rho = sqrt(nnz) ||x||_2 / ||x||_1 (1 for entries of one magnitude, up to
 // sqrt(nnz) for one dominant entry), whose maximum over the rows goes to
 // *rmax (a non-negative float compared as its bits).
-// exact (single precision): the code is the exponent of the row's lowest bit
-// instead, and *rmax the largest log2 of the 2-norm of a row scaled to
-// integers by it (infinite when a row holds Inf / NaN).
+// exact (single precision): *rmax is the largest number of bits from a row's
+// lowest set bit up to its norm's exponent instead (infinite when a row holds
+// Inf / NaN): with at least that budget H the scaled rows are integers.
 __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* code,
                           unsigned* rmax, int exact) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -422,9 +416,6 @@ __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* c
       if (exact) rho = __int_as_float(0x7f800000);
     } else if (mx == 0.0) {
       code[l] = kCodeZero;
-    } else if (exact) {
-      code[l] = (int)s1;
-      rho = (float)(log2(fmax(sqrt(ss), mx)) - s1 + 1e-3);  // >= 0: the row has a bit at s1
     } else {
       // bound on the row 2-norm (the sum of squares may overflow for huge entries)
       double nrm = isfinite(ss) ? sqrt(ss) : mx * sqrt((double)K);
@@ -432,9 +423,10 @@ __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* c
       int e;
       frexp(nrm, &e);  // nrm < 2^e
       code[l] = e;
+      if (exact) rho = (float)(e - (int)s1);
       // scale-free form: sqrt(nnz) * (nrm / mx) / (s1 / mx), all ratios <= nnz
       const double r = sqrt(nz) * (nrm / mx) / fmax(s1 / mx, 1.0);
-      rho = (float)fmin(r, 3.0e38);
+      if (!exact) rho = (float)fmin(r, 3.0e38);
     }
   }
   // warp maximum, one atomic per warp
@@ -452,28 +444,28 @@ __global__ void k_oz_stat(int L, int K, int nchunks, const double4* part, int* c
 // FP64 rounding; if the largest count cannot, the call runs the plain FP64
 // kernel instead (fallback = 1), or, where that is not allowed, the largest
 // count.  fixed > 0: that count, no data rule.
-// Exact products (single-precision operands): the operands are scaled to
-// integers without rounding, so the product is the exact one whenever
-// ||a'_i|| ||b'_j|| < P/4 for all rows and columns: the smallest count for
-// which it is; else the plain kernel.
+// Exact products (single-precision operands): the smallest count whose budget
+// scales every row and column to integers without rounding, so that the
+// product is the exact one; else the plain kernel.
 struct PickP {
   int fixed, lo, hi, allow_fallback, exact;
   int H[kMaxMod + 1];        // exponent budget per count
   int np[kMaxMod + 1];       // moduli multiplied per count
-  float lim[kMaxC + 1];      // exact: log2 of P/4 per moduli multiplied
+  int Hx[kMaxC + 1];         // exact: budget per moduli multiplied
 };
 
 __global__ void k_oz_pick(const unsigned* rmax, OzSel* sel, const PickP q) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int n = q.fixed, fb = 0;
   if (q.exact) {
-    const float ra = __uint_as_float(rmax[0]), rb = __uint_as_float(rmax[1]);
+    const float need = fmaxf(__uint_as_float(rmax[0]), __uint_as_float(rmax[1]));
+    int h = 0;
     n = 0;
 #pragma unroll
     for (int c = kMaxC; c >= 2; --c)
-      if (c >= q.lo && c <= q.hi && ra < 61.5f && rb < 61.5f && ra + rb <= q.lim[c]) n = c;
+      if (c >= q.lo && c <= q.hi && (float)q.Hx[c] >= need) n = c, h = q.Hx[c];
     sel->n = n;
-    sel->H = 0;  // the codes are the shifts
+    sel->H = h;
     sel->fallback = n == 0;
     sel->np = n;
     return;
@@ -1182,19 +1174,18 @@ struct CrtP {
 
 // Recombination on the FP64 pipe.  S = sum_l r_l w_l < 4080 P; the shifts
 // keep |C'| <= P/8, so the wanted value is S - qP with q = round(S / P).
-// r_l enters as the double 4096 + r_l, one byte permutation (an int -> double
-// conversion per residue would take longer than the sums), and the sums start
-// at -4096 sum_l w_l.
-// With w = w1 + w2 (w1: multiples of 2^csplit, <= 36 significant bits):
-//  - S1 = sum r_l w1_l is exact (13-bit x 36-bit products, multiples of
-//    2^csplit, every partial sum below 2^(53+csplit));
-//  - q = rint(S1 / P) is exact: S2 / P < 2^-23 and S / P lies within 1/8 of
+// With w = w1 + w2 (w1: multiples of 2^csplit, <= 41 significant bits):
+//  - S1 = sum r_l w1_l is exact (8-bit x 41-bit products, multiples of
+//    2^csplit, sum below 2^(53+csplit));
+//  - q = rint(S1 / P) is exact: S2 / P < 2^-28 and S / P lies within 1/8 of
 //    an integer (q < 2^12);
-//  - S1 - q P1 is exact (a 48-bit product, the difference a multiple of
-//    2^csplit below 2^(38+csplit));
-//  - S2 - q P2 carries absolute errors of order 2^(csplit-36) (2^54 at 16
-//    moduli), 2^-67 of the largest result and far below the 2^(2H-61) sqrt(K)
+//  - S1 - q P1 is exact (a 53-bit product, the difference a multiple of
+//    2^csplit below 2^(42+csplit));
+//  - S2 - q P2 carries absolute errors of order 2^(csplit-37) plus the
+//    rounding of w2 (2^43 at 16 moduli), far below the 2^(2H-61) sqrt(K)
 //    already left by rounding the scaled operands to integers.
+// r_l becomes a double by one byte permutation (4096 + r_l) and an FP64 add: a
+// conversion from int per residue takes longer than the sums.
 // 2 FP64 FMAs per modulus and element (a 128-bit integer sum would take 4
 // 64-bit integer multiply-adds).  The weights are constant loads, not operands
 // of an FP64 FMA, so each is used for eight elements at once.
@@ -1209,6 +1200,11 @@ __device__ __forceinline__ double scale2(double x, int e) {
     return __hiloint2double(hi + (int)((unsigned)e << 20), __double2loint(x));
   const int e1 = e / 2, e2 = e - e1;
   return x * pow2(e1) * pow2(e2);
+}
+
+// byte b of w as a double: bytes 40 B0 r 00 are the high word of 4096 + r
+__device__ __forceinline__ double crt_byte(uint32_t w, int b) {
+  return __hiloint2double((int)__byte_perm(w, 0x40B00000u, 0x7604 + (b << 4)), 0) - 4096.0;
 }
 
 // A warp takes 16 rows x 16 columns: lane l row l / 2 and columns 8 (l % 2)
@@ -1247,19 +1243,13 @@ __device__ __forceinline__ void crt_cols(const CrtP& p, const Consts& c, int H, 
   };
   double s1[8], s2[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    s1[e] = c.s1;
-    s2[e] = c.s2;
-  }
+  for (int e = 0; e < 8; ++e) s1[e] = s2[e] = 0.0;
 #pragma unroll
   for (int m = 0; m < NM; ++m) {
     const double w1 = c.w1[m], w2 = c.w2[m];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      // bytes 40 B0 r 00: the high word of the double 4096 + r
-      const uint32_t hi = __byte_perm(e < 4 ? words[m].x : words[m].y, 0x40B00000u,
-                                      0x7604 + ((e & 3) << 4));
-      const double rv = __hiloint2double((int)hi, 0);
+      const double rv = crt_byte(e < 4 ? words[m].x : words[m].y, e & 3);
       s1[e] = fma(rv, w1, s1[e]);
       s2[e] = fma(rv, w2, s2[e]);
     }
@@ -1280,33 +1270,32 @@ __device__ __forceinline__ void crt_cols(const CrtP& p, const Consts& c, int H, 
   }
 }
 
-template <int NM, class E>
+template <int NM>
 __device__ __forceinline__ void crt_body(const CrtP& p, const Consts& c, int H) {
   const bool beta = p.br != 0.0;
-  E* C = static_cast<E*>(p.C);
+  double* C = static_cast<double*>(p.C);
   double cr[8];
   crt_cols<NM>(
       p, c, H,
       [&](int i, int j, int e) {
-        if (beta) cr[e] = (double)C[(size_t)i + (size_t)j * p.ldc];
+        if (beta) cr[e] = C[(size_t)i + (size_t)j * p.ldc];
       },
       [&](int i, int j, int e, double y) {
         double out = p.ar * y;
         if (beta) out = fma(p.br, cr[e], out);
-        C[(size_t)i + (size_t)j * p.ldc] = (E)out;
+        C[(size_t)i + (size_t)j * p.ldc] = out;
       });
 }
 
 // Complex recombination: a warp takes 8 rows x 16 columns, a lane row l / 4
 // and the four columns 4 (l % 4) .. + 3; both parts of an element come from
-// the planes 2m (c+) and 2m + 1 (c-) in one pass.  c+ and c- enter as 4096 + r
-// (see above): their sum, offset by 8192, meets the real part's weights, their
-// difference the imaginary part's.  Same bounds as the real form: the real
-// part's partial sums stay below 17 * 8702 P < 2^(53+csplit), |q| < 2^14, and
-// |C'| <= P/4 leaves q = rint(S1 / P) exact.
+// the planes 2m (c+) and 2m + 1 (c-) in one pass: c+ + c- meets the real
+// part's weights, c+ - c- the imaginary part's.  Bounds as in the real form:
+// the sums stay below 17 * 510 P < 2^(53+csplit), |q| < 2^14, and |C'| <= P/4
+// leaves q = rint(S1 / P) exact.
 constexpr int kCrtRowsC = 8;
 
-template <int NM, class E>
+template <int NM>
 __device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, int H) {
   const size_t plane = (size_t)p.Mpad * (size_t)p.Npad;
   const int lane = threadIdx.x & 31;
@@ -1326,19 +1315,14 @@ __device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, i
   double r1[4], r2[4], x1[4], x2[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    r1[e] = c.s1;
-    r2[e] = c.s2;
-    x1[e] = x2[e] = 0.0;
+    r1[e] = r2[e] = x1[e] = x2[e] = 0.0;
   }
 #pragma unroll
   for (int m = 0; m < NM; ++m) {
     const double w1 = c.w1[m], w2 = c.w2[m], v1 = c.v1[m], v2 = c.v2[m];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const double a =
-          __hiloint2double((int)__byte_perm(wp[m], 0x40B00000u, 0x7604 + (e << 4)), 0);
-      const double b =
-          __hiloint2double((int)__byte_perm(wm[m], 0x40B00000u, 0x7604 + (e << 4)), 0);
+      const double a = crt_byte(wp[m], e), b = crt_byte(wm[m], e);
       const double su = a + b, di = a - b;
       r1[e] = fma(su, w1, r1[e]);
       r2[e] = fma(su, w2, r2[e]);
@@ -1348,7 +1332,7 @@ __device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, i
   }
   const bool beta = p.br != 0.0 || p.bi != 0.0;
   const bool mask = p.uplo != XKB_FULL;
-  E* C = static_cast<E*>(p.C);
+  double* C = static_cast<double*>(p.C);
   auto in = [&](int e) {
     if (j0 + e >= p.N) return false;
     if (!mask) return true;
@@ -1361,8 +1345,8 @@ __device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, i
     cr[e] = ci[e] = 0.0;
     if (beta && in(e)) {
       const size_t idx = (size_t)i + (size_t)(j0 + e) * p.ldc;
-      cr[e] = (double)C[2 * idx];
-      ci[e] = (double)C[2 * idx + 1];
+      cr[e] = C[2 * idx];
+      ci[e] = C[2 * idx + 1];
     }
   }
   const int mui = shift_of(p.mu[i], H);
@@ -1387,8 +1371,8 @@ __device__ __forceinline__ void crt_body_c(const CrtP& p, const CCrtConsts& c, i
     }
     if (p.herm_diag && (long)i + p.diag == (long)(j0 + e)) vi = 0.0;
     const size_t idx = (size_t)i + (size_t)(j0 + e) * p.ldc;
-    C[2 * idx] = (E)vr;
-    C[2 * idx + 1] = (E)vi;
+    C[2 * idx] = vr;
+    C[2 * idx + 1] = vi;
   }
 }
 
@@ -1401,39 +1385,186 @@ template <int NM>
 __global__ void __launch_bounds__(256, 3) k_oz_crt(const CrtP p, const Consts c) {
   const OzSel s = *p.sel;
   if (s.n != NM) return;
-  crt_body<NM, double>(p, c, s.H);
+  crt_body<NM>(p, c, s.H);
 }
 __global__ void __launch_bounds__(256, 3) k_oz_crt_15_16(const CrtP p, const Consts c15,
                                                          const Consts c16) {
   const OzSel s = *p.sel;
-  if (s.n == 15) crt_body<15, double>(p, c15, s.H);
-  else if (s.n == 16) crt_body<16, double>(p, c16, s.H);
+  if (s.n == 15) crt_body<15>(p, c15, s.H);
+  else if (s.n == 16) crt_body<16>(p, c16, s.H);
 }
 
-constexpr int kExactLo = 8, kExactLoC = 9;  // fewest moduli of an exact product
-struct CrtTabS {
-  Consts c[kMaxMod - kExactLo + 1];
+// Exact products (single precision).  A row whose entries are small beside
+// the operand's largest may meet a column the same way, and its C' is then far
+// below the 2^(csplit-36) that the two-part weights leave: here the weights
+// have three parts of 41 (complex 39, 39, 40) bits and every sum is exact.
+// Real: r_l < 2^8 and at most 15 moduli, P < 2^118: with c1 = bits(P) - 41,
+// c2 = max(0, c1 - 41) <= 36, the sums S1, S2, S3 of r_l times the parts are
+// multiples of 2^c1, 2^c2, 1 below 2^(53 + c1), 2^(53 + c2), 2^53, and so are
+// S_i - q P_i (q = rint(S1 / P) < 2^12 as above, the products 53 bits).  Their
+// sum is formed with one compensated addition: relative error 2^-52.
+constexpr int kExactLo = 8, kExactHi = 15;    // moduli of an exact product
+constexpr int kExactLoC = 9, kExactHiC = 16;  // and of a complex one
+struct Crt3 {
+  double w[3][kMaxC];  // times r, complex: the real part's, times c+ + c-
+  double v[3][kMaxC];  // complex: the imaginary part's, times c+ - c-
+  double P[3], invP;
 };
-template <int NM>
-__device__ __forceinline__ void crt_any_s(const CrtP& p, const CrtTabS& t, const OzSel& s) {
-  if (s.np == NM) crt_body<NM, float>(p, t.c[NM - kExactLo], s.H);
-  else if constexpr (NM < kMaxMod) crt_any_s<NM + 1>(p, t, s);
+struct Crt3Tab {
+  Crt3 c[kExactHi - kExactLo + 1];
+};
+static_assert(kExactHi - kExactLo == kExactHiC - kExactLoC, "one table type");
+
+static void split3(u128 x, int c1, int c2, double* p0, double* p1, double* p2) {
+  *p0 = std::ldexp((double)(uint64_t)(x >> c1), c1);
+  x &= (((u128)1) << c1) - 1;
+  *p1 = std::ldexp((double)(uint64_t)(x >> c2), c2);
+  x &= c2 ? (((u128)1) << c2) - 1 : 0;
+  *p2 = (double)(uint64_t)x;
 }
-__global__ void __launch_bounds__(256, 3) k_oz_crt_s(const CrtP p,
-                                                     const __grid_constant__ CrtTabS t) {
+
+static const Crt3Tab& crt3_tab(bool cplx) {
+  auto make = [](bool cx) {
+    Crt3Tab t;
+    std::memset(&t, 0, sizeof(t));
+    const std::vector<int> rm = moduli_list();
+    const int lo = cx ? kExactLoC : kExactLo, hi = cx ? kExactHiC : kExactHi;
+    for (int n = lo; n <= hi; ++n) {
+      Crt3& c = t.c[n - lo];
+      auto mod = [&](int i) { return cx ? kCMod[i] : rm[i]; };
+      u128 P = 1;
+      for (int i = 0; i < n; ++i) P *= (u128)mod(i);
+      int bitsP = 0;
+      for (u128 q = P; q; q >>= 1) ++bitsP;
+      const int w = cx ? 39 : 41;
+      const int c1 = std::max(1, bitsP - w), c2 = std::max(0, c1 - w);
+      for (int i = 0; i < n; ++i) {
+        const int p = mod(i);
+        const u128 Mi = P / (u128)p;
+        const int im = inv_mod((int)(Mi % (u128)p), p);
+        const int f = cx ? (int)((long)im * inv_mod(2, p) % p) : im;
+        split3(Mi * (u128)f, c1, c2, &c.w[0][i], &c.w[1][i], &c.w[2][i]);
+        if (cx) {
+          const int j = sqrt_minus_one(p);
+          const int fi = (int)((long)im * inv_mod(2 * j % p, p) % p);
+          split3(Mi * (u128)fi, c1, c2, &c.v[0][i], &c.v[1][i], &c.v[2][i]);
+        }
+      }
+      split3(P, c1, c2, &c.P[0], &c.P[1], &c.P[2]);
+      c.invP = 1.0 / (double)P;
+    }
+    return t;
+  };
+  static const Crt3Tab real = make(false), comp = make(true);
+  return cplx ? comp : real;
+}
+
+// The value of the exact sums s[0..2].
+__device__ __forceinline__ double crt3_value(const double (&s)[3], const Crt3& c) {
+  const double q = rint(s[0] * c.invP);
+  const double d0 = fma(-q, c.P[0], s[0]), d1 = fma(-q, c.P[1], s[1]),
+               d2 = fma(-q, c.P[2], s[2]);
+  const double t = d0 + d1, z = t - d0;  // t + e = d0 + d1
+  const double e = (d0 - (t - z)) + (d1 - z);
+  return t + (e + d2);
+}
+// A warp takes 8 rows x 16 columns, a lane row l / 4 and the four columns
+// 4 (l % 4) .. + 3 (as crt_body_c).
+template <int NM, bool CPLX>
+__device__ __forceinline__ void crt_body_x(const CrtP& p, const Crt3& c, int H) {
+  constexpr int PL = CPLX ? 2 : 1;
+  const size_t plane = (size_t)p.Mpad * (size_t)p.Npad;
+  const int lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * kCrtRowsC, i = i0 + (lane >> 2);
+  const int jw = blockIdx.y * kCrtCols + (int)(threadIdx.x >> 5) * 16;
+  const int j0 = jw + 4 * (lane & 3);
+  if (p.uplo == XKB_LOWER && (long)i0 + kCrtRowsC - 1 + p.diag < (long)jw) return;
+  if (p.uplo == XKB_UPPER && (long)i0 + p.diag > (long)jw + 15) return;
+  if (i >= p.M || j0 >= p.N) return;
+  uint32_t word[PL * NM];
+  const uint8_t* src = p.R + (size_t)jw * (size_t)p.Mpad + (size_t)i * 16 + (size_t)(4 * (lane & 3));
+#pragma unroll
+  for (int m = 0; m < PL * NM; ++m)
+    word[m] = __ldcs(reinterpret_cast<const uint32_t*>(src + (size_t)m * plane));
+  double r[4][3], x[4][3];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) r[e][q] = x[e][q] = 0.0;
+#pragma unroll
+  for (int m = 0; m < NM; ++m) {
+    const double w0 = c.w[0][m], w1 = c.w[1][m], w2 = c.w[2][m];
+    const double v0 = CPLX ? c.v[0][m] : 0.0, v1 = CPLX ? c.v[1][m] : 0.0,
+                 v2 = CPLX ? c.v[2][m] : 0.0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      double su = crt_byte(word[PL * m], e);
+      if constexpr (CPLX) {
+        const double b = crt_byte(word[2 * m + 1], e), di = su - b;
+        su += b;
+        x[e][0] = fma(di, v0, x[e][0]);
+        x[e][1] = fma(di, v1, x[e][1]);
+        x[e][2] = fma(di, v2, x[e][2]);
+      }
+      r[e][0] = fma(su, w0, r[e][0]);
+      r[e][1] = fma(su, w1, r[e][1]);
+      r[e][2] = fma(su, w2, r[e][2]);
+    }
+  }
+  const bool beta = p.br != 0.0 || p.bi != 0.0;
+  const bool mask = p.uplo != XKB_FULL;
+  float* C = static_cast<float*>(p.C);
+  const int mui = shift_of(p.mu[i], H);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int j = j0 + e;
+    if (j >= p.N) break;
+    if (mask && (p.uplo == XKB_LOWER ? (long)i + p.diag < (long)j : (long)i + p.diag > (long)j))
+      continue;
+    const int sh = -(mui + shift_of(p.nu[j], H));
+    const size_t idx = (size_t)i + (size_t)j * p.ldc;
+    const double xr = scale2(crt3_value(r[e], c), sh);
+    if constexpr (CPLX) {
+      const double xi = scale2(crt3_value(x[e], c), sh);
+      double vr = p.ar * xr - p.ai * xi;
+      double vi = p.ar * xi + p.ai * xr;
+      if (beta) {
+        const double cr = (double)C[2 * idx], ci = (double)C[2 * idx + 1];
+        vr += p.br * cr - p.bi * ci;
+        vi += p.br * ci + p.bi * cr;
+      }
+      if (p.herm_diag && (long)i + p.diag == (long)j) vi = 0.0;
+      C[2 * idx] = (float)vr;
+      C[2 * idx + 1] = (float)vi;
+    } else {
+      double out = p.ar * xr;
+      if (beta) out = fma(p.br, (double)C[idx], out);
+      C[idx] = (float)out;
+    }
+  }
+}
+template <int NM, bool CPLX>
+__device__ __forceinline__ void crt_any_x(const CrtP& p, const Crt3Tab& t, const OzSel& s) {
+  constexpr int LO = CPLX ? kExactLoC : kExactLo, HI = CPLX ? kExactHiC : kExactHi;
+  if (s.np == NM) crt_body_x<NM, CPLX>(p, t.c[NM - LO], s.H);
+  else if constexpr (NM < HI) crt_any_x<NM + 1, CPLX>(p, t, s);
+}
+template <bool CPLX>
+__global__ void __launch_bounds__(256, 2) k_oz_crt_x(const CrtP p,
+                                                     const __grid_constant__ Crt3Tab t) {
   const OzSel s = *p.sel;
-  if (s.np >= kExactLo) crt_any_s<kExactLo>(p, t, s);
+  crt_any_x<CPLX ? kExactLoC : kExactLo, CPLX>(p, t, s);
 }
-template <int NM, class E>
+
+template <int NM>
 __device__ __forceinline__ void crt_any_c(const CrtP& p, const CCrtTab& t, const OzSel& s) {
-  if (s.np == NM) crt_body_c<NM, E>(p, t.c[NM], s.H);
-  else if constexpr (NM < kMaxC) crt_any_c<NM + 1, E>(p, t, s);
+  if (s.np == NM) crt_body_c<NM>(p, t.c[NM], s.H);
+  else if constexpr (NM < kMaxC) crt_any_c<NM + 1>(p, t, s);
 }
-template <class E>
 __global__ void __launch_bounds__(256, 2) k_oz_crt_c(const CrtP p,
                                                      const __grid_constant__ CCrtTab t) {
   const OzSel s = *p.sel;
-  if (s.np >= 2) crt_any_c<2, E>(p, t, s);
+  if (s.np >= 2) crt_any_c<2>(p, t, s);
 }
 
 // lo == hi: that count; (lo, hi) == (15, 16): the count the device chose.
@@ -1572,8 +1703,9 @@ static int launch_pick(CallWords* w, const ModPlan& pl, bool allow_fallback, cud
   if (exact) {
     q.exact = 1;
     q.lo = cplx ? kExactLoC : kExactLo;
-    q.hi = cplx ? kMaxC : kMaxMod;
-    for (int n = 2; n <= q.hi; ++n) q.lim[n] = (float)((cplx ? log2Pc(n) : log2P(n)) - 2.01);
+    q.hi = cplx ? kExactHiC : kExactHi;
+    for (int n = 2; n <= q.hi; ++n)
+      q.Hx[n] = cplx ? (int)std::floor((log2Pc(n) - 2.0) / 2.0) : consts_for(n)->H;
   }
   const long long tv = evlog_kern_begin(st, "k_oz_pick");
   k_oz_pick<<<1, 32, 0, st>>>(w->rmax, &w->sel, q);
@@ -1600,7 +1732,7 @@ static int res_real(const View& v, int L, int K, const int* code, const OzSel* s
                                                      Kpad);
   };
   if constexpr (sizeof(E) == 4) {  // exact products plan for every count
-    go(std::integral_constant<int, kMaxMod>());
+    go(std::integral_constant<int, kExactHi>());
     return XKB_OK;
   } else {
     switch (c->nmod) {
@@ -1658,14 +1790,14 @@ static bool encode_planes(CUtensorMap* m, const int8_t* base, long Kpad, long Lp
 // Npad; equal when one buffer serves both operands).  a_stride / b_stride
 // (0: the same): rows between consecutive planes, when Ap / Bp point at a
 // block of rows of larger planes.
-// c: the plan's largest count; null: a complex product, 2 kMaxC planes
+// c: the plan's largest count; null: a complex product of cplanes planes
 // (bxor: see GemmP).
 static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_rows, long Mpad,
                        long Npad, long Kpad, const Consts* c, const OzSel* sel, uint8_t* R,
                        int uplo, long diag, cudaStream_t st, long a_stride = 0,
-                       long b_stride = 0, int bxor = 0) {
+                       long b_stride = 0, int cplanes = 0, int bxor = 0) {
   CUtensorMap tA, tB;
-  const int npl = c ? c->nmod : 2 * kMaxC;
+  const int npl = c ? c->nmod : cplanes;
   if (a_rows < Mpad || b_rows < Npad) return XKB_EINVAL;
   if (!encode_planes(&tA, Ap, Kpad, a_rows, npl, BM, a_stride)) return XKB_EINVAL;
   if (!encode_planes(&tB, Bp, Kpad, b_rows, npl, BN, b_stride)) return XKB_EINVAL;
@@ -1806,8 +1938,9 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   const long Keff = cplx ? 2L * a->K : (long)a->K;
   if (Keff > 131072) return XKB_ERANGE;
   ModPlan pl;
-  if (!plan_moduli(exact ? kMaxMod : nmod, Keff, &pl)) return XKB_ERANGE;
-  const int nmax = cplx ? kMaxPl : pl.hi;  // planes
+  if (!plan_moduli(exact ? kExactHi : nmod, Keff, &pl)) return XKB_ERANGE;
+  // planes
+  const int nmax = exact ? (cplx ? 2 * kExactHiC : kExactHi) : (cplx ? kMaxPl : pl.hi);
   const Consts* c = cplx ? nullptr : pl.chi;
   const int M = a->M, N = a->N, K = a->K;
   const long Kpad = (long)rup(K, BKB);
@@ -1866,7 +1999,7 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   trace_mark(slot, 1, st);
   if (!err)
     err = launch_gemm(Ap, Arows, same ? Ap : Bp, same ? Arows : Npad, Mpad, Npad, Kpad, c, sel, R,
-                      a->uplo, a->diag, st, 0, 0, bxor);
+                      a->uplo, a->diag, st, 0, 0, nmax, bxor);
   trace_mark(slot, 2, st);
   if (!err) {
     CrtP cp;
@@ -1893,17 +2026,11 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
     } else {
       const long long tv = evlog_kern_begin(st, "k_oz_crt");
       const unsigned gy = (unsigned)((N + kCrtCols - 1) / kCrtCols);
-      const unsigned gr = (unsigned)((M + kCrtRows - 1) / kCrtRows);
       const unsigned gc = (unsigned)((M + kCrtRowsC - 1) / kCrtRowsC);
-      if (a->dtype == XKB_S) {
-        CrtTabS t;
-        for (int n = kExactLo; n <= kMaxMod; ++n) t.c[n - kExactLo] = *consts_for(n);
-        k_oz_crt_s<<<dim3(gr, gy), 256, 0, st>>>(cp, t);
-      } else if (a->dtype == XKB_C) {
-        k_oz_crt_c<float><<<dim3(gc, gy), 256, 0, st>>>(cp, ccrt_tab());
-      } else {
-        k_oz_crt_c<double><<<dim3(gc, gy), 256, 0, st>>>(cp, ccrt_tab());
-      }
+      const dim3 g(gc, gy);
+      if (a->dtype == XKB_S) k_oz_crt_x<false><<<g, 256, 0, st>>>(cp, crt3_tab(false));
+      else if (a->dtype == XKB_C) k_oz_crt_x<true><<<g, 256, 0, st>>>(cp, crt3_tab(true));
+      else k_oz_crt_c<<<g, 256, 0, st>>>(cp, ccrt_tab());
       evlog_kern_end(tv, st);
       count_launch();
       if (cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
@@ -1946,7 +2073,7 @@ int gemm_exact(const xkb_gemm_args* a, cudaStream_t st) {
   if (tune("gemm_exact", 1.0) == 0.0 || mn < 512 || a->K < 512 ||
       (double)a->M * a->N * a->K * (cplx ? 4.0 : 1.0) < tune("gemm_exact_min", 3.4e9))
     return XKB_ERANGE;
-  const double planes = cplx ? kMaxPl : kMaxMod;
+  const double planes = cplx ? 2 * kExactHiC : kExactHi;
   if (planes * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N) > 17.2e9)
     return XKB_ERANGE;  // at most 16 GiB of scratch
   return oz_run(a, 0, st);
