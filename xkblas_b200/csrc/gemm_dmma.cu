@@ -70,49 +70,71 @@ __global__ void k_scale(int M, int N, double br, double bi, T* Cv, long ldc, int
   }
 }
 
-// Copy a rows x cols column-major array (element size es) into a packed
-// array with leading dimension ldd.  Used to give TMA a 16-byte aligned view
-// of an operand whose base or leading dimension is not 16-byte aligned.
+// Copies of up to two column-major arrays, one per blockIdx.z: rows x cols
+// words of W, wpe words per element, optionally only the elements of a
+// triangle.  A block takes 256 rows x 8 columns (no index division: with one
+// per element the copy ran at a third of the memory rate; 8 loads in flight
+// per thread).
+struct CopyWords {
+  const void* src;
+  void* dst;
+  long lds, ldd;  // words
+  int rows, cols, wpe, uplo;
+};
 template <class W>
-__global__ void k_repack(int rows_w, int cols, const W* __restrict__ src, long lds_w,
-                         W* __restrict__ dst, long ldd_w, const int* run_if) {
+__global__ void __launch_bounds__(256) k_repack(const CopyWords d0, const CopyWords d1,
+                                                const int* run_if) {
   if (run_if && *run_if == 0) return;
-  const size_t total = (size_t)rows_w * (size_t)cols;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = e % (size_t)rows_w, j = e / (size_t)rows_w;
-    dst[i + j * (size_t)ldd_w] = src[i + j * (size_t)lds_w];
+  const CopyWords& d = blockIdx.z ? d1 : d0;
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= d.rows) return;
+  const W* src = static_cast<const W*>(d.src);
+  W* dst = static_cast<W*>(d.dst);
+  const int er = d.wpe == 1 ? r : d.wpe == 2 ? r >> 1 : r >> 2;
+  for (int c0 = blockIdx.y * 8; c0 < d.cols; c0 += gridDim.y * 8) {
+    W v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (c0 + q < d.cols && in_mask(d.uplo, 0, er, c0 + q))
+        v[q] = src[(size_t)r + (size_t)(c0 + q) * (size_t)d.lds];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (c0 + q < d.cols && in_mask(d.uplo, 0, er, c0 + q))
+        dst[(size_t)r + (size_t)(c0 + q) * (size_t)d.ldd] = v[q];
   }
 }
 
-static bool tma_ok(const void* p, long ld, int es) {
-  return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ((size_t)ld * es) % 16 == 0;
-}
-
-// Packed copy of a stored operand (rows x cols, element size es); *out is a
-// stream-ordered allocation the caller frees on the same stream.
-static int repack(const void* src, long ld, int rows, int cols, int es, void** out, long* ldo,
-                  cudaStream_t st, const int* run_if) {
-  const long ldp = (long)(((size_t)rows * es + 15) / 16 * 16 / es);
-  if (cudaMallocAsync(out, std::max<size_t>((size_t)ldp * cols * es, 16), st) != cudaSuccess)
-    return XKB_ENOMEM;
-  *ldo = ldp;
-  const size_t total = (size_t)rows * cols;
-  const unsigned grid = (unsigned)std::max<size_t>(
-      1, std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 16));
+int copy_arrays(const CopyArray* d, int n, int es, cudaStream_t st, const int* run_if) {
+  if (n < 1 || n > 2) return n == 0 ? XKB_OK : XKB_EINVAL;
+  bool wide = es % 8 == 0;
+  for (int i = 0; i < n; ++i)
+    wide = wide && reinterpret_cast<uintptr_t>(d[i].src) % 8 == 0 &&
+           reinterpret_cast<uintptr_t>(d[i].dst) % 8 == 0;
+  const int wb = wide ? 8 : 4, wpe = es / wb;
+  CopyWords w[2];
+  int mr = 0, mc = 0;
+  for (int i = 0; i < n; ++i) {
+    w[i] = {d[i].src, d[i].dst, d[i].lds * wpe, d[i].ldd * wpe, d[i].rows * wpe, d[i].cols, wpe,
+            d[i].uplo};
+    mr = std::max(mr, w[i].rows);
+    mc = std::max(mc, w[i].cols);
+  }
+  if (n == 1) w[1] = w[0];
+  const dim3 g((unsigned)((mr + 255) / 256), (unsigned)std::min((mc + 7) / 8, 32768), (unsigned)n);
   const long long tv = evlog_kern_begin(st, "k_repack");
-  if (es % 8 == 0 && reinterpret_cast<uintptr_t>(src) % 8 == 0)
-    k_repack<double><<<grid, 256, 0, st>>>(rows * (es / 8), cols,
-                                           static_cast<const double*>(src), ld * (es / 8),
-                                           static_cast<double*>(*out), ldp * (es / 8), run_if);
-  else
-    k_repack<float><<<grid, 256, 0, st>>>(rows * (es / 4), cols, static_cast<const float*>(src),
-                                          ld * (es / 4), static_cast<float*>(*out),
-                                          ldp * (es / 4), run_if);
+  if (wide) k_repack<double><<<g, 256, 0, st>>>(w[0], w[1], run_if);
+  else k_repack<float><<<g, 256, 0, st>>>(w[0], w[1], run_if);
   evlog_kern_end(tv, st);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
 }
+
+bool tma_ok(const void* p, long ld, int es) {
+  return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ((size_t)ld * es) % 16 == 0;
+}
+
+// Leading dimension of a packed, 16-byte aligned copy.
+long packed_ld(long rows, int es) { return (long)(((size_t)rows * es + 15) / 16 * 16 / es); }
 
 template <class T>
 static int launch_scale(int M, int N, const double* beta, void* C, long ldc, int uplo,
@@ -178,17 +200,38 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
       reinterpret_cast<uintptr_t>(a->C) % 4)
     return XKB_EINVAL;
   xkb_gemm_args pa = *a;
-  void* packA = nullptr;
-  void* packB = nullptr;
+  void* pack = nullptr;  // one allocation and one launch for both operands
   int r = XKB_OK;
-  if (!tma_ok(a->A, a->lda, es))
-    r = repack(a->A, a->lda, a->opA == XKB_OP_N ? a->M : a->K,
-               a->opA == XKB_OP_N ? a->K : a->M, es, &packA, &pa.lda, st, run_if);
-  if (r == XKB_OK && !tma_ok(a->B, a->ldb, es))
-    r = repack(a->B, a->ldb, a->opB == XKB_OP_N ? a->K : a->N,
-               a->opB == XKB_OP_N ? a->N : a->K, es, &packB, &pa.ldb, st, run_if);
-  if (packA) pa.A = packA;
-  if (packB) pa.B = packB;
+  const bool okA = tma_ok(a->A, a->lda, es), okB = tma_ok(a->B, a->ldb, es);
+  if (!okA || !okB) {
+    const int ra = a->opA == XKB_OP_N ? a->M : a->K, ca = a->opA == XKB_OP_N ? a->K : a->M;
+    const int rb = a->opB == XKB_OP_N ? a->K : a->N, cb = a->opB == XKB_OP_N ? a->N : a->K;
+    // the same array as both operands (a rank-k update) is copied once
+    const bool same = a->A == a->B && a->lda == a->ldb && ra == rb && ca == cb;
+    const long la = packed_ld(ra, es), lb = packed_ld(rb, es);
+    const size_t za = okA ? 0 : ((size_t)la * ca * es + 255) / 256 * 256;
+    const size_t zb = okB || same ? 0 : (size_t)lb * cb * es;
+    if (cudaMallocAsync(&pack, std::max<size_t>(za + zb, 256), st) != cudaSuccess) {
+      cudaGetLastError();
+      return XKB_ENOMEM;
+    }
+    CopyArray d[2];
+    int n = 0;
+    if (!okA) {
+      d[n++] = {a->A, pack, a->lda, la, ra, ca, XKB_FULL};
+      pa.A = pack;
+      pa.lda = la;
+    }
+    if (same) {
+      pa.B = pa.A;
+      pa.ldb = pa.lda;
+    } else if (!okB) {
+      pa.B = static_cast<char*>(pack) + za;
+      pa.ldb = lb;
+      d[n++] = {a->B, const_cast<void*>(pa.B), a->ldb, lb, rb, cb, XKB_FULL};
+    }
+    r = copy_arrays(d, n, es, st, run_if);
+  }
   if (r == XKB_OK) {
     r = XKB_EINVAL;
     switch (a->dtype) {
@@ -198,8 +241,7 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
       case XKB_Z: r = gemm_dmma_z(&pa, st, run_if); break;
     }
   }
-  if (packA) cudaFreeAsync(packA, st);
-  if (packB) cudaFreeAsync(packB, st);
+  if (pack) cudaFreeAsync(pack, st);
   trace_mark(slot, 2, st);
   trace_mark(slot, 3, st);
   return r;

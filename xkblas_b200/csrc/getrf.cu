@@ -570,11 +570,24 @@ extern "C" int xkb_cuda_getrf_nopiv(int dtype, int N, void* A, long lda, int* d_
   const int mode = (int)tune("getrf_blocked", 3.0);
   const long nb = std::max(nmax, ((long)tune(c.ozaki ? "getrf_nb_oz" : "getrf_nb",
                                              c.ozaki ? 2048.0 : 512.0) + 63) / 64 * 64);
+  // a matrix TMA cannot read in place is factored in an aligned copy
+  AlignedArray w;
+  int e = XKB_OK;
+  if (N > nmax && (e = w.take(A, lda, N, N, XKB_FULL, c.es, c.st))) return e;
+  if (w.buf) {
+    c.A = static_cast<char*>(w.p);
+    c.lda = w.ld;
+  }
+  auto done = [&](int r) {
+    if (!r) r = w.put_back(c.st);
+    w.release(c.st);
+    return r;
+  };
   if (N > 2 * nmax && (mode == 2 || (mode == 1 && c.ozaki == 0)))
-    return factor_blocked(c, 0, N, nb);
+    return done(factor_blocked(c, 0, N, nb));
   if (mode == 3) {  // in plain mode too: DMMA couplings (8192: 18.3 against 18.9 ms)
     c.blk_leaf = std::max(2 * nmax + 1, (long)tune("getrf_oz_leaf", 4096.0));
     c.blk_nb = std::max(nmax, ((long)tune("getrf_nb", 512.0) + 63) / 64 * 64);
   }
-  return factor(c, 0, N);
+  return done(factor(c, 0, N));
 }

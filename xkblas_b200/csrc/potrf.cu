@@ -639,11 +639,25 @@ extern "C" int xkb_cuda_potrf(int dtype, int uplo, int N, void* A, long lda, int
   const int mode = (int)tune("potrf_blocked", 3.0);
   const long nb = std::max(nmax, ((long)tune(c.ozaki ? "potrf_nb_oz" : "potrf_nb", 512.0) + 63) /
                                      64 * 64);
-  if (N > 2 * nmax && (mode == 2 || ((mode == 1 || mode == 3) && c.ozaki == 0)))
-    return factor_blocked(c, 0, N, nb);
-  if (mode == 3 && c.ozaki > 0) {
-    c.blk_leaf = std::max(2 * nmax + 1, (long)tune("potrf_oz_leaf", 4096.0));
-    c.blk_nb = nb;
+  // a matrix TMA cannot read in place is factored in an aligned copy: one copy
+  // in and out instead of one per operand of every product
+  AlignedArray w;
+  int e = XKB_OK;
+  if (N > nmax && (e = w.take(A, lda, N, N, uplo, c.es, c.st))) return e;
+  if (w.buf) {
+    c.A = static_cast<char*>(w.p);
+    c.lda = w.ld;
   }
-  return factor(c, 0, N, true, false);
+  if (N > 2 * nmax && (mode == 2 || ((mode == 1 || mode == 3) && c.ozaki == 0))) {
+    e = factor_blocked(c, 0, N, nb);
+  } else {
+    if (mode == 3 && c.ozaki > 0) {
+      c.blk_leaf = std::max(2 * nmax + 1, (long)tune("potrf_oz_leaf", 4096.0));
+      c.blk_nb = nb;
+    }
+    e = factor(c, 0, N, true, false);
+  }
+  if (!e) e = w.put_back(c.st);
+  w.release(c.st);
+  return e;
 }

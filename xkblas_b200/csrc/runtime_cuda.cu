@@ -184,13 +184,29 @@ int sm_count() {
   return n;
 }
 
-static std::vector<ErrReader>& readers() {
-  static std::vector<ErrReader> r;
+static std::vector<ErrAddr>& error_addrs() {
+  static std::vector<ErrAddr> r;
   return r;
 }
-int register_error_reader(ErrReader r) {
-  readers().push_back(r);
+int register_error_addr(ErrAddr f) {
+  error_addrs().push_back(f);
   return 1;
+}
+
+// First error word that is set, in registration order; clears all.  One launch
+// and one wait for all units: read one by one, a blocking copy per unit made
+// up to 80 us of every xkblas_sync.
+constexpr int kMaxUnits = 32;
+struct ErrWords {
+  int* p[kMaxUnits];
+  int n;
+};
+__global__ void k_take_errors(const ErrWords w, int* out) {
+  const int t = threadIdx.x;
+  const int v = t < w.n ? atomicExch(w.p[t], 0) : 0;
+  const unsigned set = __ballot_sync(0xffffffffu, v != 0);
+  const int first = __shfl_sync(0xffffffffu, v, set ? __ffs((int)set) - 1 : 0);
+  if (t == 0) *out = first;
 }
 
 void set_library_stream(cudaStream_t s) { g_lib_stream = s; }
@@ -278,12 +294,37 @@ namespace xkb {
 }  // namespace xkb
 
 extern "C" int xkb_cuda_take_device_error(void) {
-  int v = 0;
-  for (auto r : xkb::readers()) {
-    int e = r();
-    if (e && !v) v = e;
+  using namespace xkb;
+  static std::mutex mu;
+  static int* host[64] = {nullptr};  // pinned result word and stream per device
+  static cudaStream_t stream[64] = {nullptr};
+  std::lock_guard<std::mutex> g(mu);
+  ErrWords w;
+  w.n = 0;
+  for (ErrAddr f : error_addrs())
+    if (void* p = f())
+      if (w.n < kMaxUnits) w.p[w.n++] = static_cast<int*>(p);
+  int dev = 0;
+  if (w.n == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    cudaGetLastError();
+    return 0;
   }
-  return v;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (!host[dev] &&
+        (cudaHostAlloc(reinterpret_cast<void**>(&host[dev]), sizeof(int), cudaHostAllocMapped) !=
+             cudaSuccess ||
+         cudaStreamCreateWithFlags(&stream[dev], cudaStreamNonBlocking) != cudaSuccess)) {
+      host[dev] = nullptr;
+      cudaGetLastError();
+      return 0;
+    }
+    k_take_errors<<<1, 32, 0, stream[dev]>>>(w, host[dev]);
+    if (cudaPeekAtLastError() == cudaSuccess && cudaStreamSynchronize(stream[dev]) == cudaSuccess)
+      return *static_cast<volatile int*>(host[dev]);
+    cudaGetLastError();
+    host[dev] = nullptr;  // gone with a reset context: make them again
+  }
+  return 0;
 }
 
 extern "C" uint64_t xkb_cuda_kernel_count(void) { return xkb::g_launches.load(); }

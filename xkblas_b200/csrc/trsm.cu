@@ -429,46 +429,63 @@ __global__ void __launch_bounds__(kBlkThreads, 2)
   }
 }
 
+// Triangle / full copies: a block takes 256 rows x 8 columns (no index
+// division; 8 loads in flight per thread).
 template <class T>
-__global__ void k_tri_fill(int n, const T* A, long lda, int lower, int unit, T* O, long ldo) {
-  const size_t total = (size_t)n * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    double re = 0, im = 0;
-    if (i == j && unit) re = 1.0;
-    else if (lower ? i >= j : i <= j) ldv<T>(A, (size_t)i + (size_t)j * lda, re, im);
-    stv<T>(O, (size_t)i + (size_t)j * ldo, re, im);
+__global__ void __launch_bounds__(256) k_tri_fill(int n, const T* A, long lda, int lower, int unit,
+                                                  T* O, long ldo) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  for (int c0 = blockIdx.y * 8; c0 < n; c0 += gridDim.y * 8) {
+    double re[8], im[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int j = c0 + q;
+      re[q] = im[q] = 0.0;
+      if (j >= n) continue;
+      if (i == j && unit) re[q] = 1.0;
+      else if (lower ? i >= j : i <= j) ldv<T>(A, (size_t)i + (size_t)j * lda, re[q], im[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (c0 + q < n) stv<T>(O, (size_t)i + (size_t)(c0 + q) * ldo, re[q], im[q]);
   }
 }
 
 // out = full symmetric (herm = 0) or Hermitian (herm = 1) matrix from the
-// stored uplo triangle of A; Hermitian diagonal taken real.
+// stored uplo triangle of A; Hermitian diagonal taken real.  Block (bi, bj),
+// bi >= bj, reads one 32 x 32 tile of the stored triangle and writes it and,
+// through shared memory, its mirror image: both stores run along columns.
 template <class T>
-__global__ void k_sym_fill(int n, const T* A, long lda, int lower, int herm, T* O, long ldo) {
-  const size_t total = (size_t)n * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    const bool stored = lower ? i >= j : i <= j;
-    double re, im;
-    if (stored) ldv<T>(A, (size_t)i + (size_t)j * lda, re, im);
-    else {
-      ldv<T>(A, (size_t)j + (size_t)i * lda, re, im);
-      if (herm) im = -im;
-    }
+__global__ void __launch_bounds__(256) k_sym_fill(int n, const T* A, long lda, int lower, int herm,
+                                                  T* O, long ldo) {
+  if (blockIdx.x < blockIdx.y) return;
+  __shared__ double tr[32][33], ti[TT<T>::C ? 32 : 1][33];
+  // stored tile: rows r0.., columns c0..
+  const int r0 = 32 * (lower ? blockIdx.x : blockIdx.y);
+  const int c0 = 32 * (lower ? blockIdx.y : blockIdx.x);
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = r0 + x, j = c0 + y + 8 * q;
+    double re = 0, im = 0;
+    if (i < n && j < n && (lower ? i >= j : i <= j)) ldv<T>(A, (size_t)i + (size_t)j * lda, re, im);
     if (herm && i == j) im = 0.0;
-    stv<T>(O, (size_t)i + (size_t)j * ldo, re, im);
+    tr[y + 8 * q][x] = re;  // [column][row]
+    if (TT<T>::C) ti[y + 8 * q][x] = im;
   }
-}
-
-template <class T>
-__global__ void k_copy2d(int m, int n, const T* S, long lds, T* D, long ldd) {
-  const size_t total = (size_t)m * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % m), j = (int)(e / m);
-    D[(size_t)i + (size_t)j * ldd] = S[(size_t)i + (size_t)j * lds];
+  __syncthreads();
+  const double sg = herm ? -1.0 : 1.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = y + 8 * q;
+    int i = r0 + x, j = c0 + k;  // the stored tile
+    if (i < n && j < n && (lower ? i >= j : i <= j))
+      stv<T>(O, (size_t)i + (size_t)j * ldo, tr[k][x], TT<T>::C ? ti[k][x] : 0.0);
+    i = c0 + x;  // its mirror image
+    j = r0 + k;
+    if (i < n && j < n && (lower ? i < j : i > j))
+      stv<T>(O, (size_t)i + (size_t)j * ldo, tr[x][k], TT<T>::C ? sg * ti[x][k] : 0.0);
   }
 }
 
@@ -482,10 +499,9 @@ static int esize(int dt) {
   return 0;
 }
 
-static unsigned grid_for(size_t total, int per_block = 256) {
-  size_t b = (total + per_block - 1) / per_block;
-  const size_t cap = (size_t)sm_count() * 16;
-  return (unsigned)std::max<size_t>(1, std::min(b, cap));
+// grid of the 256-row x 8-column copy kernels
+static dim3 copy_grid(long rows, long cols) {
+  return dim3((unsigned)((rows + 255) / 256), (unsigned)std::min<long>((cols + 7) / 8, 32768));
 }
 
 template <class T>
@@ -966,8 +982,24 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
 extern "C" int xkb_cuda_trsm(int dtype, int side, int uplo, int trans, int diag, int M, int N,
                              const double* alpha, const void* A, long lda, void* B, long ldb,
                              int ozaki, void* stream) {
-  return trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, A, lda, B, ldb, ozaki,
-                    resolve_stream(stream), true);
+  const long n = side == 0 ? M : N;
+  cudaStream_t st = resolve_stream(stream);
+  if (dtype < XKB_S || dtype > XKB_Z || M <= 0 || N <= 0 || n <= kBlk || !A || !B)
+    return trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, A, lda, B, ldb, ozaki, st,
+                      true);
+  // operands TMA cannot read in place: one aligned copy each instead of one per
+  // coupling product
+  const int es = esize(dtype);
+  AlignedArray wa, wb;
+  int e = wa.take(const_cast<void*>(A), lda, (int)n, (int)n, uplo, es, st);
+  if (!e) e = wb.take(B, ldb, M, N, XKB_FULL, es, st);
+  if (!e)
+    e = trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, wa.p, wa.ld, wb.p, wb.ld, ozaki,
+                   st, true);
+  if (!e) e = wb.put_back(st);
+  wa.release(st);
+  wb.release(st);
+  return e;
 }
 
 // The product on the materialised operand: Ozaki INT8 form when ozaki > 0,
@@ -997,29 +1029,19 @@ extern "C" int xkb_cuda_trmm(int dtype, int side, int uplo, int trans, int diag,
     cudaFreeAsync(T, st);
     return XKB_ENOMEM;
   }
-  const unsigned g1 = grid_for((size_t)na * na), g2 = grid_for((size_t)M * N);
+  const dim3 g1 = copy_grid(na, na);
   const int lower = uplo == XKB_LOWER, unit = diag != 0;
+  const CopyArray bc{B, Bc, ldb, ldc, M, N, XKB_FULL};
   const long long tv = evlog_kern_begin(st, "k_tri_fill+k_copy2d");
   switch (dtype) {
-    case XKB_S:
-      k_tri_fill<float><<<g1, 256, 0, st>>>((int)na, (const float*)A, lda, lower, unit, (float*)T, ldt);
-      k_copy2d<float><<<g2, 256, 0, st>>>(M, N, (const float*)B, ldb, (float*)Bc, ldc);
-      break;
-    case XKB_D:
-      k_tri_fill<double><<<g1, 256, 0, st>>>((int)na, (const double*)A, lda, lower, unit, (double*)T, ldt);
-      k_copy2d<double><<<g2, 256, 0, st>>>(M, N, (const double*)B, ldb, (double*)Bc, ldc);
-      break;
-    case XKB_C:
-      k_tri_fill<float2><<<g1, 256, 0, st>>>((int)na, (const float2*)A, lda, lower, unit, (float2*)T, ldt);
-      k_copy2d<float2><<<g2, 256, 0, st>>>(M, N, (const float2*)B, ldb, (float2*)Bc, ldc);
-      break;
-    case XKB_Z:
-      k_tri_fill<double2><<<g1, 256, 0, st>>>((int)na, (const double2*)A, lda, lower, unit, (double2*)T, ldt);
-      k_copy2d<double2><<<g2, 256, 0, st>>>(M, N, (const double2*)B, ldb, (double2*)Bc, ldc);
-      break;
+    case XKB_S: k_tri_fill<float><<<g1, 256, 0, st>>>((int)na, (const float*)A, lda, lower, unit, (float*)T, ldt); break;
+    case XKB_D: k_tri_fill<double><<<g1, 256, 0, st>>>((int)na, (const double*)A, lda, lower, unit, (double*)T, ldt); break;
+    case XKB_C: k_tri_fill<float2><<<g1, 256, 0, st>>>((int)na, (const float2*)A, lda, lower, unit, (float2*)T, ldt); break;
+    case XKB_Z: k_tri_fill<double2><<<g1, 256, 0, st>>>((int)na, (const double2*)A, lda, lower, unit, (double2*)T, ldt); break;
   }
   evlog_kern_end(tv, st);
-  count_launch(2);
+  count_launch();
+  int e = copy_arrays(&bc, 1, es, st);
   xkb_gemm_args g{};
   g.dtype = dtype;
   g.M = M;
@@ -1046,7 +1068,7 @@ extern "C" int xkb_cuda_trmm(int dtype, int side, int uplo, int trans, int diag,
   }
   g.C = B;
   g.ldc = ldb;
-  int e = product(g, ozaki, st);
+  if (!e) e = product(g, ozaki, st);
   cudaFreeAsync(T, st);
   cudaFreeAsync(Bc, st);
   return e;
@@ -1064,7 +1086,8 @@ extern "C" int xkb_cuda_symm(int dtype, int herm, int side, int uplo, int M, int
   const long ldt = (na + 31) / 32 * 32;
   void* S = nullptr;
   if (cudaMallocAsync(&S, (size_t)ldt * na * es, st) != cudaSuccess) return XKB_ENOMEM;
-  const unsigned g1 = grid_for((size_t)na * na);
+  const unsigned nb32 = (unsigned)((na + 31) / 32);
+  const dim3 g1(nb32, nb32);
   const int lower = uplo == XKB_LOWER;
   const int hm = herm && (dtype == XKB_C || dtype == XKB_Z);
   const long long tv = evlog_kern_begin(st, "k_sym_fill");

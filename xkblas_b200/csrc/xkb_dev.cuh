@@ -16,7 +16,7 @@ namespace xkb {
 constexpr uint64_t kWaitLimitNs = 4000000000ull;  // 4 s
 
 // Device error word, one per translation unit (no relocatable device code);
-// each unit registers a reader so xkb_cuda_take_device_error() sees all.
+// each unit registers its address so xkb_cuda_take_device_error() sees all.
 static __device__ int g_dev_error;
 
 enum DevErr : int {  // the XKB_DEV_* words of xkb_cuda.h
@@ -110,16 +110,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
 
 // Host-side helpers shared by the launch code (defined in runtime_cuda.cu).
 namespace xkb {
-typedef int (*ErrReader)();
-int register_error_reader(ErrReader r);
-// Reads and clears this unit's error word.
-static int take_unit_error() {
-  int v = 0, z = 0;
-  if (cudaMemcpyFromSymbol(&v, g_dev_error, sizeof v) != cudaSuccess) return 0;
-  if (v) cudaMemcpyToSymbol(g_dev_error, &z, sizeof z);
-  return v;
+// Each unit registers the device address of its error word.
+typedef void* (*ErrAddr)();
+int register_error_addr(ErrAddr f);
+static void* unit_error_addr() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_dev_error) == cudaSuccess ? p : nullptr;
 }
-static int g_unit_reader_registered = register_error_reader(&take_unit_error);
+static int g_unit_error_registered = register_error_addr(&unit_error_addr);
 // Encode a 2-D tiled tensor map: rows x cols column-major with leading
 // dimension ld (elements of `elem_bytes`), box bx (along rows) x by.
 // Returns false if the driver entry point is missing or encoding fails.
@@ -171,6 +169,52 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
 // xkb_cuda_gemm whose kernel runs only where the device word *run_if is
 // non-zero (gemm_dmma.cu): the plain fallback of a data-chosen Ozaki call.
 int gemm_if(const xkb_gemm_args* a, const int* run_if, cudaStream_t st);
+// TMA operands: base and leading dimension multiples of 16 bytes.
+bool tma_ok(const void* p, long ld, int es);
+long packed_ld(long rows, int es);
+// One launch copying up to two rows x cols arrays of es-byte elements (uplo:
+// only that triangle's elements); run_if as for gemm_if (gemm_dmma.cu).
+struct CopyArray {
+  const void* src;
+  void* dst;
+  long lds, ldd;
+  int rows, cols, uplo;
+};
+int copy_arrays(const CopyArray* d, int n, int es, cudaStream_t st, const int* run_if = nullptr);
+// An array some of whose solves / factorization's products go through TMA, as
+// an aligned copy when its base or leading dimension is not: p, ld give the
+// array to work on; put_back() copies the uplo part of the result into the
+// array (out only) and release() frees the copy.  Without memory for a copy
+// the products repack their operands one by one instead.
+struct AlignedArray {
+  void* p = nullptr;
+  long ld = 0;
+  void* buf = nullptr;
+  CopyArray back{};
+  int es = 0;
+  int take(void* a, long lda, int rows, int cols, int uplo, int es_, cudaStream_t st) {
+    p = a;
+    ld = lda;
+    es = es_;
+    if (tma_ok(a, lda, es)) return XKB_OK;
+    const long l = packed_ld(rows, es);
+    if (cudaMallocAsync(&buf, (size_t)l * cols * es, st) != cudaSuccess) {
+      cudaGetLastError();
+      buf = nullptr;
+      return XKB_OK;
+    }
+    back = {buf, a, l, lda, rows, cols, uplo};
+    const CopyArray in{a, buf, lda, l, rows, cols, uplo};
+    p = buf;
+    ld = l;
+    return copy_arrays(&in, 1, es, st);
+  }
+  int put_back(cudaStream_t st) { return buf ? copy_arrays(&back, 1, es, st) : XKB_OK; }
+  void release(cudaStream_t st) {
+    if (buf) cudaFreeAsync(buf, st);
+    buf = nullptr;
+  }
+};
 // A large single-precision product by exact INT8 arithmetic (ozaki.cu);
 // XKB_ERANGE / XKB_ENOMEM: not taken, nothing was launched.
 int gemm_exact(const xkb_gemm_args* a, cudaStream_t st);
