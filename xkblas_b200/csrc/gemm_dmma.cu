@@ -84,6 +84,8 @@ struct CopyWords {
 template <class W>
 __global__ void __launch_bounds__(256) k_repack(const CopyWords d0, const CopyWords d1,
                                                 const int* run_if) {
+  pdl_wait();
+  pdl_launch();
   if (run_if && *run_if == 0) return;
   const CopyWords& d = blockIdx.z ? d1 : d0;
   const int r = blockIdx.x * 256 + threadIdx.x;
@@ -122,8 +124,7 @@ int copy_arrays(const CopyArray* d, int n, int es, cudaStream_t st, const int* r
   if (n == 1) w[1] = w[0];
   const dim3 g((unsigned)((mr + 255) / 256), (unsigned)std::min((mc + 7) / 8, 32768), (unsigned)n);
   const long long tv = evlog_kern_begin(st, "k_repack");
-  if (wide) k_repack<double><<<g, 256, 0, st>>>(w[0], w[1], run_if);
-  else k_repack<float><<<g, 256, 0, st>>>(w[0], w[1], run_if);
+  launch_pdl(wide ? k_repack<double> : k_repack<float>, g, dim3(256), 0, st, w[0], w[1], run_if);
   evlog_kern_end(tv, st);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;

@@ -302,10 +302,6 @@ template <class C_, bool A_KC, bool B_KC>
 __global__ void __launch_bounds__(C_::CTA, C_::MINB)
     k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const GemmParams p) {
-  // a launch predicated on a device word (the Ozaki data rule's plain
-  // fallback): every thread reads the same word, so the whole CTA leaves
-  // before touching shared memory, barriers or C
-  if (p.run_if && *p.run_if == 0) return;
   constexpr int STG = C_::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -316,9 +312,6 @@ __global__ void __launch_bounds__(C_::CTA, C_::MINB)
   const int ntiles = p.tiles_m * p.tiles_n;
   const int slice = (int)blockIdx.x / ntiles;  // 0 unless split-K
   const int bid = (int)blockIdx.x - slice * ntiles;
-  int m0, n0;
-  if (!dmma_tile<C_::BM, C_::BN>(p, bid, m0, n0)) return;
-
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     tma_prefetch(&tmA);
@@ -329,6 +322,14 @@ __global__ void __launch_bounds__(C_::CTA, C_::MINB)
     }
     fence_barrier_init();
   }
+  pdl_wait();
+  pdl_launch();
+  // a launch predicated on a device word (the Ozaki data rule's plain
+  // fallback): every thread reads the same word, so the whole CTA leaves
+  // before touching shared memory, barriers or C
+  if (p.run_if && *p.run_if == 0) return;
+  int m0, n0;
+  if (!dmma_tile<C_::BM, C_::BN>(p, bid, m0, n0)) return;
   __syncthreads();
 
   // this CTA's stages: [kt0, kt0 + KT)
@@ -418,6 +419,8 @@ __device__ __forceinline__ void sum_slots(const double* w0, size_t stride, int n
 // block per (tile, fragment) spreads the reads of the slices over many SMs.
 template <class C_, bool A_KC, bool B_KC>
 __global__ void __launch_bounds__(C_::THREADS) k_gemm_splitk(const GemmParams p) {
+  pdl_wait();
+  pdl_launch();
   if (p.run_if && *p.run_if == 0) return;
   constexpr int NACC = C_::NACC, STRIDE = C_::NREG * C_::THREADS;
   const int ntiles = p.tiles_m * p.tiles_n;
@@ -499,15 +502,17 @@ static int launch_dmma(const xkb_gemm_args* a, cudaStream_t st, const int* run_i
   }
   const long long tv = evlog_kern_begin(st, p.ksplit > 1 ? "k_gemm_dmma+k_gemm_splitk"
                                                          : "k_gemm_dmma");
-  kern<<<(unsigned)(ntiles * p.ksplit), C_::CTA, C_::SMEM, st>>>(tA, tB, p);
+  cudaError_t le =
+      launch_pdl(kern, dim3((unsigned)(ntiles * p.ksplit)), dim3(C_::CTA), C_::SMEM, st, tA, tB, p);
   if (p.ksplit > 1) {
     const dim3 rg((unsigned)ntiles, (unsigned)FRAGS);
-    k_gemm_splitk<C_, A_KC, B_KC><<<rg, C_::THREADS, 0, st>>>(p);
+    if (le == cudaSuccess)
+      le = launch_pdl(k_gemm_splitk<C_, A_KC, B_KC>, rg, dim3(C_::THREADS), 0, st, p);
     cudaFreeAsync(p.ws, st);
   }
   evlog_kern_end(tv, st);
   count_launch(p.ksplit > 1 ? 2 : 1);
-  return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
+  return le == cudaSuccess && cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
 }
 
 template <class C_>

@@ -55,6 +55,8 @@ __global__ void __launch_bounds__(kLuThreads, 1)
   constexpr int LD = Sh::LD;
   constexpr int W = CP ? 2 : 1;
   extern __shared__ double sm_lu[];
+  pdl_wait();
+  pdl_launch();
   double* Xr = sm_lu;  // A(i, k) at X[k * LD + i]
   double* Xi = Xr + (CP ? Sh::COLS * LD : 0);
   double* Fr = sm_lu + (size_t)Sh::PL * Sh::COLS * LD;  // 8 x 8 factors (L below, U on/above)
@@ -343,7 +345,8 @@ static int launch_block(const LuCtx& c, char* Ad, long n, long i0) {
     attr = true;
   }
   const long long tv = evlog_kern_begin(c.st, "k_getrf_block");
-  k_getrf_block<T><<<1, kLuThreads, Sh::SMEM, c.st>>>(
+  launch_pdl(
+      k_getrf_block<T>, dim3(1), dim3(kLuThreads), Sh::SMEM, c.st,
       (int)n, reinterpret_cast<typename St<T>::S*>(Ad), c.lda, (int)i0, c.info);
   evlog_kern_end(tv, c.st);
   count_launch();

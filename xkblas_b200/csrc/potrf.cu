@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(kPoThreads, 1)
   constexpr int W = CP ? 2 : 1;
   constexpr unsigned FULL = 0xffffffffu;
   extern __shared__ double sm_po[];
+  pdl_wait();
+  pdl_launch();
   double* Xr = sm_po;  // L(i, k) at X[k * LD + i], lower part only
   double* Xi = Xr + (CP ? Sh::COLS * LD : 0);
   double* Lsr = sm_po + (size_t)Sh::PL * Sh::COLS * LD;  // 8 x 8 factor, [i][k]
@@ -346,8 +348,8 @@ static int launch_leaf(const PotrfCtx& c, char* Ad, long n, long i0) {
     attr = true;
   }
   const long long tv = evlog_kern_begin(c.st, "k_potrf_block");
-  k_potrf_block<T><<<1, kPoThreads, Sh::SMEM, c.st>>>(
-      (int)n, reinterpret_cast<typename St<T>::S*>(Ad), c.lda, c.upper, (int)i0, c.info);
+  launch_pdl(
+      k_potrf_block<T>, dim3(1), dim3(kPoThreads), Sh::SMEM, c.st, (int)n, reinterpret_cast<typename St<T>::S*>(Ad), c.lda, c.upper, (int)i0, c.info);
   evlog_kern_end(tv, c.st);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;

@@ -127,6 +127,8 @@ __global__ void __launch_bounds__(kBlkThreads, 2)
   constexpr bool CP = Sh::CP;
   constexpr int CW = Sh::CW, XS = Sh::XS, YW = Sh::YW, SRL = Sh::SRL, PE = Sh::PE;
   constexpr int W = CP ? 2 : 1;
+  pdl_wait();
+  pdl_launch();
   int nb = nb_, nrhs = nrhs_;
   const S* A = A_;
   S* B = B_;
@@ -434,6 +436,8 @@ __global__ void __launch_bounds__(kBlkThreads, 2)
 template <class T>
 __global__ void __launch_bounds__(256) k_tri_fill(int n, const T* A, long lda, int lower, int unit,
                                                   T* O, long ldo) {
+  pdl_wait();
+  pdl_launch();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   for (int c0 = blockIdx.y * 8; c0 < n; c0 += gridDim.y * 8) {
@@ -459,6 +463,8 @@ __global__ void __launch_bounds__(256) k_tri_fill(int n, const T* A, long lda, i
 template <class T>
 __global__ void __launch_bounds__(256) k_sym_fill(int n, const T* A, long lda, int lower, int herm,
                                                   T* O, long ldo) {
+  pdl_wait();
+  pdl_launch();
   if (blockIdx.x < blockIdx.y) return;
   __shared__ double tr[32][33], ti[TT<T>::C ? 32 : 1][33];
   // stored tile: rows r0.., columns c0..
@@ -522,9 +528,8 @@ static int launch_block(int n, int nrhs, const void* A, long lda, int swap, int 
     attr[lower ? 1 : 0] = true;
   }
   const long long tv = evlog_kern_begin(st, "k_trsm_block");
-  kb<<<grid, kBlkThreads, Sh::SMEM, st>>>(n, nrhs, static_cast<const S*>(A), lda, swap, conj,
-                                          unit, static_cast<S*>(B), ldb, rhs_rows, al[0], al[1],
-                                          leaves);
+  launch_pdl(kb, grid, dim3(kBlkThreads), Sh::SMEM, st, n, nrhs, static_cast<const S*>(A), lda, swap,
+             conj, unit, static_cast<S*>(B), ldb, rhs_rows, al[0], al[1], leaves);
   evlog_kern_end(tv, st);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
@@ -1034,10 +1039,10 @@ extern "C" int xkb_cuda_trmm(int dtype, int side, int uplo, int trans, int diag,
   const CopyArray bc{B, Bc, ldb, ldc, M, N, XKB_FULL};
   const long long tv = evlog_kern_begin(st, "k_tri_fill+k_copy2d");
   switch (dtype) {
-    case XKB_S: k_tri_fill<float><<<g1, 256, 0, st>>>((int)na, (const float*)A, lda, lower, unit, (float*)T, ldt); break;
-    case XKB_D: k_tri_fill<double><<<g1, 256, 0, st>>>((int)na, (const double*)A, lda, lower, unit, (double*)T, ldt); break;
-    case XKB_C: k_tri_fill<float2><<<g1, 256, 0, st>>>((int)na, (const float2*)A, lda, lower, unit, (float2*)T, ldt); break;
-    case XKB_Z: k_tri_fill<double2><<<g1, 256, 0, st>>>((int)na, (const double2*)A, lda, lower, unit, (double2*)T, ldt); break;
+    case XKB_S: launch_pdl(k_tri_fill<float>, g1, dim3(256), 0, st, (int)na, (const float*)A, lda, lower, unit, (float*)T, ldt); break;
+    case XKB_D: launch_pdl(k_tri_fill<double>, g1, dim3(256), 0, st, (int)na, (const double*)A, lda, lower, unit, (double*)T, ldt); break;
+    case XKB_C: launch_pdl(k_tri_fill<float2>, g1, dim3(256), 0, st, (int)na, (const float2*)A, lda, lower, unit, (float2*)T, ldt); break;
+    case XKB_Z: launch_pdl(k_tri_fill<double2>, g1, dim3(256), 0, st, (int)na, (const double2*)A, lda, lower, unit, (double2*)T, ldt); break;
   }
   evlog_kern_end(tv, st);
   count_launch();
@@ -1092,10 +1097,10 @@ extern "C" int xkb_cuda_symm(int dtype, int herm, int side, int uplo, int M, int
   const int hm = herm && (dtype == XKB_C || dtype == XKB_Z);
   const long long tv = evlog_kern_begin(st, "k_sym_fill");
   switch (dtype) {
-    case XKB_S: k_sym_fill<float><<<g1, 256, 0, st>>>((int)na, (const float*)A, lda, lower, 0, (float*)S, ldt); break;
-    case XKB_D: k_sym_fill<double><<<g1, 256, 0, st>>>((int)na, (const double*)A, lda, lower, 0, (double*)S, ldt); break;
-    case XKB_C: k_sym_fill<float2><<<g1, 256, 0, st>>>((int)na, (const float2*)A, lda, lower, hm, (float2*)S, ldt); break;
-    case XKB_Z: k_sym_fill<double2><<<g1, 256, 0, st>>>((int)na, (const double2*)A, lda, lower, hm, (double2*)S, ldt); break;
+    case XKB_S: launch_pdl(k_sym_fill<float>, g1, dim3(256), 0, st, (int)na, (const float*)A, lda, lower, 0, (float*)S, ldt); break;
+    case XKB_D: launch_pdl(k_sym_fill<double>, g1, dim3(256), 0, st, (int)na, (const double*)A, lda, lower, 0, (double*)S, ldt); break;
+    case XKB_C: launch_pdl(k_sym_fill<float2>, g1, dim3(256), 0, st, (int)na, (const float2*)A, lda, lower, hm, (float2*)S, ldt); break;
+    case XKB_Z: launch_pdl(k_sym_fill<double2>, g1, dim3(256), 0, st, (int)na, (const double2*)A, lda, lower, hm, (double2*)S, ldt); break;
   }
   evlog_kern_end(tv, st);
   count_launch();

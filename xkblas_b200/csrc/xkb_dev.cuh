@@ -91,6 +91,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
   }
 }
 
+// ---- programmatic dependent launch --------------------------------------------
+// Kernels launched with launch_pdl start while the previous kernel of their
+// stream drains: they call pdl_wait before they touch global memory (every
+// thread of every block, before any early return, so that a grid never ends
+// before its predecessor has) and pdl_launch to let their own successor start.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -110,6 +122,22 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
 
 // Host-side helpers shared by the launch code (defined in runtime_cuda.cu).
 namespace xkb {
+// Launch of a kernel that calls pdl_wait (see above).
+template <class... KA, class... A>
+inline cudaError_t launch_pdl(void (*k)(KA...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, KA(args)...);
+}
 // Each unit registers the device address of its error word.
 typedef void* (*ErrAddr)();
 int register_error_addr(ErrAddr f);
