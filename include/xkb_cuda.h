@@ -71,7 +71,10 @@ typedef struct xkb_gemm_args {
 } xkb_gemm_args;
 
 /* C <- alpha*op(A)*op(B) + beta*C on the masked part of C, FP64 DMMA
- * tensor cores (float storage computed in double and rounded once). */
+ * tensor cores (float storage computed in double and rounded once; large S
+ * and C products whose operands fit are computed exactly on the INT8 tensor
+ * cores and rounded to double, then to float: the device decides, the plain
+ * kernel runs otherwise). */
 int xkb_cuda_gemm(const xkb_gemm_args* a, void* stream);
 
 /* Triangular solve, all side/uplo/trans/diag cases:
@@ -241,15 +244,17 @@ int xkb_cuda_batch_release(void);
 /* Tuning table: choices measured on the device by the autotuner
  * (python -m xkblas_b200.autotune --out FILE; the runtime loads
  * XKBLAS_TUNE_FILE at init).  Keys (built-in default):
- *   gemm_big_min_tiles      whole-matrix GEMM uses 128-wide tiles when it has
- *                           at least this many of them (SM count)
+ *   gemm_big_min_tiles      real whole-matrix GEMM uses 64 x 64 tiles when C has
+ *                           at least this many 128 x 128 blocks, else 32 x 32
+ *                           ones (unset: chosen by a model of the time)
+ *   gemm_exact              large S / C products by exact INT8 arithmetic where
+ *                           the operands allow it (1); gemm_exact_min: from
+ *                           this M N K on (3.4e9; C a quarter of it)
  *   ozaki_min_dim           tensor-op mode uses Ozaki when min(M,N,K) >= (2048;
  *                           read per call; XKBLAS_OZAKI_MIN_DIM overrides)
  *   ozaki_moduli_k<=<K>     moduli count for contractions with inner size <= K
  *                           (the smallest band covering K; else the K rule)
  *   batch_schedule          executor claim order, 0 solves first / 1 gemms (0)
- *   batch_tile128_min_rows  executor: real gemm calls this tall use 128-row
- *                           tiles (96)
  *   oz_group_m              Ozaki INT8 GEMM raster: M tiles per group of the
  *                           persistent tile walk (8)
  *   oz_2cta                 Ozaki INT8 GEMM on CTA pairs (tcgen05 cta_group::2,

@@ -12,9 +12,10 @@
 // banks.  Two free permutations make that possible without copying: which
 // physical k a lane's two MMA k slots hold (the same for A and B, so sums
 // are unchanged), and which physical row an MMA row (column of op(B)) is
-// (undone where the accumulators are stored).  MMA row g + 8h of a 16-row
-// block is physical row 2 perm(g) + h, so a lane's two accumulator rows are
-// neighbours in memory and C moves in 16-byte accesses.
+// (undone where the accumulators are stored).  Where elements are 4 or 8
+// bytes, MMA row g + 8h of a 16-row block is physical row 2 q(g) + h, so a
+// lane's two accumulator rows are neighbours in memory and C moves in 8- and
+// 16-byte accesses.
 // Without the swizzle (rows at 128-byte or 1 KB strides) the A loads had
 // 4-way and the B loads 2-way bank conflicts: hidden behind the DMMA pipe in
 // 128 x 128 tiles, but 64 x 64 tiles then ran at 74 % of the big tiles' rate
@@ -29,14 +30,16 @@ struct OpTile {
   static constexpr int ES = (int)sizeof(T);
   static constexpr int BK = 128 / ES;   // k per stage; rows per panel when !KC
   static constexpr int KS = BK / 8;     // MMA k steps per stage (double complex: 1)
-  static constexpr bool SWAP = ES == 16 || (ES == 8 && KC);
+  // rows between a lane's two accumulator rows: neighbours, or (16-byte
+  // elements, one access each) MMA rows g and g + 8 where they are
+  static constexpr int PS = ES == 16 ? 8 : 1;
 
-  // physical row pair of MMA row g (0..7)
-  static __device__ __forceinline__ int perm(int g) {
-    return SWAP ? ((g >> 1) & 1) | ((g & 1) << 1) | (g & 4) : g;
-  }
   // physical row in a 16-row block of MMA row g + 8h
-  static __device__ __forceinline__ int prow(int g, int h) { return 2 * perm(g) + h; }
+  static __device__ __forceinline__ int prow(int g, int h) {
+    if (ES == 16) return g + 8 * h;
+    const int q = ES == 8 && KC ? ((g >> 1) & 1) | ((g & 1) << 1) | (g & 4) : g;
+    return 2 * q + h;
+  }
 
   // byte offset of element (row r, k) in the tile
   static __device__ __forceinline__ int off(int r, int k) {
@@ -45,7 +48,7 @@ struct OpTile {
   }
   // physical k of this lane's MMA k slot v (0, 1) in step kc
   static __device__ __forceinline__ int kof(int t, int v, int kc) {
-    return ES == 16 ? t + 4 * v : kc * 8 + 2 * t + v;
+    return kc * 8 + 2 * t + v;
   }
 
   // Rows [r0, r0 + 16) (r0 a multiple of 16), k step kc: re/im[h][v] = element
@@ -102,17 +105,18 @@ __device__ __forceinline__ double xor_sign(double x, unsigned flip) {
   return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
 }
 
-// Two values of C in neighbouring rows, or one when `two` is false; vec: the
-// pair is one aligned access.
+// Two values of C, PS rows apart (see OpTile); one, two: which of them are
+// wanted; vec: aligned for one access (16-byte elements: one each).
 template <class T>
 __device__ __forceinline__ void ld_pair(const typename St<T>::S* c, bool vec, bool one, bool two,
                                         double (&re)[2], double (&im)[2]) {
   using S = typename St<T>::S;
+  constexpr int D = St<T>::W * OpTile<T, true>::PS;
   re[0] = re[1] = im[0] = im[1] = 0.0;
   if (vec && one && two) {
     if constexpr (sizeof(T) == 16) {
       const double2 a = reinterpret_cast<const double2*>(c)[0];
-      const double2 b = reinterpret_cast<const double2*>(c)[1];
+      const double2 b = *reinterpret_cast<const double2*>(c + D);
       re[0] = a.x, im[0] = a.y, re[1] = b.x, im[1] = b.y;
     } else if constexpr (St<T>::CPLX) {
       const float4 a = *reinterpret_cast<const float4*>(c);
@@ -131,18 +135,19 @@ __device__ __forceinline__ void ld_pair(const typename St<T>::S* c, bool vec, bo
     if (St<T>::CPLX) im[0] = (double)c[1];
   }
   if (two) {
-    re[1] = (double)c[St<T>::W];
-    if (St<T>::CPLX) im[1] = (double)c[St<T>::CPLX ? 3 : 1];
+    re[1] = (double)c[D];
+    if (St<T>::CPLX) im[1] = (double)c[D + 1];
   }
 }
 template <class T>
 __device__ __forceinline__ void st_pair(typename St<T>::S* c, bool vec, bool one, bool two,
                                         const double (&re)[2], const double (&im)[2]) {
   using S = typename St<T>::S;
+  constexpr int D = St<T>::W * OpTile<T, true>::PS;
   if (vec && one && two) {
     if constexpr (sizeof(T) == 16) {
       reinterpret_cast<double2*>(c)[0] = make_double2(re[0], im[0]);
-      reinterpret_cast<double2*>(c)[1] = make_double2(re[1], im[1]);
+      *reinterpret_cast<double2*>(c + D) = make_double2(re[1], im[1]);
     } else if constexpr (St<T>::CPLX) {
       *reinterpret_cast<float4*>(c) =
           make_float4((float)re[0], (float)im[0], (float)re[1], (float)im[1]);
@@ -158,8 +163,8 @@ __device__ __forceinline__ void st_pair(typename St<T>::S* c, bool vec, bool one
     if (St<T>::CPLX) c[1] = static_cast<S>(im[0]);
   }
   if (two) {
-    c[St<T>::W] = static_cast<S>(re[1]);
-    if (St<T>::CPLX) c[St<T>::CPLX ? 3 : 1] = static_cast<S>(im[1]);
+    c[D] = static_cast<S>(re[1]);
+    if (St<T>::CPLX) c[D + 1] = static_cast<S>(im[1]);
   }
 }
 

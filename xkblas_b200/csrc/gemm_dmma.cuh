@@ -69,8 +69,8 @@ struct Cfg {
 };
 
 // The pair of C elements of this thread in fragment (mf, nf), column slot
-// i & 1: rows row, row + 1 of column col; `one`, `two`: which of them lie in
-// C and the triangle mask.
+// i & 1: rows row, row + PS (see OpTile) of column col; `one`, `two`: which of
+// them lie in C and the triangle mask.
 template <class C_, bool A_KC, bool B_KC>
 __device__ __forceinline__ void dmma_elem(const GemmParams& p, int m0, int n0, int mf, int nf,
                                           int i, int& row, int& col, bool& one, bool& two) {
@@ -81,7 +81,8 @@ __device__ __forceinline__ void dmma_elem(const GemmParams& p, int m0, int n0, i
   row = m0 + wm * C_::WTM + mf * 16 + OpTile<T, A_KC>::prow(g, 0);
   col = n0 + wn * C_::WTN + (nf >> 1) * 16 + OpTile<T, B_KC>::prow(2 * t + (i & 1), nf & 1);
   one = row < p.M && col < p.N && in_mask(p.uplo, p.diag, row, col);
-  two = row + 1 < p.M && col < p.N && in_mask(p.uplo, p.diag, row + 1, col);
+  constexpr int PS = OpTile<T, A_KC>::PS;
+  two = row + PS < p.M && col < p.N && in_mask(p.uplo, p.diag, row + PS, col);
 }
 
 // The C values of fragment (mf, nf) that beta multiplies: cv[i] in
@@ -137,7 +138,7 @@ __device__ __forceinline__ void dmma_store_frag(const GemmParams& p, int m0, int
         im[h] = p.ar * a[4 + v] + p.ai * a[v];
         re[h] += p.br * cv[v] - p.bi * cv[4 + v];
         im[h] += p.br * cv[4 + v] + p.bi * cv[v];
-        if (p.herm_diag && (long)(row + h) + p.diag == (long)col) im[h] = 0.0;
+        if (p.herm_diag && (long)(row + h * OpTile<T, A_KC>::PS) + p.diag == (long)col) im[h] = 0.0;
       } else {
         re[h] = fma(p.br, cv[v], p.ar * a[v]);
       }

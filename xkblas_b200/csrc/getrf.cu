@@ -431,7 +431,7 @@ static int factor(const LuCtx& c, long i0, long i1) {
 // width (tuning key getrf_shrink, default 12): wide blocks while the
 // trailing update bounds each step, narrow ones once the critical path does.
 static long block_width(long m, long nb, long nmin) {
-  const double shrink = tune("getrf_shrink", 12.0);
+  const double shrink = tune("getrf_shrink", 16.0);
   long w = nb;
   while (w > nmin && (double)m <= shrink * (double)w) w = std::max(nmin, (w / 2) / 64 * 64);
   return w;

@@ -12,12 +12,15 @@
 // instead of one launch (or thousands of tile tasks with host round trips)
 // per call.
 //
-// Task bodies (256 threads):
-//   gemm     C[<=BM x <=BN] = alpha op(A) op(B) + beta C over the full K,
-//            cp.async 3-stage shared-memory ring (16-byte copies, or 8-byte
-//            L2 loads when a leading dimension is odd; zero fill at ragged
-//            edges), DMMA m16n8k8; BM x BN = 64 x 64 (real), 32 x 64
-//            (complex, four real MMAs per product);
+// Task bodies (four MMA warps and a copy warp, three CTAs per SM):
+//   gemm     C[<=BM x <=BN] = alpha op(A) op(B) + beta C over the full K, with
+//            the operand tiles, fragments and epilogue of the whole-matrix GEMM
+//            (dmma_tile.cuh, gemm_dmma.cuh); the copy warp fills its 4-stage
+//            ring by cp.async (16-byte copies, 8-byte ones for an operand not
+//            16-byte aligned; zero fill at ragged edges), since a batch has no
+//            tensor maps; BM x BN = 64 x 64 (real), 32 x 32 (complex).  Before
+//            (eight warps that copied and multiplied, a CTA barrier per stage,
+//            128 x 64 tiles, two CTAs per SM): 22 TFLOP/s on mixed DGEMM calls;
 //   trsm     one 64-row block X_i of a left triangular solve against up to
 //            64 right-hand sides, left-looking: X_i = alpha B_i - sum_k
 //            op(A)[i,k] X_k over the blocks already solved (one gemm tile
@@ -29,15 +32,15 @@
 //            registers once instead of read-modified-written per step.
 // Ordering rules: a producer stores, then __syncthreads, then thread 0
 // issues __threadfence and decrements its successors' dependency counts;
-// the consumer's thread 0 takes the queued task, issues __threadfence, and
-// the CTA reads through L2 (cp.async.cg / ld.global.cg) -- no stale L1
-// lines, no async-proxy reads.
+// the consumer's thread 0 takes the queued task, issues __threadfence (a
+// gpu-scope acquire, which also leaves no stale L1 line), and after the CTA's
+// barrier every warp reads what the producers wrote -- no async-proxy reads.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
-#include "dmma_common.cuh"
+#include "gemm_dmma.cuh"
 #include "trsm_leaf.cuh"
 #include "xkb_dev.cuh"
 
@@ -45,13 +48,18 @@ namespace xkb {
 namespace sched {
 
 enum : int { kTaskGemm = 0, kTaskTrsm = 1 };
-// kFlagNarrow: an operand base or leading dimension is not 16-byte aligned,
-// so the gemm tile stages it with 8-byte L2 loads instead of 16-byte copies
-enum : int { kFlagSwap = 1, kFlagConj = 2, kFlagLower = 4, kFlagUnit = 8, kFlagNarrow = 16 };
+// kFlagNarrowA / B: that operand's base or leading dimension is not 16-byte
+// aligned, so the gemm tile stages it with 8-byte copies
+enum : int {
+  kFlagSwap = 1, kFlagConj = 2, kFlagLower = 4, kFlagUnit = 8, kFlagNarrowA = 16,
+  kFlagNarrowB = 32
+};
 
 // One task.  succ0 / nsucc: its successors in the batch's successor array
 // (tasks whose dependency count it decrements when it completes).
-//   gemm:  C = (ar,ai) op(A) op(B) + (br,bi) C, C is M x N, inner K.
+//   gemm:  C = (ar,ai) op(A) op(B) + (br,bi) C, C is M x N, inner K: a whole
+//          call, whose tiles are the bulk entries from tile0 on (tile index =
+//          entry - tile0, column by column); a CTA cuts its tile out of it.
 //   trsm:  C = X_i (M rows, N right-hand sides); A, B = the op(A) panel and
 //          the solved X rows it multiplies (K = their inner length, 0 for
 //          the first block); D = the diagonal block; (ar,ai) = alpha.
@@ -64,13 +72,13 @@ struct alignas(16) Task {
   const void* D;
   long lda, ldb, ldc;
   double ar, ai, br, bi;
-  int succ0, nsucc, flags, pad;
+  int succ0, nsucc, flags, tile0;
 };
 static_assert(sizeof(Task) == 144, "task record");
 
 // Device-side queues of one batch (ints in global memory):
-//   bulk[nbulk]   tasks without dependencies (gemm tiles of gemm calls), in
-//                 call order; claimed with an atomic head;
+//   bulk[nbulk]   the gemm calls' tiles (entry: the call's task), in call
+//                 order; claimed with an atomic head;
 //   urq[nurg]     the solve tasks: a ready queue.  The first block of every
 //                 chain is queued at launch; a task is appended (atomic
 //                 tail, then the slot is written) when its last dependency
@@ -83,10 +91,13 @@ struct Ctl {
   int head_bulk, head_urg, tail_urg, pad;
 };
 
-constexpr int kThreads = 256;
-constexpr int kBK = 16;
-constexpr int kSt = 3;      // cp.async stages
+template <class T>
+using TileCfg = Cfg<T, St<T>::CPLX ? 32 : 64, St<T>::CPLX ? 32 : 64, 2, 2, 3, 4>;
+constexpr int kMma = TileCfg<double>::THREADS;  // MMA threads
+constexpr int kThreads = kMma + 32;             // and the copy warp
+constexpr int kStages = 4;
 constexpr int kLeafS = kLeafRows;  // trsm block (trsm_leaf.cuh)
+static_assert(TileCfg<double2>::THREADS == kMma, "one CTA shape");
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem)),
@@ -98,12 +109,11 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int src_
                "r"(src_bytes)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// The barrier's pending count (32: one per lane) drops once this thread's
+// copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
 }
 
 __device__ __forceinline__ int ld_volatile(const int* p) { return *(const volatile int*)p; }
@@ -111,10 +121,12 @@ __device__ __forceinline__ int ld_volatile(const int* p) { return *(const volati
 // Claim the next task for this CTA (thread 0 only): from the ready queue of
 // the solves or from the bulk list, in the order `urgent_first` asks.  Spins
 // (bounded) while every remaining task still waits for a dependency.
-// Returns the task id, -1 when every task has been claimed, -2 on timeout or
-// when another CTA recorded an error.
+// Returns the task id (entry: its bulk index, -1 for a solve), -1 when every
+// task has been claimed, -2 on timeout or when another CTA recorded an error.
 __device__ __forceinline__ int claim_task(Ctl* ctl, const int* bulk, int nbulk, const int* urq,
-                                          int nurg, bool urgent_first, uint64_t wait_ns) {
+                                          int nurg, bool urgent_first, uint64_t wait_ns,
+                                          int& entry) {
+  entry = -1;
   uint64_t t0 = 0;
   for (uint32_t spin = 0;; ++spin) {
     for (int pass = 0; pass < 2; ++pass) {
@@ -142,7 +154,10 @@ __device__ __forceinline__ int claim_task(Ctl* ctl, const int* bulk, int nbulk, 
         }
       } else if (ld_volatile(&ctl->head_bulk) < nbulk) {
         const int b = atomicAdd(&ctl->head_bulk, 1);
-        if (b < nbulk) return bulk[b];
+        if (b < nbulk) {
+          entry = b;
+          return bulk[b];
+        }
       }
     }
     if (ld_volatile(&ctl->head_bulk) >= nbulk && ld_volatile(&ctl->head_urg) >= nurg) return -1;
@@ -160,380 +175,191 @@ __device__ __forceinline__ int claim_task(Ctl* ctl, const int* bulk, int nbulk, 
 }
 
 // ---- gemm tile ---------------------------------------------------------------
-// Shared layout of a stage: op(A) as BM x kBK, op(B) as kBK x BN, each in the
-// orientation of its global storage so that 16-byte copies run along the
-// contiguous dimension.  "KC" = k contiguous (row m of op(A) / column n of
-// op(B) holds kBK consecutive k).  Real tiles are padded: KC rows by 8
-// doubles (a lane's k-pair is one 16-byte load, conflict-free across the
-// eight lanes of a phase), the other orientation by 2 (the 16 lanes of a
-// phase hit 16 distinct 8-byte bank pairs).  Warp grid: real 64 x 64 tiles
-// 2 x 4 warps (32 x 16 each), real 128 x 64 tiles 4 x 2 (32 x 32), complex
-// 32 x 64 tiles 2 x 4 (16 x 16).
-template <class T, bool A_KC, bool B_KC, int BM>
-struct TileShape {
-  static constexpr bool CPLX = St<T>::CPLX;
-  static constexpr int BN = 64;
-  static constexpr int WM = BM == 128 ? 4 : 2, WN = kThreads / 32 / WM;
-  static constexpr int WTM = BM / WM, WTN = BN / WN;
-  static constexpr int MF = WTM / 16, NF = WTN / 8;
-  static constexpr int PKC = CPLX ? 0 : 8, PMN = CPLX ? 0 : 2;
-  static constexpr int LDA = A_KC ? kBK + PKC : BM + PMN;  // smem stride (elements)
-  static constexpr int LDB = B_KC ? kBK + PKC : BN + PMN;
-  static constexpr int A_S = A_KC ? BM * LDA : kBK * LDA;  // smem elements per stage
-  static constexpr int B_S = B_KC ? BN * LDB : kBK * LDB;
-  static constexpr int ES = (int)sizeof(T);
-  static constexpr int STAGE_BYTES = (A_S + B_S) * ES;
-};
-
-// Staging modes: kCopy16 16-byte cp.async.cg copies (aligned operands);
-// kCopy8 8-byte cp.async.ca copies (an operand not 16-byte aligned, operands
-// not written while the batch runs: L1 may keep them); kLoad8 8-byte L2 loads
-// through registers, one stage ahead (not 16-byte aligned, and B holds rows
-// other CTAs solved during this launch).
-enum : int { kCopy16 = 0, kCopy8 = 1, kLoad8 = 2 };
-
-// not inlined: each instantiation keeps its own register allocation
-template <class T, bool A_KC, bool B_KC, int BM, int MODE>
-__device__ __noinline__ void gemm_tile(const Task& t, uint8_t* smem) {
-  using Sh = TileShape<T, A_KC, B_KC, BM>;
-  using S = typename St<T>::S;
-  constexpr bool CPLX = Sh::CPLX;
-  constexpr int BN = Sh::BN, WTM = Sh::WTM, WTN = Sh::WTN, MF = Sh::MF, NF = Sh::NF;
-  constexpr int LDA = Sh::LDA, LDB = Sh::LDB, ES = Sh::ES;
-  constexpr int EPC = 16 / ES;  // elements per 16-byte chunk
-  constexpr int A_ELEMS = BM * kBK, B_ELEMS = BN * kBK;
-  constexpr int STAGE_BYTES = Sh::STAGE_BYTES;
-  constexpr int NACC = CPLX ? 8 : 4;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const char* Ag = static_cast<const char*>(t.A);
-  const char* Bg = static_cast<const char*>(t.B);
-  const int M = t.M, N = t.N, K = t.K;
-  const int KT = (K + kBK - 1) / kBK;
-  // shared offset (elements) of op(A)(m, k) / op(B)(k, n)
-  auto a_off = [](int m, int k) { return A_KC ? m * LDA + k : k * LDA + m; };
-  auto b_off = [](int k, int n) { return B_KC ? n * LDB + k : k * LDB + n; };
-
-  // cp.async paths: 16-byte chunks (kCopy16) or 8-byte words (kCopy8)
-  auto load_stage = [&](int it, int buf) {
-    uint8_t* sa = smem + buf * STAGE_BYTES;
-    uint8_t* sb = sa + Sh::A_S * ES;
-    const int k0 = it * kBK;
-    if constexpr (MODE == kCopy8) {
-      constexpr int W = ES / 8;  // words per element
-      for (int w = tid; w < A_ELEMS * W; w += kThreads) {
-        const int e = w / W, h = w % W;
-        const int mm = A_KC ? e / kBK : e % BM, kk = A_KC ? e % kBK : e / BM;
-        const int gk = k0 + kk;
-        const bool v = mm < M && gk < K;
-        const size_t gi =
-            A_KC ? (size_t)gk + (size_t)mm * t.lda : (size_t)mm + (size_t)gk * t.lda;
-        cp_async8(sa + a_off(mm, kk) * ES + h * 8, v ? Ag + gi * ES + h * 8 : Ag, v ? 8 : 0);
-      }
-      for (int w = tid; w < B_ELEMS * W; w += kThreads) {
-        const int e = w / W, h = w % W;
-        const int nn = B_KC ? e / kBK : e % BN, kk = B_KC ? e % kBK : e / BN;
-        const int gk = k0 + kk;
-        const bool v = nn < N && gk < K;
-        const size_t gi =
-            B_KC ? (size_t)gk + (size_t)nn * t.ldb : (size_t)nn + (size_t)gk * t.ldb;
-        cp_async8(sb + b_off(kk, nn) * ES + h * 8, v ? Bg + gi * ES + h * 8 : Bg, v ? 8 : 0);
+// One operand's ROWS lines of 128 bytes (OpTile's layout) for k [k0, k0 + BK):
+// g = its element (row 0, k 0) in op(A) / op(B)^T; rows past `rows` and k past
+// K are zero.  All lanes of the copy warp; consecutive lanes, consecutive
+// bytes.  16-byte copies (L2 only), or, narrow, 8-byte ones (through L1, which
+// the claim's fence left without lines that other CTAs wrote before it).
+template <class T, bool KC, int ROWS>
+__device__ __forceinline__ void copy_lines(uint8_t* dst, const char* g, long ld, int rows, int k0,
+                                           int K, bool narrow) {
+  constexpr int ES = (int)sizeof(T), BK = 128 / ES;
+  const int lane = threadIdx.x & 31;
+  const size_t ldb = (size_t)ld * ES;
+  if (!narrow) {
+    constexpr int EPC = 16 / ES;  // elements per chunk
+    const int c = lane & 7, l0 = lane >> 3;
+    if (rows >= ROWS && k0 + BK <= K) {
+      const char* src = KC ? g + (size_t)k0 * ES + c * 16 + l0 * ldb
+                           : g + c * 16 + (size_t)(k0 + l0) * ldb;
+#pragma unroll
+      for (int q = 0; q < ROWS / 4; ++q) {
+        const int L = l0 + 4 * q;
+        // KC: line = row; else panel L / BK, k = L % BK
+        const char* x = KC ? src + (size_t)(4 * q) * ldb
+                           : src + (4 * q / BK) * 128 + (size_t)(4 * q % BK) * ldb;
+        cp_async16(dst + L * 128 + ((c ^ (L & 7)) << 4), x, 16);
       }
       return;
     }
-    constexpr int A_CH = A_ELEMS / EPC;
-    for (int c = tid; c < A_CH; c += kThreads) {
-      int mm, kk;  // first element of the chunk
-      if (A_KC) {
-        mm = c / (kBK / EPC);
-        kk = (c % (kBK / EPC)) * EPC;
-      } else {
-        kk = c / (BM / EPC);
-        mm = (c % (BM / EPC)) * EPC;
-      }
-      const int gk = k0 + kk;
+#pragma unroll 4
+    for (int q = 0; q < ROWS / 4; ++q) {
+      const int L = l0 + 4 * q;
       int valid;
-      const char* src;
-      if (A_KC) {  // element (m,k) at A[k + m*lda]; chunk runs along k
-        valid = (mm < M) ? max(0, min(EPC, K - gk)) : 0;
-        src = Ag + ((size_t)gk + (size_t)mm * t.lda) * ES;
-      } else {     // element (m,k) at A[m + k*lda]; chunk runs along m
-        valid = (gk < K) ? max(0, min(EPC, M - mm)) : 0;
-        src = Ag + ((size_t)mm + (size_t)gk * t.lda) * ES;
-      }
-      cp_async16(sa + a_off(mm, kk) * ES, valid ? src : Ag, valid * ES);
-    }
-    constexpr int B_CH = B_ELEMS / EPC;
-    for (int c = tid; c < B_CH; c += kThreads) {
-      int nn, kk;
-      if (B_KC) {
-        nn = c / (kBK / EPC);
-        kk = (c % (kBK / EPC)) * EPC;
+      const char* x;
+      if (KC) {
+        valid = L < rows ? max(0, min(EPC, K - k0 - c * EPC)) : 0;
+        x = g + (size_t)k0 * ES + c * 16 + (size_t)L * ldb;
       } else {
-        kk = c / (BN / EPC);
-        nn = (c % (BN / EPC)) * EPC;
+        const int kk = k0 + L % BK, m = L / BK * BK + c * EPC;
+        valid = kk < K ? max(0, min(EPC, rows - m)) : 0;
+        x = g + (size_t)(L / BK) * 128 + c * 16 + (size_t)kk * ldb;
       }
-      const int gk = k0 + kk;
-      int valid;
-      const char* src;
-      if (B_KC) {  // element (k,n) at B[k + n*ldb]
-        valid = (nn < N) ? max(0, min(EPC, K - gk)) : 0;
-        src = Bg + ((size_t)gk + (size_t)nn * t.ldb) * ES;
-      } else {     // element (k,n) at B[n + k*ldb]
-        valid = (gk < K) ? max(0, min(EPC, N - nn)) : 0;
-        src = Bg + ((size_t)nn + (size_t)gk * t.ldb) * ES;
-      }
-      cp_async16(sb + b_off(kk, nn) * ES, valid ? src : Bg, valid * ES);
+      cp_async16(dst + L * 128 + ((c ^ (L & 7)) << 4), valid ? x : g, valid * ES);
     }
-  };
-
-  // 8-byte register-staged path (an operand not 16-byte aligned): word w of
-  // a stage is 8-byte word w % WPE of element w / WPE
-  constexpr int WPE = ES / 8;
-  constexpr int NWA = A_ELEMS * WPE / kThreads, NWB = B_ELEMS * WPE / kThreads;
-  static_assert(NWA * kThreads == A_ELEMS * WPE && NWB * kThreads == B_ELEMS * WPE, "stage split");
-  double ra[MODE == kLoad8 ? NWA : 1], rb[MODE == kLoad8 ? NWB : 1];
-  auto a_elem = [](int e, int& mm, int& kk) {
-    if (A_KC) { mm = e / kBK; kk = e % kBK; } else { kk = e / BM; mm = e % BM; }
-  };
-  auto b_elem = [](int e, int& nn, int& kk) {
-    if (B_KC) { nn = e / kBK; kk = e % kBK; } else { kk = e / BN; nn = e % BN; }
-  };
-  auto fetch = [&](int it) {
-    const int k0 = it * kBK;
-    const double* Ad = reinterpret_cast<const double*>(Ag);
-    const double* Bd = reinterpret_cast<const double*>(Bg);
-#pragma unroll
-    for (int q = 0; q < NWA; ++q) {
-      const int w = tid + q * kThreads, e = w / WPE, h = w % WPE;
-      int mm, kk;
-      a_elem(e, mm, kk);
-      const int gk = k0 + kk;
-      const size_t gi = A_KC ? (size_t)gk + (size_t)mm * t.lda : (size_t)mm + (size_t)gk * t.lda;
-      ra[q] = (mm < M && gk < K) ? __ldcg(Ad + gi * WPE + h) : 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < NWB; ++q) {
-      const int w = tid + q * kThreads, e = w / WPE, h = w % WPE;
-      int nn, kk;
-      b_elem(e, nn, kk);
-      const int gk = k0 + kk;
-      const size_t gi = B_KC ? (size_t)gk + (size_t)nn * t.ldb : (size_t)nn + (size_t)gk * t.ldb;
-      rb[q] = (nn < N && gk < K) ? __ldcg(Bd + gi * WPE + h) : 0.0;
-    }
-  };
-  auto put = [&](int buf) {
-    double* sa = reinterpret_cast<double*>(smem + buf * STAGE_BYTES);
-    double* sb = sa + Sh::A_S * WPE;
-#pragma unroll
-    for (int q = 0; q < NWA; ++q) {
-      const int w = tid + q * kThreads, e = w / WPE, h = w % WPE;
-      int mm, kk;
-      a_elem(e, mm, kk);
-      sa[a_off(mm, kk) * WPE + h] = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < NWB; ++q) {
-      const int w = tid + q * kThreads, e = w / WPE, h = w % WPE;
-      int nn, kk;
-      b_elem(e, nn, kk);
-      sb[b_off(kk, nn) * WPE + h] = rb[q];
-    }
-  };
-
-  const int wm = warp / Sh::WN, wn = warp % Sh::WN;
-  const int g = lane >> 2, tq = lane & 3;
-  double acc[MF][NF][NACC];
-#pragma unroll
-  for (int i = 0; i < MF; ++i)
-#pragma unroll
-    for (int j = 0; j < NF; ++j)
-#pragma unroll
-      for (int v = 0; v < NACC; ++v) acc[i][j][v] = 0.0;
-  const double sgnA = (t.opA == XKB_OP_C) ? -1.0 : 1.0;
-  const double sgnB = (t.opB == XKB_OP_C) ? -1.0 : 1.0;
-
-  auto compute = [&](int buf) {
-    const uint8_t* sbase = smem + buf * STAGE_BYTES;
-    const S* sa = reinterpret_cast<const S*>(sbase);
-    const S* sb = reinterpret_cast<const S*>(sbase + Sh::A_S * ES);
-#pragma unroll
-    for (int kc = 0; kc < kBK / 8; ++kc) {
-      // logical k = tq and tq + 4 of the MMA are physical k0 = 2 tq, k1 = k0 + 1
-      const int k0 = kc * 8 + 2 * tq, k1 = k0 + 1;
-      double br[NF][2], bi[NF][2];
-#pragma unroll
-      for (int nf = 0; nf < NF; ++nf) {
-        const int n = wn * WTN + nf * 8 + g;
-        if constexpr (B_KC && !CPLX) {
-          const double2 v = *reinterpret_cast<const double2*>(sb + b_off(k0, n));
-          br[nf][0] = v.x;
-          br[nf][1] = v.y;
-        } else {
-          ld_elem<T>(sb, b_off(k0, n), br[nf][0], bi[nf][0]);
-          ld_elem<T>(sb, b_off(k1, n), br[nf][1], bi[nf][1]);
-          if (CPLX) {
-            bi[nf][0] *= sgnB;
-            bi[nf][1] *= sgnB;
-          }
-        }
-      }
-#pragma unroll
-      for (int mf = 0; mf < MF; ++mf) {
-        const int r0 = wm * WTM + mf * 16 + g, r1 = r0 + 8;
-        double ar[4], ai[4];
-        if constexpr (A_KC && !CPLX) {
-          const double2 v0 = *reinterpret_cast<const double2*>(sa + a_off(r0, k0));
-          const double2 v1 = *reinterpret_cast<const double2*>(sa + a_off(r1, k0));
-          ar[0] = v0.x;
-          ar[1] = v1.x;
-          ar[2] = v0.y;
-          ar[3] = v1.y;
-        } else {
-          ld_elem<T>(sa, a_off(r0, k0), ar[0], ai[0]);
-          ld_elem<T>(sa, a_off(r1, k0), ar[1], ai[1]);
-          ld_elem<T>(sa, a_off(r0, k1), ar[2], ai[2]);
-          ld_elem<T>(sa, a_off(r1, k1), ar[3], ai[3]);
-        }
-        if constexpr (CPLX) {
-          double nai[4];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            ai[v] *= sgnA;
-            nai[v] = -ai[v];
-          }
-#pragma unroll
-          for (int nf = 0; nf < NF; ++nf) {
-            double* a = acc[mf][nf];
-            double (&re)[4] = *reinterpret_cast<double(*)[4]>(a);
-            double (&im)[4] = *reinterpret_cast<double(*)[4]>(a + 4);
-            dmma_k8(re, ar, br[nf]);
-            dmma_k8(re, nai, bi[nf]);
-            dmma_k8(im, ar, bi[nf]);
-            dmma_k8(im, ai, br[nf]);
-          }
-        } else {
-#pragma unroll
-          for (int nf = 0; nf < NF; ++nf) {
-            double (&d)[4] = *reinterpret_cast<double(*)[4]>(acc[mf][nf]);
-            dmma_k8(d, ar, br[nf]);
-          }
-        }
-      }
-    }
-  };
-
-  if constexpr (MODE != kLoad8) {
-    for (int s = 0; s < kSt - 1; ++s) {
-      if (s < KT) load_stage(s, s);
-      cp_async_commit();
-    }
-    for (int it = 0; it < KT; ++it) {
-      cp_async_wait<kSt - 2>();
-      __syncthreads();  // stage `it` landed for everyone; stage it-1 no longer read
-      if (it + kSt - 1 < KT) load_stage(it + kSt - 1, (it + kSt - 1) % kSt);
-      cp_async_commit();
-      compute(it % kSt);
-    }
-    cp_async_wait<0>();
-  } else {
-    // registers carry stage it+1 while stage it is computed (two buffers)
-    if (KT > 0) {
-      fetch(0);
-      put(0);
-      if (KT > 1) fetch(1);
-    }
-    for (int it = 0; it < KT; ++it) {
-      __syncthreads();  // buffer it%2 written; buffer (it+1)%2 no longer read
-      if (it + 1 < KT) put((it + 1) & 1);
-      if (it + 2 < KT) fetch(it + 2);
-      compute(it & 1);
-    }
+    return;
   }
-  __syncthreads();  // smem free for the next task
-  S* C = reinterpret_cast<S*>(t.C);
-  const bool use_beta = (t.br != 0.0) || (t.bi != 0.0);
-  // one row of fragments at a time: all of its C loads, then its stores (C
-  // is read and written through one pointer; a load after a store would
-  // wait for it)
-#pragma unroll
-  for (int mf = 0; mf < MF; ++mf) {
-    double cv[NF][CPLX ? 8 : 4];
-#pragma unroll
-    for (int nf = 0; nf < NF; ++nf)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = wm * WTM + mf * 16 + g + ((i >> 1) << 3);
-        const int col = wn * WTN + nf * 8 + 2 * tq + (i & 1);
-        cv[nf][i] = 0.0;
-        if (CPLX) cv[nf][CPLX ? 4 + i : i] = 0.0;
-        if (!use_beta || row >= M || col >= N) continue;
-        const size_t idx = (size_t)row + (size_t)col * (size_t)t.ldc;
-        if constexpr (CPLX) {
-          cv[nf][i] = __ldcg(C + 2 * idx);
-          cv[nf][4 + i] = __ldcg(C + 2 * idx + 1);
-        } else {
-          cv[nf][i] = __ldcg(C + idx);
-        }
-      }
-#pragma unroll
-    for (int nf = 0; nf < NF; ++nf)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = wm * WTM + mf * 16 + g + ((i >> 1) << 3);
-        const int col = wn * WTN + nf * 8 + 2 * tq + (i & 1);
-        if (row >= M || col >= N) continue;
-        const size_t idx = (size_t)row + (size_t)col * (size_t)t.ldc;
-        if constexpr (CPLX) {
-          const double xr = acc[mf][nf][i], xi = acc[mf][nf][4 + i];
-          const double cr = cv[nf][i], ci = cv[nf][CPLX ? 4 + i : i];
-          C[2 * idx] = t.ar * xr - t.ai * xi + (t.br * cr - t.bi * ci);
-          C[2 * idx + 1] = t.ar * xi + t.ai * xr + (t.br * ci + t.bi * cr);
-        } else {
-          C[idx] = fma(t.br, cv[nf][i], t.ar * acc[mf][nf][i]);
-        }
-      }
+  // 8-byte words: 16 per line
+  const int w = lane & 15, l0 = lane >> 4;
+  auto at = [&](int L, const char*& x) {
+    if (KC) {
+      x = g + (size_t)k0 * ES + w * 8 + (size_t)L * ldb;
+      return L < rows && k0 + w * 8 / ES < K;
+    }
+    const int kk = k0 + L % BK, m = L / BK * BK + w * 8 / ES;
+    x = g + (size_t)(L / BK) * 128 + w * 8 + (size_t)kk * ldb;
+    return kk < K && m < rows;
+  };
+  auto to = [&](int L) { return dst + L * 128 + (((w >> 1) ^ (L & 7)) << 4) + (w & 1) * 8; };
+#pragma unroll 8
+  for (int q = 0; q < ROWS / 2; ++q) {
+    const int L = l0 + 2 * q;
+    const char* x;
+    const bool v = at(L, x);
+    cp_async8(to(L), v ? x : g, v ? 8 : 0);
   }
 }
 
-template <class T, int BM, int MODE>
-__device__ __forceinline__ void gemm_dispatch2(const Task& t, uint8_t* smem) {
+// The copy warp's part of a tile: stages [pos, pos + KT) of the ring.  False
+// if a bounded wait gave up.
+template <class T, bool A_KC, bool B_KC>
+__device__ __noinline__ bool copy_tile(const Task& t, uint8_t* ring, uint64_t* full,
+                                       uint64_t* empty, int pos, bool narrowA, bool narrowB) {
+  using C_ = TileCfg<T>;
+  const int KT = (t.K + C_::BK - 1) / C_::BK;
+  for (int j = pos; j < pos + KT; ++j) {
+    const int s = j % kStages;
+    if (j >= kStages) {
+      const bool free_ = mbar_wait(&empty[s], (j / kStages - 1) & 1, kErrEmptyWait);
+      if (!__all_sync(0xffffffffu, free_)) return false;
+    }
+    uint8_t* sa = ring + s * C_::STAGE_BYTES;
+    const int k0 = (j - pos) * C_::BK;
+    copy_lines<T, A_KC, C_::BM>(sa, static_cast<const char*>(t.A), t.lda, t.M, k0, t.K, narrowA);
+    copy_lines<T, B_KC, C_::BN>(sa + C_::A_BYTES, static_cast<const char*>(t.B), t.ldb, t.N, k0,
+                                t.K, narrowB);
+    cp_async_arrive(&full[s]);
+  }
+  return true;
+}
+
+// The MMA warps' part: accumulate the stages, then alpha / beta and the store.
+// Not inlined: each instantiation keeps its own register allocation.
+template <class T, bool A_KC, bool B_KC>
+__device__ __noinline__ bool mma_tile(const Task& t, uint8_t* ring, uint64_t* full,
+                                      uint64_t* empty, int pos) {
+  using C_ = TileCfg<T>;
+  const int KT = (t.K + C_::BK - 1) / C_::BK;
+  const int warp = threadIdx.x >> 5;
+  double acc[C_::MF][C_::NF][C_::NACC];
+#pragma unroll
+  for (int i = 0; i < C_::MF; ++i)
+#pragma unroll
+    for (int j = 0; j < C_::NF; ++j)
+#pragma unroll
+      for (int v = 0; v < C_::NACC; ++v) acc[i][j][v] = 0.0;
+  const unsigned fA = t.opA == XKB_OP_C ? 0x80000000u : 0u,
+                 fB = t.opB == XKB_OP_C ? 0x80000000u : 0u;
+  if (!dmma_mainloop<C_, A_KC, B_KC>(ring, full, empty, pos, KT, acc, (warp / C_::WN) * C_::WTM,
+                                     (warp % C_::WN) * C_::WTN, fA, fB))
+    return false;
+  GemmParams p;
+  p.M = t.M;
+  p.N = t.N;
+  p.C = t.C;
+  p.ldc = t.ldc;
+  p.ar = t.ar;
+  p.ai = t.ai;
+  p.br = t.br;
+  p.bi = t.bi;
+  p.uplo = XKB_FULL;
+  p.herm_diag = 0;
+  p.diag = 0;
+  p.vec = reinterpret_cast<uintptr_t>(t.C) % 16 == 0 && ((size_t)t.ldc * sizeof(T)) % 16 == 0;
+  dmma_epilogue<C_, A_KC, B_KC>(p, 0, 0, &acc[0][0][0]);
+  return true;
+}
+
+// One tile by the whole CTA.  Returns the ring positions used.
+template <class T>
+__device__ __forceinline__ int run_tile(const Task& t, uint8_t* ring, uint64_t* full,
+                                        uint64_t* empty, int pos, int* fail) {
   const bool akc = t.opA != XKB_OP_N, bkc = t.opB == XKB_OP_N;
-  if (akc && bkc) gemm_tile<T, true, true, BM, MODE>(t, smem);
-  else if (akc) gemm_tile<T, true, false, BM, MODE>(t, smem);
-  else if (bkc) gemm_tile<T, false, true, BM, MODE>(t, smem);
-  else gemm_tile<T, false, false, BM, MODE>(t, smem);
+  bool ok;
+  if (threadIdx.x >= kMma) {
+    const bool ma = t.flags & kFlagNarrowA, mb = t.flags & kFlagNarrowB;
+    if (akc && bkc) ok = copy_tile<T, true, true>(t, ring, full, empty, pos, ma, mb);
+    else if (akc) ok = copy_tile<T, true, false>(t, ring, full, empty, pos, ma, mb);
+    else if (bkc) ok = copy_tile<T, false, true>(t, ring, full, empty, pos, ma, mb);
+    else ok = copy_tile<T, false, false>(t, ring, full, empty, pos, ma, mb);
+  } else {
+    if (akc && bkc) ok = mma_tile<T, true, true>(t, ring, full, empty, pos);
+    else if (akc) ok = mma_tile<T, true, false>(t, ring, full, empty, pos);
+    else if (bkc) ok = mma_tile<T, false, true>(t, ring, full, empty, pos);
+    else ok = mma_tile<T, false, false>(t, ring, full, empty, pos);
+  }
+  if (!ok) *reinterpret_cast<volatile int*>(fail) = 1;
+  return (t.K + TileCfg<T>::BK - 1) / TileCfg<T>::BK;
+}
+
+// Rows [r0, ..) x columns [c0, ..) of a product, at most BM x BN of them.
+template <class T>
+__device__ __forceinline__ void cut_tile(Task& t, int r0, int c0) {
+  using C_ = TileCfg<T>;
+  constexpr size_t ES = sizeof(T);
+  t.A = static_cast<const char*>(t.A) + (size_t)r0 * (t.opA == XKB_OP_N ? 1 : t.lda) * ES;
+  t.B = static_cast<const char*>(t.B) + (size_t)c0 * (t.opB == XKB_OP_N ? t.ldb : 1) * ES;
+  t.C = static_cast<char*>(t.C) + ((size_t)r0 + (size_t)c0 * t.ldc) * ES;
+  t.M = min(C_::BM, t.M - r0);
+  t.N = min(C_::BN, t.N - c0);
 }
 
 // ---- trsm diagonal block ------------------------------------------------------
-// One 64-row diagonal block against up to 64 right-hand sides: the shared
-// register-resident substitution of trsm_leaf.cuh.  Not inlined: its
-// register allocation stays apart from the gemm tile's.
-constexpr size_t kTrsmSmem = LeafShape<double2>::SMEM;  // complex, the larger
-
+// One 64-row diagonal block against up to 64 right-hand sides
+// (trsm_leaf.cuh).  Not inlined: its register allocation stays apart from the
+// gemm tile's.
 template <class T>
 __device__ __noinline__ void trsm_tile(const Task& t, uint8_t* smem, double ar, double ai) {
   using S = typename St<T>::S;
   double* sm = reinterpret_cast<double*>(smem);
   const bool swap = t.flags & kFlagSwap, conj = t.flags & kFlagConj;
   const bool lower = t.flags & kFlagLower, unit = t.flags & kFlagUnit;
-  leaf_stage<T, kThreads>(static_cast<const S*>(t.D), t.lda, t.M, swap, conj, lower, unit, sm);
+  const S* D = static_cast<const S*>(t.D);
   S* X = static_cast<S*>(t.C);
-  if (lower) leaf_solve<T, kThreads, true>(X, t.ldc, false, t.M, 0, t.N, ar, ai, sm);
-  else leaf_solve<T, kThreads, false>(X, t.ldc, false, t.M, 0, t.N, ar, ai, sm);
-  __syncthreads();
+  if (lower) leaf_solve<T, true>(D, t.lda, t.M, swap, conj, unit, X, t.ldc, t.N, ar, ai, sm);
+  else leaf_solve<T, false>(D, t.lda, t.M, swap, conj, unit, X, t.ldc, t.N, ar, ai, sm);
 }
 
-// dynamic shared memory: the largest task body (the complex solve's staging,
-// 81 KB; gemm stages: real 128 x 64 3 x 26 KB, complex 3 x 24 KB) + alignment
-constexpr size_t kSmemMax(size_t a, size_t b) { return a > b ? a : b; }
-constexpr size_t kSmemBytes =
-    kSmemMax(kTrsmSmem,
-             kSmemMax((size_t)kSt * TileShape<double, true, true, 128>::STAGE_BYTES,
-                      kSmemMax((size_t)kSt * TileShape<double, false, false, 128>::STAGE_BYTES,
-                               (size_t)kSt * TileShape<double2, false, false, 32>::STAGE_BYTES))) +
-    128;
+// dynamic shared memory: the ring, or the solve's staging in its place; a
+// batch with a complex solve needs more and runs two CTAs per SM
+constexpr size_t kRingBytes = kStages * (size_t)TileCfg<double>::STAGE_BYTES;
+static_assert(TileCfg<double2>::STAGE_BYTES <= TileCfg<double>::STAGE_BYTES, "one ring");
+constexpr size_t sched_smem(bool ztrsm) {
+  const size_t s = ztrsm ? LeafShape<double2>::SMEM : LeafShape<double>::SMEM;
+  return (s > kRingBytes ? s : kRingBytes) + 128;
+}
 
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 3)
     k_sched(const Task* __restrict__ tasks, int* ndep, const int* __restrict__ succ,
             const int* __restrict__ bulk, int nbulk, int* urq, int nurg, Ctl* ctl,
             int urgent_first, int* call_left, unsigned long long* call_end,
@@ -541,98 +367,93 @@ __global__ void __launch_bounds__(kThreads, 2)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem =
       reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  __shared__ int s_idx;
-  __shared__ Task s_task;  // the claimed task, read by every thread from here
+  __shared__ int s_idx, s_fail;
+  __shared__ Task s_task;  // the claimed task (a gemm call: its tile), read by every thread
   __shared__ Task s_sub;   // a gemm step of a solve task
-  if (threadIdx.x == 0) atomicMin(t_start, (unsigned long long)globaltimer());
+  __shared__ uint64_t s_full[kStages], s_empty[kStages];
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < kStages; ++q) {
+      mbar_init(&s_full[q], 32);
+      mbar_init(&s_empty[q], kMma / 32);
+    }
+    fence_barrier_init();
+    s_fail = 0;
+    atomicMin(t_start, (unsigned long long)globaltimer());
+  }
+  int pos = 0;  // ring position, the same in every thread
   for (;;) {
     if (threadIdx.x == 0) {
-      const int i = claim_task(ctl, bulk, nbulk, urq, nurg, urgent_first != 0, wait_ns);
+      int entry;
+      const int i =
+          claim_task(ctl, bulk, nbulk, urq, nurg, urgent_first != 0, wait_ns, entry);
       if (i >= 0) {
         __threadfence();  // acquire: the producers' outputs before the reads
-        s_task = tasks[i];
+        Task t = tasks[i];
+        if (t.kind == kTaskGemm) {
+          const int b = t.dtype == XKB_Z ? TileCfg<double2>::BM : TileCfg<double>::BM;
+          const int tm = (t.M + b - 1) / b, tile = entry - t.tile0;
+          if (t.dtype == XKB_Z) cut_tile<double2>(t, tile % tm * b, tile / tm * b);
+          else cut_tile<double>(t, tile % tm * b, tile / tm * b);
+        }
+        s_task = t;
       }
       s_idx = i;
     }
     __syncthreads();
-    if (s_idx < 0) break;
+    if (s_idx < 0 || *reinterpret_cast<volatile int*>(&s_fail)) break;
     // only thread 0 rewrites s_task, after every thread is past the barrier
     // that ends this task
     const Task& t = s_task;
     if (t.kind == kTaskGemm) {  // a gemm call's tile: operands read-only here
-      const bool nar = t.flags & kFlagNarrow;
-      if (t.dtype == XKB_Z) {
-        if (nar) gemm_dispatch2<double2, 32, kCopy8>(t, smem);
-        else gemm_dispatch2<double2, 32, kCopy16>(t, smem);
-      } else if (t.M > 64) {
-        if (nar) gemm_dispatch2<double, 128, kCopy8>(t, smem);
-        else gemm_dispatch2<double, 128, kCopy16>(t, smem);
-      } else {
-        if (nar) gemm_dispatch2<double, 64, kCopy8>(t, smem);
-        else gemm_dispatch2<double, 64, kCopy16>(t, smem);
-      }
+      if (t.dtype == XKB_Z) pos += run_tile<double2>(t, smem, s_full, s_empty, pos, &s_fail);
+      else pos += run_tile<double>(t, smem, s_full, s_empty, pos, &s_fail);
     } else {
-      // X_i = alpha B_i - op(A)[i, solved] X_solved in gemm tiles of BM rows,
-      // then the diagonal solve of X_i (same CTA: the tiles' stores are
-      // ordered before its loads by the barrier, both go through L2)
+      // X_i = alpha B_i - op(A)[i, solved] X_solved in gemm tiles, then the
+      // diagonal solve of X_i (same CTA: the tiles' stores are ordered before
+      // its loads by the barrier, both go through L2)
       const bool cplx = t.dtype == XKB_Z;
       double sar = t.ar, sai = t.ai;
       if (t.K > 0) {
-        const int bm = cplx ? 32 : 64;
-        const int es = cplx ? 16 : 8;
-        for (int r0 = 0; r0 < t.M; r0 += bm) {
-          if (threadIdx.x == 0) {
-            s_sub = t;
-            s_sub.M = min(bm, t.M - r0);
-            s_sub.A = static_cast<const char*>(t.A) +
-                      (size_t)r0 * (t.opA == XKB_OP_N ? 1 : t.lda) * es;
-            s_sub.C = static_cast<char*>(t.C) + (size_t)r0 * es;
-            s_sub.ar = -1.0;
-            s_sub.ai = 0.0;
-            s_sub.br = t.ar;
-            s_sub.bi = t.ai;
-          }
-          __syncthreads();
-          // op(B) = X rows solved by other CTAs of this launch: L2 only
-          const bool nar = t.flags & kFlagNarrow;
-          if (!cplx) {
-            if (t.opA == XKB_OP_N) {
-              if (nar) gemm_tile<double, false, true, 64, kLoad8>(s_sub, smem);
-              else gemm_tile<double, false, true, 64, kCopy16>(s_sub, smem);
-            } else {
-              if (nar) gemm_tile<double, true, true, 64, kLoad8>(s_sub, smem);
-              else gemm_tile<double, true, true, 64, kCopy16>(s_sub, smem);
+        const int b = cplx ? TileCfg<double2>::BM : TileCfg<double>::BM;
+        for (int c0 = 0; c0 < t.N; c0 += b)
+          for (int r0 = 0; r0 < t.M; r0 += b) {
+            if (threadIdx.x == 0) {
+              s_sub = t;
+              if (cplx) cut_tile<double2>(s_sub, r0, c0);
+              else cut_tile<double>(s_sub, r0, c0);
+              s_sub.ar = -1.0;
+              s_sub.ai = 0.0;
+              s_sub.br = t.ar;
+              s_sub.bi = t.ai;
             }
-          } else {
-            if (t.opA == XKB_OP_N) {
-              if (nar) gemm_tile<double2, false, true, 32, kLoad8>(s_sub, smem);
-              else gemm_tile<double2, false, true, 32, kCopy16>(s_sub, smem);
-            } else {
-              if (nar) gemm_tile<double2, true, true, 32, kLoad8>(s_sub, smem);
-              else gemm_tile<double2, true, true, 32, kCopy16>(s_sub, smem);
-            }
+            __syncthreads();
+            if (cplx) pos += run_tile<double2>(s_sub, smem, s_full, s_empty, pos, &s_fail);
+            else pos += run_tile<double>(s_sub, smem, s_full, s_empty, pos, &s_fail);
+            __syncthreads();  // s_sub is rewritten by the next part
           }
-          __syncthreads();  // s_sub is rewritten by the next row part
-        }
         sar = 1.0;
         sai = 0.0;
       }
-      if (!cplx) trsm_tile<double>(t, smem, sar, sai);
-      else trsm_tile<double2>(t, smem, sar, sai);
+      if (threadIdx.x < kMma) {
+        if (!cplx) trsm_tile<double>(t, smem, sar, sai);
+        else trsm_tile<double2>(t, smem, sar, sai);
+      }
     }
     __syncthreads();  // every output of the task is stored
+    if (*reinterpret_cast<volatile int*>(&s_fail)) break;  // a bounded wait gave up
     if (threadIdx.x == 0) {
       __threadfence();  // release the outputs before any successor is queued
       for (int k = 0; k < t.nsucc; ++k) {
         const int sidx = succ[t.succ0 + k];
         if (atomicSub(ndep + sidx, 1) == 1) {
-          const int pos = atomicAdd(&ctl->tail_urg, 1);
-          atomicExch(urq + pos, sidx);
+          const int q = atomicAdd(&ctl->tail_urg, 1);
+          atomicExch(urq + q, sidx);
         }
       }
       if (atomicSub(call_left + t.call, 1) == 1) call_end[t.call] = globaltimer();
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // copies in flight after an error
 }
 
 // ---------------------------------------------------------------------------
@@ -659,8 +480,6 @@ static bool aligned_ok(const void* p, long ld, int es) {
 }
 
 static bool ptr8(const void* p) { return reinterpret_cast<uintptr_t>(p) % 8 == 0; }
-
-static int tile128_rows() { return (int)tune("batch_tile128_min_rows", 96.0); }
 
 static Task gemm_task(int dtype, int opA, int opB, int M, int N, int K, int call, const void* A,
                       long lda, const void* B, long ldb, void* C, long ldc, double ar, double ai,
@@ -689,34 +508,25 @@ static Task gemm_task(int dtype, int opA, int opB, int M, int N, int K, int call
   return t;
 }
 
-// A gemm call: independent C tiles (the reference's tile loop,
-// blas/zgemm.c:279-367, with the whole K range in one task).
+// C tiles of a gemm call.
+static size_t gemm_tiles(const xkb_batch_op& o) {
+  const size_t b = o.dtype == XKB_Z ? TileCfg<double2>::BM : TileCfg<double>::BM;
+  return ((size_t)o.M + b - 1) / b * (((size_t)o.N + b - 1) / b);
+}
+
+// A gemm call: one task record, and a bulk entry per C tile (the reference's
+// tile loop, blas/zgemm.c:279-367, with the whole K range in one tile).
 static int add_gemm(Built& b, const xkb_batch_op& o, int call) {
   const int es = esz(o.dtype);
-  // real calls of at least batch_tile128_min_rows rows (tuning table,
-  // default 96) use 128-row tiles (the kernel picks the 128 x 64 body for
-  // any real task taller than 64 rows)
-  const int BM = o.dtype == XKB_Z ? 32 : (o.M >= tile128_rows() ? 128 : 64), BN = 64;
   if (!ptr8(o.A) || !ptr8(o.B) || !ptr8(o.C)) return XKB_EINVAL;
-  const int narrow =
-      (aligned_ok(o.A, o.lda, es) && aligned_ok(o.B, o.ldb, es)) ? 0 : kFlagNarrow;
-  const char* A = static_cast<const char*>(o.A);
-  const char* B = static_cast<const char*>(o.B);
-  char* C = static_cast<char*>(o.C);
-  int n = 0;
-  for (int n0 = 0; n0 < o.N; n0 += BN)
-    for (int m0 = 0; m0 < o.M; m0 += BM) {
-      const char* Ap = o.opA == XKB_OP_N ? A + (size_t)m0 * es : A + (size_t)m0 * o.lda * es;
-      const char* Bp = o.opB == XKB_OP_N ? B + (size_t)n0 * o.ldb * es : B + (size_t)n0 * es;
-      char* Cp = C + ((size_t)m0 + (size_t)n0 * o.ldc) * es;
-      b.bulk.push_back(b.add(gemm_task(o.dtype, o.opA, o.opB, std::min(BM, o.M - m0),
-                                       std::min(BN, o.N - n0), o.K, call, Ap, o.lda, Bp, o.ldb,
-                                       Cp, o.ldc, o.alpha[0], o.alpha[1], o.beta[0],
-                                       o.beta[1], narrow),
-                             0));
-      ++n;
-    }
-  return n;
+  const int flags = (aligned_ok(o.A, o.lda, es) ? 0 : kFlagNarrowA) |
+                    (aligned_ok(o.B, o.ldb, es) ? 0 : kFlagNarrowB);
+  const size_t n = gemm_tiles(o);
+  Task t = gemm_task(o.dtype, o.opA, o.opB, o.M, o.N, o.K, call, o.A, o.lda, o.B, o.ldb, o.C,
+                     o.ldc, o.alpha[0], o.alpha[1], o.beta[0], o.beta[1], flags);
+  t.tile0 = (int)b.bulk.size();
+  b.bulk.insert(b.bulk.end(), n, b.add(t, 0));
+  return (int)n;
 }
 
 // Left triangular solve: the reference's block algorithm (blas/ztrsm.c:
@@ -732,8 +542,8 @@ static int add_trsm(Built& b, const xkb_batch_op& o, int call) {
   const int es = esz(o.dtype);
   if (o.side != 0) return XKB_EINVAL;  // right side: not a batch task
   if (!ptr8(o.A) || !ptr8(o.C)) return XKB_EINVAL;
-  const int narrow =
-      (aligned_ok(o.A, o.lda, es) && aligned_ok(o.C, o.ldc, es)) ? 0 : kFlagNarrow;
+  const int narrow = (aligned_ok(o.A, o.lda, es) ? 0 : kFlagNarrowA) |
+                     (aligned_ok(o.C, o.ldc, es) ? 0 : kFlagNarrowB);
   const bool cplx = o.dtype == XKB_Z;
   const int trans = (!cplx && o.trans == XKB_OP_C) ? XKB_OP_T : o.trans;
   const bool fwd = (o.uplo == XKB_LOWER) ^ (trans != XKB_OP_N);
@@ -792,6 +602,7 @@ static int add_trsm(Built& b, const xkb_batch_op& o, int call) {
 // call_left and ctl are consumed by it.
 struct Layout {
   int ntasks = 0, nops = 0;
+  bool ztrsm = false;  // holds a complex solve (larger shared memory)
   size_t nbulk = 0, nurg = 0, nsucc = 0;
   size_t o_ndep = 0, o_succ = 0, o_bulk = 0, o_urq = 0, o_left = 0, o_ctl = 0, bytes = 0;
   void set(int nt, size_t ns, size_t nb, size_t nu, int no) {
@@ -947,18 +758,19 @@ static Batch& batch() {
 }
 static std::mutex g_batch_mu;
 
-static int grid_size() {
+// CTAs of a launch: as many as fit, at most one per tile and solve task.
+static int grid_size(const Layout& L) {
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sched, kThreads, kSmemBytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sched, kThreads, sched_smem(L.ztrsm));
   if (per <= 0) per = 1;
-  return per * sm_count();
+  return (int)std::min<size_t>((size_t)per * sm_count(), std::max<size_t>(1, L.nbulk + L.nurg));
 }
 
 static int set_smem_attr() {
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(k_sched, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmemBytes) != cudaSuccess)
+                             (int)sched_smem(true)) != cudaSuccess)
       return XKB_ECUDA;
     attr = true;
   }
@@ -1014,9 +826,9 @@ static int build_graph(GraphEntry* e) {
   KArgs a(e->d_run, L, e->schedule, e->d_times);
   cudaKernelNodeParams kp{};
   kp.func = reinterpret_cast<void*>(k_sched);
-  kp.gridDim = dim3((unsigned)std::min(grid_size(), std::max(1, L.ntasks)));
+  kp.gridDim = dim3((unsigned)grid_size(L));
   kp.blockDim = dim3(kThreads);
-  kp.sharedMemBytes = (unsigned)kSmemBytes;
+  kp.sharedMemBytes = (unsigned)sched_smem(L.ztrsm);
   kp.kernelParams = a.params;
   const cudaGraphNode_t deps[3] = {cp, m0, m1};
   if (cudaGraphAddKernelNode(&kn, e->graph, deps, 3, &kp) != cudaSuccess) return XKB_ECUDA;
@@ -1058,10 +870,8 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
       const xkb_batch_op& o = ops[c];
       if (o.M <= 0 || o.N <= 0) continue;
       if (o.kind == XKB_BATCH_GEMM) {
-        const size_t bm = o.dtype == XKB_Z ? 32 : (o.M >= tile128_rows() ? 128 : 64);
-        const size_t t = ((size_t)o.M + bm - 1) / bm * (((size_t)o.N + 63) / 64);
-        nt += t;
-        nb += t;
+        nt += 1;
+        nb += gemm_tiles(o);
       } else {
         const size_t t = ((size_t)o.M + kLeafS - 1) / kLeafS * (((size_t)o.N + kLeafS - 1) / kLeafS);
         nt += t;
@@ -1108,6 +918,8 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   }
   Layout L;
   L.set(ntasks, succ.size(), b.bulk.size(), (size_t)b.nurg, nops);
+  for (int c = 0; c < nops; ++c)
+    L.ztrsm = L.ztrsm || (ops[c].kind == XKB_BATCH_TRSM && ops[c].dtype == XKB_Z);
   // the previous batch may still read the pinned staging buffer
   if (B.h_stage) cudaStreamSynchronize(st);
   if (L.bytes > B.h_cap) {
@@ -1200,11 +1012,10 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   cudaMemsetAsync(B.d_times + nops, 0xff, sizeof(unsigned long long), st);
   B.cur_times = B.d_times;
   KArgs a(d, L, schedule, B.d_times);
-  const int grid = std::min(grid_size(), std::max(1, ntasks));
   const long long tv = evlog_kern_begin(st, "k_sched");
-  k_sched<<<grid, kThreads, kSmemBytes, st>>>(a.tasks, a.ndep, a.succ, a.bulk, a.nbulk, a.urq,
-                                              a.nurg, a.ctl, a.urgent_first, a.left,
-                                              a.call_end, a.t_start, a.wait_ns);
+  k_sched<<<grid_size(L), kThreads, sched_smem(L.ztrsm), st>>>(
+      a.tasks, a.ndep, a.succ, a.bulk, a.nbulk, a.urq, a.nurg, a.ctl, a.urgent_first, a.left,
+      a.call_end, a.t_start, a.wait_ns);
   evlog_kern_end(tv, st);
   trace_calls(tv, st, B.d_times, ops, nops);
   count_launch();
@@ -1277,7 +1088,7 @@ extern "C" int xkb_cuda_sched_wait_test(int wait_ms, void* stream) {
   auto* times = reinterpret_cast<unsigned long long*>(d + o_times);
   cudaMemsetAsync(times + 1, 0xff, sizeof(unsigned long long), st);
   const long long tv = evlog_kern_begin(st, "k_sched");
-  k_sched<<<1, kThreads, kSmemBytes, st>>>(
+  k_sched<<<1, kThreads, sched_smem(false), st>>>(
       reinterpret_cast<const Task*>(d + o_task), reinterpret_cast<int*>(d + o_ndep), nullptr,
       nullptr, 0, reinterpret_cast<int*>(d + o_urq), 1, reinterpret_cast<Ctl*>(d), 1,
       reinterpret_cast<int*>(d + o_left), times, times + 1, (unsigned long long)wait_ms * 1000000ull);

@@ -799,7 +799,7 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
   // then carry the condition number of the pairs' triangles.
   const bool inv = (dtype == XKB_D || dtype == XKB_Z) && n > kBlk && c.nrhs >= 64 &&
                    tune("trsm_inv_leaves", 1.0) != 0.0;
-  const bool pairs = inv && c.left && c.trans == XKB_OP_N && c.fwd && n >= 2048 &&
+  const bool pairs = inv && c.left && c.trans == XKB_OP_N && c.fwd && n >= 2048 && c.ozaki == 0 &&
                      tune("trsm_pair_leaves", 1.0) != 0.0;
   int npairs = 0;
   std::vector<SolveOp> ops;

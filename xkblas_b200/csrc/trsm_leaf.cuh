@@ -1,18 +1,18 @@
 // trsm_leaf.cuh -- FP64 solve of one diagonal block of a triangular system
-// (n <= 64 unknowns) against a range of right-hand sides, used by the
-// tile-task executor's solve tasks (sched.cu); leaf_at is shared with the
-// whole-matrix solver (trsm.cu).  It is the body the reference hands to
-// cublasZtrsm for a diagonal tile (blas/ztask_trsm.c:162-180).
+// (n <= 64 unknowns) against up to 64 right-hand sides by the MMA warps of the
+// tile-task executor (sched.cu); leaf_at is shared with the whole-matrix
+// solver (trsm.cu).  It is the body the reference hands to cublasZtrsm for a
+// diagonal tile (blas/ztask_trsm.c:162-180).
 //
-// X = alpha op(T)^-1 B by substitution.  A right-hand side is held by G lanes
-// of one warp, lane g keeping rows RPL*g .. RPL*g + RPL-1 in registers (real
-// RPL 16, G 4; complex RPL 8, G 8).  At step i the owner of row i scales it
-// by the reciprocal of T(i,i) (the packed-reciprocal form CPU BLAS kernels
-// use), the G lanes share it by shuffle, and each lane updates its rows below
-// (lower) or above (upper) i.  op(T) is staged column by column in shared
-// memory, row groups GS = RPL + 2 doubles apart so that the G lanes' 16-byte
-// loads fall in distinct banks.  Storage types float / double / float2 /
-// double2; arithmetic in FP64.
+// op(T), the right-hand sides and the inverses of the block's 8 x 8 diagonal
+// sub-blocks lie in shared memory.  A warp owns 16 (complex 8) right-hand
+// sides and walks the block in steps of 8 unknowns without waiting for another
+// warp: Y = inv(T_ss) X_s by one DMMA (formed as Y^T, whose accumulators are
+// the B fragment the update needs), then the rank-8 update of the unknowns
+// still to solve by DMMA, as in k_trsm_block (trsm.cu).  What bounds it is
+// latency: 8 steps of two dependent DMMAs and their shared-memory trips.  The
+// substitution it replaces (a shuffle, a product and 16 dependent updates per
+// unknown) took 40 to 60 us per block, most of a chain's time.
 #pragma once
 #include "dmma_common.cuh"
 
@@ -20,209 +20,246 @@ namespace xkb {
 
 constexpr int kLeafRows = 64;
 
-// RPL_REAL: rows per lane for real types (complex: half of it).  Fewer rows
-// per lane mean more lanes per right-hand side: more warps to hide the
-// per-step shuffle latency when right-hand sides are many, more shuffles per
-// step when they are few.
-template <class T, int RPL_REAL = 16>
+template <class T>
 struct LeafShape {
-  static constexpr bool CPLX = St<T>::CPLX;
-  static constexpr int RPL = CPLX ? RPL_REAL / 2 : RPL_REAL;  // rows per lane
-  static constexpr int G = kLeafRows / RPL;     // lanes per right-hand side
-  static constexpr int GS = RPL + 2;            // staged row-group stride
-  static constexpr int COL = G * GS;            // staged column stride
-  // shared bytes: op(T) (real [+ imaginary]) and the reciprocal diagonal
-  static constexpr size_t SMEM = (CPLX ? 2 : 1) * sizeof(double) * (kLeafRows * COL) +
-                                 2 * sizeof(double) * kLeafRows;
+  static constexpr bool CP = St<T>::CPLX;
+  static constexpr int PL = CP ? 2 : 1;
+  static constexpr int LD = kLeafRows + 2;   // column stride of T and X, = 2 mod 16
+  static constexpr int CW = CP ? 8 : 16;     // right-hand sides per warp
+  static constexpr int COLS = 4 * CW;        // and per pass of the four warps
+  static constexpr size_t T_D = (size_t)PL * kLeafRows * LD;  // doubles
+  static constexpr size_t X_D = (size_t)PL * COLS * LD;
+  static constexpr size_t V_D = (size_t)PL * (kLeafRows / 8) * 64;
+  static constexpr size_t SMEM = sizeof(double) * (T_D + X_D + V_D);
 };
+
+// Barrier of the NT threads that run the solve (the CTA may hold others).
+template <int NT>
+__device__ __forceinline__ void leaf_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+}
 
 // element (row i, right-hand side c) of B: rhs_rows ? B[c + i ldb] : B[i + c ldb]
 __device__ __forceinline__ size_t leaf_at(int i, int c, long ldb, bool rhs_rows) {
   return rhs_rows ? (size_t)c + (size_t)i * (size_t)ldb : (size_t)i + (size_t)c * (size_t)ldb;
 }
 
-// Stage op(T) for the n x n block at A: T(i,j) = A[swap ? j + i lda : i + j lda]
-// (conjugated when conj), zero outside the (lower / upper) triangle, on the
-// diagonal and beyond n; reciprocal diagonal (1 for unit and beyond n).
-// Ends with __syncthreads.
-template <class T, int NT, int RPL_REAL = 16>
-__device__ __forceinline__ void leaf_stage(const typename St<T>::S* A, long lda, int n, bool swap,
-                                           bool conj, bool lower, bool unit, double* sm) {
-  using Sh = LeafShape<T, RPL_REAL>;
-  constexpr bool CP = Sh::CPLX;
-  double* Tr = sm;
-  double* Ti = Tr + kLeafRows * Sh::COL;
-  double* Dr = Ti + (CP ? kLeafRows * Sh::COL : 0);
-  double* Di = Dr + kLeafRows;
-  // element e -> (a0, a1) = (e % 64, e / 64) at A[a0 + a1 lda]: consecutive
-  // threads read consecutive addresses for op(T) = A's triangle or its
-  // transpose; loads are issued in groups of 8 before their stores
-  constexpr int PER = kLeafRows * kLeafRows / NT;
-  constexpr int GRP = PER < 8 ? PER : 8;
-  static_assert(PER % GRP == 0, "staging split");
+// X = (ar, ai) op(T)^-1 B in place for B's nrhs columns (ldb), by 128 threads:
+// T(i,j) = A[swap ? j + i lda : i + j lda], conjugated when conj, unit: ones
+// on its diagonal.  Operands are read through L2.
+template <class T, bool LOWER>
+__device__ __forceinline__ void leaf_solve(const typename St<T>::S* A, long lda, int n, bool swap,
+                                           bool conj, bool unit, typename St<T>::S* B, long ldb,
+                                           int nrhs, double ar, double ai, double* sm) {
+  using Sh = LeafShape<T>;
+  using S = typename St<T>::S;
+  constexpr bool CP = Sh::CP;
+  constexpr int LD = Sh::LD, W = CP ? 2 : 1, NT = 128;
+  double* Tr = sm;  // T(i, j) at T[j * LD + i], zero outside the strict triangle
+  double* Ti = Tr + (CP ? kLeafRows * LD : 0);
+  double* Xr = sm + Sh::T_D;  // X[c * LD + i]
+  double* Xi = Xr + (CP ? Sh::COLS * LD : 0);
+  double* Vr = Xr + Sh::X_D;  // inverse of sub-block m: V[m * 64 + i * 8 + j]
+  double* Vi = Vr + (CP ? (kLeafRows / 8) * 64 : 0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int nsub = (n + 7) / 8;
+
+  // ---- op(T): loads in groups of 8 before their stores ----
+#pragma unroll 1
+  for (int k0 = 0; k0 < kLeafRows * kLeafRows / NT; k0 += 8) {
+    double vr[8], vi[8];
 #pragma unroll
-  for (int k0 = 0; k0 < PER; k0 += GRP) {
-    double vr[GRP], vi[GRP];
-#pragma unroll
-    for (int k = 0; k < GRP; ++k) {
-      const int e = threadIdx.x + (k0 + k) * NT;
-      const int a0 = e & (kLeafRows - 1), a1 = e / kLeafRows;
+    for (int k = 0; k < 8; ++k) {
+      const int e = tid + (k0 + k) * NT, a0 = e & (kLeafRows - 1), a1 = e / kLeafRows;
       const int i = swap ? a1 : a0, j = swap ? a0 : a1;
       vr[k] = vi[k] = 0.0;
-      if (i < n && j < n && (lower ? (j < i) : (j > i))) {
+      if (i < n && j < n && (LOWER ? j < i : j > i)) {
         const size_t idx = (size_t)a0 + (size_t)a1 * (size_t)lda;
-        if (CP) {
-          vr[k] = (double)__ldcg(A + 2 * idx);
-          vi[k] = (double)__ldcg(A + 2 * idx + 1);
-        } else {
-          vr[k] = (double)__ldcg(A + idx);
-        }
+        vr[k] = (double)__ldcg(A + W * idx);
+        if (CP) vi[k] = (double)__ldcg(A + W * idx + W - 1);
       }
     }
 #pragma unroll
-    for (int k = 0; k < GRP; ++k) {
-      const int e = threadIdx.x + (k0 + k) * NT;
-      const int a0 = e & (kLeafRows - 1), a1 = e / kLeafRows;
-      const int i = swap ? a1 : a0, j = swap ? a0 : a1;
-      const int o = j * Sh::COL + (i / Sh::RPL) * Sh::GS + (i % Sh::RPL);
+    for (int k = 0; k < 8; ++k) {
+      const int e = tid + (k0 + k) * NT, a0 = e & (kLeafRows - 1), a1 = e / kLeafRows;
+      const int o = (swap ? a0 : a1) * LD + (swap ? a1 : a0);
       Tr[o] = vr[k];
       if (CP) Ti[o] = conj ? -vi[k] : vi[k];
     }
   }
-  for (int i = threadIdx.x; i < kLeafRows; i += NT) {
-    double dr = 1.0, di = 0.0;
-    if (i < n && !unit) {
-      const size_t idx = (size_t)i + (size_t)i * (size_t)lda;
+  leaf_sync<NT>();
+  // ---- inverses of the 8 x 8 sub-blocks: thread (m, kk) column kk of
+  // inv(T_m), by substitution against a unit vector; past n the identity ----
+  if (tid < kLeafRows) {
+    const int m = tid >> 3, kk = tid & 7, d = 8 * m + kk;
+    double rk = 1.0, ik = 0.0;
+    if (!unit && d < n) {
+      const size_t idx = (size_t)d + (size_t)d * (size_t)lda;
+      const double dr = (double)__ldcg(A + W * idx);
       if (CP) {
-        dr = (double)__ldcg(A + 2 * idx);
-        di = (double)__ldcg(A + 2 * idx + 1);
-        if (conj) di = -di;
+        const double di = (conj ? -1.0 : 1.0) * (double)__ldcg(A + W * idx + W - 1);
+        const double den = dr * dr + di * di;
+        rk = dr / den;
+        ik = -di / den;
       } else {
-        dr = (double)__ldcg(A + idx);
+        rk = 1.0 / dr;
       }
     }
-    if (CP) {
-      const double den = dr * dr + di * di;
-      Dr[i] = dr / den;
-      Di[i] = -di / den;
-    } else {
-      Dr[i] = 1.0 / dr;
+    double zr[8], zi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      zr[i] = i == kk ? 1.0 : 0.0;
+      zi[i] = 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int jj = LOWER ? q : 7 - q;
+      const double dr = __shfl_sync(0xffffffffu, rk, (lane & ~7) | jj);
+      const double di = CP ? __shfl_sync(0xffffffffu, ik, (lane & ~7) | jj) : 0.0;
+      if (LOWER ? jj >= kk : jj <= kk) {
+        const double vr = zr[jj] * dr - zi[jj] * di, vi = zr[jj] * di + zi[jj] * dr;
+        zr[jj] = vr;
+        zi[jj] = vi;
+        const double* col = Tr + (8 * m + jj) * LD + 8 * m;
+        const double* coi = Ti + (8 * m + jj) * LD + 8 * m;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (LOWER ? i > jj : i < jj) {
+            const double tr = col[i], ti = CP ? coi[i] : 0.0;
+            zr[i] -= tr * vr - ti * vi;
+            if (CP) zi[i] -= tr * vi + ti * vr;
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      Vr[m * 64 + i * 8 + kk] = zr[i];
+      if (CP) Vi[m * 64 + i * 8 + kk] = zi[i];
     }
   }
-  __syncthreads();
-}
-
-// Substitution core: right-hand sides c0 .. c1-1, unknown `row` of rhs `c`
-// read by ld(row, c, re, im) (rows < n of live columns only; zero elsewhere)
-// and written back by sto(row, c, re, im).  All NT threads take part (every
-// warp runs the same number of passes).
-template <class T, int NT, bool LOWER, int RPL_REAL, class Ld, class Sto>
-__device__ __forceinline__ void leaf_solve_core(int n, int c0, int c1, const double* sm, Ld ld,
-                                                Sto sto) {
-  using Sh = LeafShape<T, RPL_REAL>;
-  constexpr int RPL = Sh::RPL, G = Sh::G, GS = Sh::GS, COL = Sh::COL;
-  constexpr int CPP = NT / G;  // right-hand sides per pass
-  constexpr bool CP = Sh::CPLX;
-  const double* Tr = sm;
-  const double* Ti = Tr + kLeafRows * COL;
-  const double* Dr = Ti + (CP ? kLeafRows * COL : 0);
-  const double* Di = Dr + kLeafRows;
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int q = tid % G, gbase = lane & ~(G - 1);
-  const int passes = (c1 - c0 + CPP - 1) / CPP;
-  for (int p = 0; p < passes; ++p) {
-    const int c = c0 + p * CPP + tid / G;
-    const bool live = c < c1;
-    double xr[RPL], xi[RPL];
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = q * RPL + r;
-      xr[r] = xi[r] = 0.0;
-      if (row < n && live) ld(row, c, xr[r], xi[r]);
-    }
-    // steps in G rounds of RPL: the register index is a compile-time constant
-    // within a round, the owning lane a run-time one
+  leaf_sync<NT>();
+  // ---- this warp's right-hand sides, nothing shared with the other warps ----
+  double* xr = Xr + warp * Sh::CW * LD;
+  double* xi = Xi + warp * Sh::CW * LD;
 #pragma unroll 1
-    for (int og = 0; og < G; ++og) {
+  for (int c0 = warp * Sh::CW; c0 < nrhs; c0 += Sh::COLS) {
+#pragma unroll 1
+    for (int q0 = 0; q0 < Sh::CW; q0 += 4) {
+      double br[8], bi[8];
 #pragma unroll
-      for (int ss = 0; ss < RPL; ++ss) {
-        const int oq = LOWER ? og : G - 1 - og, oi = LOWER ? ss : RPL - 1 - ss;
-        const int i = oq * RPL + oi;
-        double vr = __shfl_sync(0xffffffffu, xr[oi], gbase | oq);
-        double vi = CP ? __shfl_sync(0xffffffffu, xi[oi], gbase | oq) : 0.0;
-        if (CP) {
-          const double dr = Dr[i], di = Di[i];
-          const double wr = vr * dr - vi * di;
-          vi = vr * di + vi * dr;
-          vr = wr;
+      for (int k = 0; k < 8; ++k) {
+        const int i = lane + 32 * (k & 1), c = c0 + q0 + (k >> 1);
+        br[k] = bi[k] = 0.0;
+        if (i < n && c < nrhs) {
+          const size_t idx = leaf_at(i, c, ldb, false);
+          br[k] = (double)__ldcg(B + W * idx);
+          if (CP) bi[k] = (double)__ldcg(B + W * idx + W - 1);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int o = (q0 + (k >> 1)) * LD + lane + 32 * (k & 1);
+        xr[o] = ar * br[k] - ai * bi[k];
+        if (CP) xi[o] = ar * bi[k] + ai * br[k];
+      }
+    }
+    __syncwarp();
+    const int k0 = 2 * t, k1 = k0 + 1;
+#pragma unroll 1
+    for (int s = 0; s < nsub; ++s) {
+      const int m = LOWER ? s : nsub - 1 - s, b = 8 * m;
+      // Y^T = X_s^T inv(T_ss)^T (k indices 2t, 2t + 1 on both sides)
+      double yr[4] = {0.0, 0.0, 0.0, 0.0}, yi[4] = {0.0, 0.0, 0.0, 0.0};
+      {
+        constexpr bool hi = Sh::CW > 8;  // right-hand sides g + 8 exist
+        const double* v = Vr + m * 64 + g * 8;
+        const double* x = xr + g * LD + b;
+        const double a_r[4] = {x[k0], hi ? x[8 * LD + k0] : 0.0, x[k1], hi ? x[8 * LD + k1] : 0.0};
+        const double b_r[2] = {v[k0], v[k1]};
+        if constexpr (CP) {
+          const double* w = Vi + m * 64 + g * 8;
+          const double* z = xi + g * LD + b;
+          const double a_i[4] = {z[k0], 0.0, z[k1], 0.0};
+          const double n_i[4] = {-a_i[0], 0.0, -a_i[2], 0.0};
+          const double b_i[2] = {w[k0], w[k1]};
+          dmma_k8(yr, a_r, b_r);
+          dmma_k8(yr, n_i, b_i);
+          dmma_k8(yi, a_r, b_i);
+          dmma_k8(yi, a_i, b_r);
         } else {
-          vr *= Dr[i];
+          dmma_k8(yr, a_r, b_r);
         }
-        if (q == oq) {
-          xr[oi] = vr;
-          if (CP) xi[oi] = vi;
+      }
+      __syncwarp();  // every lane has read X_s
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int c = g + ((v >> 1) << 3);
+        if (c < Sh::CW) {
+          xr[c * LD + b + k0 + (v & 1)] = yr[v];
+          if (CP) xi[c * LD + b + k0 + (v & 1)] = yi[v];
         }
-        // update row > i (lower) / row < i (upper): the staged column holds
-        // zeros outside the triangle, but the predicate keeps final rows
-        // untouched even when v is not finite
-        const double2* colr = reinterpret_cast<const double2*>(Tr + i * COL + q * GS);
-        const double2* coli = reinterpret_cast<const double2*>(Ti + i * COL + q * GS);
+      }
+      // rows still to solve -= T(rows, b .. b+7) Y
+      const int u0 = LOWER ? b + 8 : 0, u1 = LOWER ? 8 * nsub : b;
+#pragma unroll 1
+      for (int m0 = u0; m0 < u1; m0 += 16) {
+        // rows past u1 (a last half tile) are read in range and not stored
+        const int ra = m0 + g, rb = min(m0 + g + 8, kLeafRows - 1);
+        const double* t0 = Tr + (b + k0) * LD;
+        const double* t1 = t0 + LD;
+        const double a_r[4] = {-t0[ra], -t0[rb], -t1[ra], -t1[rb]};
+        double a_i[4] = {0.0, 0.0, 0.0, 0.0}, n_i[4] = {0.0, 0.0, 0.0, 0.0};
+        if constexpr (CP) {
+          const double* s0 = Ti + (b + k0) * LD;
+          const double* s1 = s0 + LD;
+          a_i[0] = -s0[ra], a_i[1] = -s0[rb], a_i[2] = -s1[ra], a_i[3] = -s1[rb];
 #pragma unroll
-        for (int h = 0; h < RPL / 2; ++h) {
-          const double2 tr = colr[h];
-          double2 ti = make_double2(0.0, 0.0);
-          if (CP) ti = coli[h];
+          for (int v = 0; v < 4; ++v) n_i[v] = -a_i[v];
+        }
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int r = 2 * h + u;
-            const int row = q * RPL + r;
-            const double a = u ? tr.y : tr.x;
-            if (LOWER ? row > i : row < i) {
-              if (CP) {
-                const double b = u ? ti.y : ti.x;
-                xr[r] -= a * vr - b * vi;
-                xi[r] -= a * vi + b * vr;
-              } else {
-                xr[r] -= a * vr;
-              }
+        for (int n0 = 0; n0 < Sh::CW; n0 += 8) {
+          const double b_r[2] = {n0 ? yr[2] : yr[0], n0 ? yr[3] : yr[1]};
+          double cr[4], ci[4];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int o = (n0 + 2 * t + (v & 1)) * LD + (v >> 1 ? rb : ra);
+            cr[v] = xr[o];
+            ci[v] = CP ? xi[o] : 0.0;
+          }
+          if constexpr (CP) {
+            const double b_i[2] = {yi[0], yi[1]};
+            dmma_k8(cr, a_r, b_r);
+            dmma_k8(cr, n_i, b_i);
+            dmma_k8(ci, a_r, b_i);
+            dmma_k8(ci, a_i, b_r);
+          } else {
+            dmma_k8(cr, a_r, b_r);
+          }
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int row = m0 + g + ((v >> 1) << 3);
+            const int o = (n0 + 2 * t + (v & 1)) * LD + row;
+            if (row < u1) {
+              xr[o] = cr[v];
+              if (CP) xi[o] = ci[v];
             }
           }
         }
       }
+      __syncwarp();
     }
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = q * RPL + r;
-      if (row < n && live) sto(row, c, xr[r], xi[r]);
+#pragma unroll 4
+    for (int q = 0; q < 2 * Sh::CW; ++q) {
+      const int i = lane + 32 * (q & 1), c = c0 + (q >> 1);
+      if (i < n && c < nrhs) {
+        const size_t idx = leaf_at(i, c, ldb, false);
+        B[W * idx] = static_cast<S>(xr[(q >> 1) * LD + i]);
+        if (CP) B[W * idx + W - 1] = static_cast<S>(xi[(q >> 1) * LD + i]);
+      }
     }
+    __syncwarp();
   }
-}
-
-// Solve right-hand sides c0 .. c1-1 of B in place (alpha applied on load).
-template <class T, int NT, bool LOWER, int RPL_REAL = 16>
-__device__ __forceinline__ void leaf_solve(typename St<T>::S* B, long ldb, bool rhs_rows, int n,
-                                           int c0, int c1, double ar, double ai,
-                                           const double* sm) {
-  constexpr bool CP = St<T>::CPLX;
-  using S = typename St<T>::S;
-  leaf_solve_core<T, NT, LOWER, RPL_REAL>(
-      n, c0, c1, sm,
-      [&](int row, int c, double& xr, double& xi) {
-        const size_t idx = leaf_at(row, c, ldb, rhs_rows);
-        const double br = CP ? (double)__ldcg(B + 2 * idx) : (double)__ldcg(B + idx);
-        const double bi = CP ? (double)__ldcg(B + 2 * idx + 1) : 0.0;
-        xr = ar * br - ai * bi;
-        if (CP) xi = ar * bi + ai * br;
-      },
-      [&](int row, int c, double xr, double xi) {
-        const size_t idx = leaf_at(row, c, ldb, rhs_rows);
-        if (CP) {
-          B[2 * idx] = static_cast<S>(xr);
-          B[2 * idx + 1] = static_cast<S>(xi);
-        } else {
-          B[idx] = static_cast<S>(xr);
-        }
-      });
 }
 
 }  // namespace xkb
