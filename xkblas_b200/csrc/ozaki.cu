@@ -310,33 +310,53 @@ __global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const E* X, long 
   // block: 32 rows x 8 lanes along k (KC: warp-cooperative along k instead)
   const int chunk = blockIdx.y;
   const int k0 = chunk * kNormChunk, k1 = min(K, k0 + kNormChunk);
-  double ss = 0.0, mx = 0.0, s1 = EXACT ? 1.0e6 : 0.0, nz = 0.0;
+  double ss = 0.0, mx = 0.0, s1 = 0.0, nz = 0.0;
+  int lo = 1000000, cnt = 0;
   auto merge = [](double a, double b) { return EXACT ? fmin(a, b) : a + b; };
   auto acc = [&](E x) {
     const double v = (double)x;
     ss = fma(v, v, ss);
     mx = fmax(mx, fabs(v));
     if constexpr (EXACT) {
-      if (x != 0.0f) s1 = fmin(s1, (double)lsb_exp(x));
+      if (x != 0.0f) lo = min(lo, lsb_exp(x));
     } else {
       s1 += fabs(v);
+      cnt += v != 0.0;
     }
-    nz += (v != 0.0) ? 1.0 : 0.0;
+  };
+  // eight elements (complex: pairs) in flight; zeros past the end add nothing
+  auto run = [&](int kb, int step, size_t base, size_t stride) {
+    for (int k = kb; k < k1; k += 8 * step) {
+      E a[8], b[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int kk = k + q * step;
+        a[q] = b[q] = (E)0;
+        if (kk < k1) {
+          const size_t i = base + (size_t)kk * stride;
+          if (cplx) {
+            a[q] = X[2 * i];
+            b[q] = X[2 * i + 1];
+          } else {
+            a[q] = X[i];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        acc(a[q]);
+        if (cplx) acc(b[q]);
+      }
+    }
+    if (EXACT) s1 = (double)lo;
+    nz = (double)cnt;
   };
   if constexpr (KC) {
     // one warp per row: lanes stride along contiguous k
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int l = blockIdx.x * 8 + warp;
-    if (l < L) {
-      for (int k = k0 + lane; k < k1; k += 32) {
-        if (cplx) {
-          acc(X[2 * ((size_t)k + (size_t)l * ld)]);
-          acc(X[2 * ((size_t)k + (size_t)l * ld) + 1]);
-        } else {
-          acc(X[(size_t)k + (size_t)l * ld]);
-        }
-      }
-    }
+    if (l < L) run(k0 + lane, 32, (size_t)l * ld, 1);
+    else if (EXACT) s1 = 1.0e6;
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
       ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -350,16 +370,7 @@ __global__ void __launch_bounds__(256) k_oz_norm(int L, int K, const E* X, long 
     __shared__ double4 red[8][32];
     const int tl = threadIdx.x & 31, tk = threadIdx.x >> 5;
     const int l = blockIdx.x * 32 + tl;
-    if (l < L) {
-      for (int k = k0 + tk; k < k1; k += 8) {
-        if (cplx) {
-          acc(X[2 * ((size_t)l + (size_t)k * ld)]);
-          acc(X[2 * ((size_t)l + (size_t)k * ld) + 1]);
-        } else {
-          acc(X[(size_t)l + (size_t)k * ld]);
-        }
-      }
-    }
+    if (l < L) run(k0 + tk, 8, (size_t)l, (size_t)ld);
     red[tk][tl] = make_double4(ss, mx, s1, nz);
     __syncthreads();
     if (tk == 0 && l < L) {
