@@ -697,6 +697,7 @@ struct GemmP {
   int tiles_m, tiles_n, kblocks, nmod;  // nmod: planes of the operand buffers (the most used)
   const OzSel* sel;                     // planes multiplied: mult sel->np (<= nmod)
   int mult;                             // planes per modulus: 1, complex 2
+  const int* list;  // not null: list[0] tiles (list[1 ..]) of every plane are in the triangle
   int bxor;  // plane z of op(A) meets plane z ^ bxor of op(B) (1: B is A's conjugate)
   int group;  // raster: M tiles per group (tiles in flight share A / B panels in L2)
   uint8_t* R;
@@ -749,9 +750,10 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, int
 // tile t of the (modulus-major, grouped raster) list; false if the tile lies
 // wholly outside the written triangle
 __device__ __forceinline__ bool oz_tile(const GemmP& p, int t, int& mod, int& m0, int& n0) {
-  const int tiles_mn = p.tiles_m * p.tiles_n;
+  const int tiles_mn = p.list ? p.list[0] : p.tiles_m * p.tiles_n;
   mod = t / tiles_mn;
-  const int r = t - mod * tiles_mn;
+  int r = t - mod * tiles_mn;
+  if (p.list) r = p.list[1 + r];
   const int GROUP = p.group;
   const int span = GROUP * p.tiles_n;
   const int first_m = (r / span) * GROUP;
@@ -763,6 +765,33 @@ __device__ __forceinline__ bool oz_tile(const GemmP& p, int t, int& mod, int& m0
   if (p.uplo == XKB_LOWER && (long)(m0 + BM - 1) + p.diag < (long)n0) return false;
   if (p.uplo == XKB_UPPER && (long)m0 + p.diag > (long)(n0 + BN - 1)) return false;
   return true;
+}
+
+// The tiles of one plane that meet the triangle, in raster order (one block of
+// 1024 threads).  Walking all tiles with a fixed stride and skipping those
+// outside gave the CTAs uneven shares: 4 to 10 % of a ZHERK 8192, by the
+// raster group.
+__global__ void __launch_bounds__(1024) k_oz_tiles(const GemmP p, int* list) {
+  __shared__ int sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (int r0 = 0; r0 < p.tiles_m * p.tiles_n; r0 += 1024) {
+    const int r = r0 + (int)threadIdx.x;
+    int mod, m0, n0;
+    const bool in = r < p.tiles_m * p.tiles_n && oz_tile(p, r, mod, m0, n0);
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) sums[warp] = __popc(b);
+    __syncthreads();
+    int before = base, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += sums[w];
+      all += sums[w];
+    }
+    if (in) list[1 + before + __popc(b & ((1u << lane) - 1u))] = r;
+    base += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) list[0] = base;
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t addr) {
@@ -837,7 +866,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t* acce = accf + 2;   // [2] accumulator drained
   uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
 
-  const int total = p.tiles_m * p.tiles_n * min(p.sel->np * p.mult, p.nmod);
+  const int total =
+      (p.list ? p.list[0] : p.tiles_m * p.tiles_n) * min(p.sel->np * p.mult, p.nmod);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -1802,11 +1832,13 @@ static bool encode_planes(CUtensorMap* m, const int8_t* base, long Kpad, long Lp
 // (0: the same): rows between consecutive planes, when Ap / Bp point at a
 // block of rows of larger planes.
 // c: the plan's largest count; null: a complex product of cplanes planes
-// (bxor: see GemmP).
+// (bxor: see GemmP).  list: room for the tiles of a masked product (1 + one int
+// per 128 x 256 tile), or null.
 static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_rows, long Mpad,
                        long Npad, long Kpad, const Consts* c, const OzSel* sel, uint8_t* R,
                        int uplo, long diag, cudaStream_t st, long a_stride = 0,
-                       long b_stride = 0, int cplanes = 0, int bxor = 0) {
+                       long b_stride = 0, int cplanes = 0, int bxor = 0,
+                       int* list = nullptr) {
   CUtensorMap tA, tB;
   const int npl = c ? c->nmod : cplanes;
   if (a_rows < Mpad || b_rows < Npad) return XKB_EINVAL;
@@ -1883,6 +1915,11 @@ static int launch_gemm(const int8_t* Ap, long a_rows, const int8_t* Bp, long b_r
   const long total = (long)p.tiles_m * p.tiles_n * npl;
   const unsigned grid = (unsigned)std::min<long>(total, sm_count());  // persistent
   const long long tv = evlog_kern_begin(st, "k_oz_gemm");
+  if (list && uplo != XKB_FULL) {
+    k_oz_tiles<<<1, 1024, 0, st>>>(p, list);
+    p.list = list;
+    count_launch();
+  }
   k_oz_gemm<<<grid, kGemmThreads, smem, st>>>(tA, tB, p);
   evlog_kern_end(tv, st);
   count_launch();
@@ -1976,7 +2013,9 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   auto alloc = [&](void** p, size_t n) {
     return cudaMallocAsync(p, std::max<size_t>(n, 256), st) == cudaSuccess;
   };
-  bool ok = alloc((void**)&Ap, szA) && (same || alloc((void**)&Bp, szB)) &&
+  int* list = nullptr;  // the INT8 tiles of a masked product
+  const size_t szL = a->uplo == XKB_FULL ? 0 : 4 * (1 + (size_t)(Mpad / BM) * (Npad / BN));
+  bool ok = (!szL || alloc((void**)&list, szL)) && alloc((void**)&Ap, szA) && (same || alloc((void**)&Bp, szB)) &&
             alloc((void**)&R, szR) && alloc((void**)&mu, sizeof(int) * M) &&
             alloc((void**)&nu, sizeof(int) * N) && alloc((void**)&pw, szPart);
   int err = ok ? XKB_OK : XKB_ENOMEM;
@@ -2010,7 +2049,7 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   trace_mark(slot, 1, st);
   if (!err)
     err = launch_gemm(Ap, Arows, same ? Ap : Bp, same ? Arows : Npad, Mpad, Npad, Kpad, c, sel, R,
-                      a->uplo, a->diag, st, 0, 0, nmax, bxor);
+                      a->uplo, a->diag, st, 0, 0, nmax, bxor, list);
   trace_mark(slot, 2, st);
   if (!err) {
     CrtP cp;
@@ -2051,6 +2090,7 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   if (!err && (exact || !pl.fixed)) err = gemm_if(a, &w->sel.fallback, st);
   if (!err && cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
   trace_mark(slot, 3, st);
+  if (list) cudaFreeAsync(list, st);
   if (Ap) cudaFreeAsync(Ap, st);
   if (Bp) cudaFreeAsync(Bp, st);
   if (R) cudaFreeAsync(R, st);
