@@ -313,6 +313,14 @@ __global__ void __launch_bounds__(C_::CTA, C_::MINB)
   const int ntiles = p.tiles_m * p.tiles_n;
   const int slice = (int)blockIdx.x / ntiles;  // 0 unless split-K
   const int bid = (int)blockIdx.x - slice * ntiles;
+  int m0, n0;
+  if (!dmma_tile<C_::BM, C_::BN>(p, bid, m0, n0)) {
+    // a tile outside the triangle leaves at once (behind the wait it cost a
+    // masked K = 256 update 9 %); block 0 waits all the same, so that the grid
+    // never ends before its predecessor
+    if (blockIdx.x == 0) pdl_wait();
+    return;
+  }
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     tma_prefetch(&tmA);
@@ -329,8 +337,6 @@ __global__ void __launch_bounds__(C_::CTA, C_::MINB)
   // fallback): every thread reads the same word, so the whole CTA leaves
   // before touching shared memory, barriers or C
   if (p.run_if && *p.run_if == 0) return;
-  int m0, n0;
-  if (!dmma_tile<C_::BM, C_::BN>(p, bid, m0, n0)) return;
   __syncthreads();
 
   // this CTA's stages: [kt0, kt0 + KT)
@@ -529,56 +535,67 @@ static int dispatch_ops(const xkb_gemm_args* a, cudaStream_t st, const int* run_
 // Tile and split of one call, by a model of its time on the SMs: n tiles
 // spread over the SMs make q = ceil(n / SMs) on the fullest one, R of them at
 // a time; r resident CTAs reach the fraction e[r] of an SM's DMMA rate (alone,
-// a CTA's four MMA warps wait for their own fragments), every wave of R adds
-// `wave` microseconds (fill, drain, epilogue; less once the CTAs of an SM
-// have drifted apart), and split-K adds its reduction.  e was measured with
-// 148 r tiles of K = 2048 (B200, NN): 64 x 64 0.70 / 0.88 / 0.95 for 1 / 2 /
-// 3 CTAs, 32 x 32 0.42 / 0.68 / 0.76 / 0.80 / 0.90 for 1 .. 5, complex 32 x 32
-// 0.63 / 0.84 / 0.89.  Measured (us; before: 128 x 128 tiles one CTA per SM,
-// split-K and stream-K over them, 64 x 64 tiles with unswizzled operands):
-//   8192^2 x 512: 64 x 64 1989, 32 x 32 2089 (before 2330)
-//   7680^2 lower x 256: 488, 513 (597)     2048^2 x 512: 151, 139 (183)
-//   1024^3: 78, 72, split 4 x 64 x 64 78 (93)    512^3: 29, 16 (35)
+// a CTA's four MMA warps wait for their own fragments); `base`, `wave` and
+// `tile` microseconds are added once, per wave of R (fill, drain, epilogue)
+// and per tile; split-K adds its reduction.  The constants fit these times
+// (B200, us; before: 128 x 128 tiles one CTA per SM, split-K and stream-K over
+// them, 64 x 64 tiles with unswizzled operands):
+//   8192^2 x 512: 64 x 64 1983, 32 x 32 2121 (before 2330)
+//   7680^2 lower x 256: 532, 521 (597)     2048^2 x 512: 131, 138 (183)
+//   2048^3: 502, 532 (646)     3001 x 517 x 777: 90, 83 (121)
+//   3000^2 x 300: 172, 179     1500^3: 217, 214     4096^2 x 128 lower: 108, 94
+//   1024^3: 114, 72, split 4 x 64 x 64 78 (93)    512^3: 29, 16 (35)
 //   512^2 x 4096: 183, 92, split 4 x 32 x 32 80 (86)
 //   1000 x 900 x 3000: 217, 203, split 3 x 64 x 64 189 (217)
-//   complex 1200 x 900 x 1100: 327, split 2 315 (642)
+//   complex 1200 x 900 x 1100: 327, split 2 312 (642)
 // Stream-K over the same tiles (every CTA an equal share of the k steps) lost
 // to the better of these everywhere measured, by 2 to 40 %.
 struct TilePlan {
   bool small;  // the 32 x 32 tile
   int ksplit;
 };
+struct TileCost {
+  int R;
+  double e[5], base, wave, tile;
+};
 
-inline double tile_cost(long n, double unit_us, const double* e, int R, double wave) {
+inline double tile_cost(long n, double unit_us, const TileCost& c) {
   const long sms = sm_count();
-  const long q = (n + sms - 1) / sms, full = q / R, rem = q % R;
-  double t = unit_us * ((double)(full * R) / e[R - 1] + (rem ? (double)rem / e[rem - 1] : 0.0));
-  const double waves = (double)(full + (rem ? 1 : 0));
-  return t + wave * std::min(waves, 6.0) + 0.36 * wave * std::max(0.0, waves - 6.0);
+  const long q = (n + sms - 1) / sms, full = q / c.R, rem = q % c.R;
+  return unit_us * ((double)(full * c.R) / c.e[c.R - 1] + (rem ? (double)rem / c.e[rem - 1] : 0.0)) +
+         c.base + c.wave * (double)(full + (rem ? 1 : 0)) + c.tile * (double)q;
 }
 
 template <class T>
 static TilePlan plan_tiles(const xkb_gemm_args* a) {
   constexpr bool CPLX = St<T>::CPLX;
-  static const double e64[3] = {0.70, 0.88, 0.95}, e32[5] = {0.42, 0.68, 0.76, 0.80, 0.90},
-                      ez[3] = {0.63, 0.84, 0.89};
+  static const TileCost c64{3, {0.74, 0.90, 0.985}, 8.5, 3.2, 0.0},
+      c64s{3, {0.74, 0.90, 0.985}, 1.0, 1.2, 0.0},  // a slice: no C, no epilogue
+      c32{5, {0.42, 0.68, 0.76, 0.80, 0.93}, 1.5, 0.0, 0.3},
+      cz{3, {0.63, 0.84, 0.89}, 1.5, 1.0, 0.0};
   auto tiles = [&](int b) {
     const long tm = (a->M + b - 1) / b, tn = (a->N + b - 1) / b;
     return a->uplo == XKB_FULL ? tm * tn : (tm * tn + std::max(tm, tn)) / 2;
   };
+  // tuning table: 64 x 64 tiles from this many 128 x 128 blocks of C on
+  // (XKBLAS_GEMM_TILE=big|small: always / never); the split stays the model's
+  static const char* force = getenv("XKBLAS_GEMM_TILE");
+  const double big = force ? (force[0] == 'b' ? 0.0 : 1e18) : tune("gemm_big_min_tiles", -1.0);
+  const bool fixed = !CPLX && big >= 0.0;
+  const bool want_small =
+      (double)((a->M + 127) / 128) * (double)((a->N + 127) / 128) < big;
   TilePlan best{true, 1};
   double tbest = 1e300;
   for (int c = CPLX ? 1 : 0; c < 2; ++c) {
     const bool small = c == 1;
+    if (fixed && small != want_small) continue;
     const int b = small ? 32 : 64;
-    const double* e = CPLX ? ez : (small ? e32 : e64);
-    const int R = CPLX ? 3 : (small ? 5 : 3);
     const long n = tiles(b);
     // microseconds of one tile at the SM's full rate (64 FMA a cycle)
     const double unit = (double)b * b * (CPLX ? 4.0 : 1.0) * (double)a->K / 64.0 / 1965.0;
     for (int ks = 1; ks <= 32; ks = ks < 4 ? ks + 1 : ks + ks / 2) {
       if (ks > 1 && (a->K < 128 * ks || n * ks > 32 * (long)sm_count())) break;
-      double t = tile_cost(n * ks, unit / ks, e, R, small ? 1.5 : (ks > 1 ? 1.2 : 5.5));
+      double t = tile_cost(n * ks, unit / ks, CPLX ? cz : small ? c32 : ks > 1 ? c64s : c64);
       // reduction: a launch, and every slice written and read once (L2)
       if (ks > 1) t += 4.0 + (double)n * b * b * (CPLX ? 32.0 : 16.0) * ks * 1e-7;
       if (t < tbest) {
@@ -587,12 +604,6 @@ static TilePlan plan_tiles(const xkb_gemm_args* a) {
       }
     }
   }
-  // tuning table: 64 x 64 tiles from this many 128 x 128 blocks of C on
-  // (XKBLAS_GEMM_TILE=big|small: always / never)
-  static const char* force = getenv("XKBLAS_GEMM_TILE");
-  const double big = force ? (force[0] == 'b' ? 0.0 : 1e18) : tune("gemm_big_min_tiles", -1.0);
-  if (!CPLX && big >= 0.0)
-    best = {(double)((a->M + 127) / 128) * (double)((a->N + 127) / 128) < big, 1};
   if (tune("gemm_splitk", 1.0) == 0.0) best.ksplit = 1;
   return best;
 }
