@@ -6,8 +6,10 @@ loads at init (XKBLAS_TUNE_FILE):
     XKBLAS_TUNE_FILE=xkblas_tune.txt ./app
 
 Choices (keys of the table, see include/xkb_cuda.h):
-  gemm_big_min_tiles      whole-matrix FP64 GEMM: 128-wide tiles from this many
-                          tiles on (timed: both tile shapes on square DGEMMs);
+  gemm_big_min_tiles      whole-matrix real GEMM: 64 x 64 tiles from this many
+                          128 x 128 blocks of C on, else 32 x 32 (timed: both
+                          tile shapes on square DGEMMs; without the key the
+                          library chooses by a model of the time);
   ozaki_min_dim           tensor-op mode: Ozaki from this size on (timed:
                           plain DMMA vs Ozaki on square DGEMMs);
   ozaki_moduli_k<=<K>     moduli count per inner-size band (measured error:
@@ -20,8 +22,8 @@ Choices (keys of the table, see include/xkb_cuda.h):
   ozaki_panel_cols        column width of the panels a public-API Ozaki DGEMM
                           streams through (timed end to end with pinned host
                           matrices, 8192^3, caches dropped per call);
-  batch_schedule,         tile-task executor: claim order and 128-row tile
-  batch_tile128_min_rows  threshold (timed on a mixed batch of uneven calls).
+  batch_schedule          tile-task executor: claim order (timed on a mixed
+                          batch of uneven calls).
 
 Each measurement uses seeded synthetic matrices and CUDA events (the panel
 sweep: host clock around the public calls); the table records the measured
@@ -216,16 +218,13 @@ class Tuner:
         arr = (X.BatchOp * len(ops))(*ops)
         best = None
         for sched in (0, 1):
-            for rows in ((96, 1 << 20) if self.quick else (64, 96, 160, 1 << 20)):
-                lib.xkb_tune_set(b"batch_tile128_min_rows", float(rows))
-                lib.xkb_cuda_batch_release()
-                ms = self.time(lambda: lib.xkb_cuda_batch(arr, len(ops), sched, self.sp), 3)
-                self.log("batch schedule %d tile128 rows >= %d: %.2f ms" % (sched, rows, ms))
-                if best is None or ms < best[0]:
-                    best = (ms, sched, rows)
+            lib.xkb_cuda_batch_release()
+            ms = self.time(lambda: lib.xkb_cuda_batch(arr, len(ops), sched, self.sp), 3)
+            self.log("batch schedule %d: %.2f ms" % (sched, ms))
+            if best is None or ms < best[0]:
+                best = (ms, sched)
         lib.xkb_cuda_batch_release()
         self.table["batch_schedule"] = (best[1], "%.2f ms best of the sweep" % best[0])
-        self.table["batch_tile128_min_rows"] = (best[2], "%.2f ms best of the sweep" % best[0])
 
     def ozaki_kernel(self):
         """Single-CTA or CTA-pair INT8 GEMM (oz_2cta)."""

@@ -16,7 +16,8 @@
 //   * errors are returned, never abort();
 //   * gemmt writes only the uplo triangle (the reference's GPU body writes
 //     the whole diagonal tile, blas/ztask_gemmt.c:213);
-//   * float / complex-float operands are computed in FP64 and rounded once.
+//   * float / complex-float operands are computed in FP64 (large products
+//     exactly, ozaki.cu) and rounded once.
 #include <algorithm>
 #include <cerrno>
 #include <cmath>

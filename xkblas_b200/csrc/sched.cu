@@ -6,7 +6,7 @@
 // (kaapi/kaapi_task.c:1277-1327) and the device threads that pop ready tasks
 // and launch one cuBLAS call each (kaapi/kaapi_offload_device.c:463-683,
 // 852-1210).  The host builds the task graph once; persistent CTAs (as many
-// as fit, two per SM) take dependency-free tasks from a bulk list and the
+// as fit, three per SM) take dependency-free tasks from a bulk list and the
 // others from a device-side ready queue that completing tasks append their
 // successors to.  A batch of small, uneven calls thus costs one launch
 // instead of one launch (or thousands of tile tasks with host round trips)

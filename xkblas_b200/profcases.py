@@ -10,10 +10,10 @@ ozaki2  the same with the CTA-pair INT8 kernel (tuning key oz_2cta = 1, k_oz_gem
 ozaki8192  DGEMM NN 8192^3, xkb_cuda_ozaki_gemm with the count chosen on the
         device (nmod = 0: 15 moduli on these inputs), two calls: the DRAM
         traffic of k_oz_gemm at a size whose residue planes exceed L2
-splitk  DGEMM NN 512 x 512 x 4096 through xkb_cuda_gemm: 16 output tiles,
-        split-K (k_gemm_dmma slices + k_gemm_splitk)
-streamk DGEMM TN 640 x 1280 x 2048 through xkb_cuda_gemm: 50 output tiles,
-        stream-K (k_gemm_dmma_sk pieces + k_gemm_sk_reduce), two calls
+splitk  DGEMM NN 512 x 512 x 4096 through xkb_cuda_gemm: 256 output tiles of
+        32 x 32, split-K (k_gemm_dmma slices + k_gemm_splitk)
+streamk DGEMM TN 640 x 1280 x 2048 through xkb_cuda_gemm: few tiles and a
+        long K, tile and split by the time model, two calls
 repack  the DGEMM with lda = ldb = 4097 (k_repack, then k_gemm_dmma)
 trsm    DTRSM L/L/N/N 4096 x 4096, diagonally dominant (k_trsm_block, GEMMs)
 potrf   DPOTRF lower 4096 (k_potrf_block, k_trsm_block, GEMMs)
