@@ -203,6 +203,12 @@ int xkb_trace_take(xkb_trace_rec* out, int max);
  * the context stays usable.  Returns once launched. */
 int xkb_cuda_sched_wait_test(int wait_ms, void* stream);
 
+/* Check of the paths without device scratch (no counterpart in the
+ * reference): the fail-th scratch request that this thread's calls make from
+ * now on is refused, and only that one (0: none).  Returns the requests made
+ * since the last call of this function. */
+int xkb_cuda_scratch_test(int fail);
+
 /* Batched execution: a list of independent GEMM / left-TRSM calls on device
  * operands run as ONE persistent launch of tile tasks (a DAG with device
  * dependency counters; replaces the reference's task runtime,

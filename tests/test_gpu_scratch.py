@@ -1,0 +1,88 @@
+"""Calls whose device scratch is refused: for every scratch request that a call
+makes, the same call with that one request refused either returns the right
+result or XKB_ENOMEM with its output untouched.  Large single-precision and
+tensor-op products are the ones that could write C and then be refused (they
+launch a predicated plain product with scratch of its own).  Requires a B200."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+XKB_ENOMEM = -3
+CODE = {"s": 0, "d": 1, "c": 2, "z": 3}
+NP = {"s": np.float32, "d": np.float64, "c": np.complex64, "z": np.complex128}
+
+
+def rnd(r, t, rows, cols):
+    v = r.random((rows, cols)) - 0.5
+    if t in "cz":
+        v = v + 1j * (r.random((rows, cols)) - 0.5)
+    return np.asfortranarray(v.astype(NP[t]))
+
+
+def dev(X, pad):
+    import torch
+    b = np.zeros((X.shape[1], X.shape[0] + pad), X.dtype)
+    b[:, :X.shape[0]] = X.T
+    return torch.from_numpy(b).cuda()
+
+
+def each_refusal(xk, out0, ref, tol, call):
+    """call(out) on a fresh device copy of out0, once per scratch request."""
+    import torch
+    lib = xk.lib()
+    lib.xkb_cuda_scratch_test(0)
+    seen = refused = 0
+    for nth in range(40):  # 0: no refusal, then each request in turn
+        out = out0.clone()
+        torch.cuda.synchronize()
+        lib.xkb_cuda_scratch_test(nth)
+        rc = call(out)
+        n = lib.xkb_cuda_scratch_test(0)
+        xk.sync()
+        if rc == 0:
+            err = np.linalg.norm(out.cpu().numpy() - ref) / np.linalg.norm(ref)
+            assert err < tol, (nth, err)
+        else:
+            assert rc == XKB_ENOMEM, (nth, rc)
+            assert torch.equal(out, out0), "request %d refused, output changed" % nth
+            refused += 1
+        if nth == 0:
+            assert rc == 0
+            seen = n
+        elif nth >= seen and n < nth:
+            break  # no request was refused
+    assert lib.xkb_cuda_take_device_error() == 0
+    return seen, refused
+
+
+@pytest.mark.parametrize("t,M,N,K,pad,tensor_op", [
+    ("s", 520, 540, 600, 1, False), ("c", 520, 540, 600, 1, False),
+    ("s", 512, 512, 4096, 0, False), ("c", 512, 512, 2048, 0, False),
+    ("d", 520, 540, 600, 1, True), ("z", 300, 270, 400, 1, True), ("d", 512, 512, 4096, 0, True),
+])
+def test_product(xk, t, M, N, K, pad, tensor_op):
+    lib = xk.lib()
+    r = np.random.default_rng(5)
+    A, B, C0 = rnd(r, t, M, K), rnd(r, t, K, N), rnd(r, t, M, N)
+    wide = np.complex128 if t in "cz" else np.float64
+    ref = np.zeros((N, M + pad), wide)
+    ref[:, :M] = (0.75 * (A.astype(wide) @ B.astype(wide)) + 0.5 * C0).T
+    dA, dB, dC = dev(A, pad), dev(B, pad), dev(C0, pad)
+
+    def call(out):
+        g = xk.GemmArgs(CODE[t], 0, 0, M, N, K, dA.data_ptr(), M + pad, dB.data_ptr(), K + pad,
+                        out.data_ptr(), M + pad)
+        g.alpha[0], g.beta[0] = 0.75, 0.5
+        if tensor_op:
+            return lib.xkb_cuda_ozaki_gemm(ctypes.byref(g), 0, None)
+        return lib.xkb_cuda_gemm(ctypes.byref(g), None)
+
+    lib.xkb_tune_set(b"gemm_exact_min", 0.0)
+    try:
+        seen, _ = each_refusal(xk, dC, ref, 1e-6 if t in "sc" else 1e-14, call)
+    finally:
+        lib.xkb_tune_set(b"gemm_exact_min", 3.4e9)
+    assert seen >= 6  # the INT8 form ran

@@ -172,8 +172,9 @@ extern "C" int xkb_cuda_scale(int dtype, int M, int N, const double* beta, void*
 }
 
 namespace xkb {
-// The whole-matrix product; run_if not null: the kernel runs only where the
-// device word is non-zero (operand repacking, if any, runs regardless).
+// The whole-matrix product; run_if not null: its kernels (an operand copy among
+// them) do nothing unless the device word is non-zero.  XKB_ENOMEM is returned
+// before the kernel that writes C is launched.
 static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if) {
   if (!a || a->M < 0 || a->N < 0 || a->K < 0) return XKB_EINVAL;
   if (a->dtype < XKB_S || a->dtype > XKB_Z) return XKB_EINVAL;
@@ -212,10 +213,7 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
     const long la = packed_ld(ra, es), lb = packed_ld(rb, es);
     const size_t za = okA ? 0 : ((size_t)la * ca * es + 255) / 256 * 256;
     const size_t zb = okB || same ? 0 : (size_t)lb * cb * es;
-    if (cudaMallocAsync(&pack, std::max<size_t>(za + zb, 256), st) != cudaSuccess) {
-      cudaGetLastError();
-      return XKB_ENOMEM;
-    }
+    if (!scratch_alloc(&pack, za + zb, st)) return XKB_ENOMEM;
     CopyArray d[2];
     int n = 0;
     if (!okA) {

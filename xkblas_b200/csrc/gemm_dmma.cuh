@@ -500,13 +500,10 @@ static int launch_dmma(const xkb_gemm_args* a, cudaStream_t st, const int* run_i
       return XKB_ECUDA;
     attr_done = true;
   }
-  if (p.ksplit > 1) {
-    const size_t ws = (size_t)p.ksplit * ntiles * C_::NREG * C_::THREADS * 8;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&p.ws), ws, st) != cudaSuccess) {
-      cudaGetLastError();
-      return XKB_ENOMEM;
-    }
-  }
+  if (p.ksplit > 1 &&
+      !scratch_alloc(reinterpret_cast<void**>(&p.ws),
+                     (size_t)p.ksplit * ntiles * C_::NREG * C_::THREADS * 8, st))
+    return XKB_ENOMEM;
   const long long tv = evlog_kern_begin(st, p.ksplit > 1 ? "k_gemm_dmma+k_gemm_splitk"
                                                          : "k_gemm_dmma");
   cudaError_t le =

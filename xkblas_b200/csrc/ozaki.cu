@@ -1976,6 +1976,7 @@ extern "C" int xkb_ozaki_counts(unsigned long long* out, int* last, int reset) {
 // moduli cannot carry to FP64 accuracy are computed by the plain FP64
 // kernel instead, launched here and predicated on the device's choice.
 // Single precision (S, C): the exact product or the plain kernel.
+// XKB_ENOMEM, XKB_ERANGE: nothing that writes C was queued.
 // Scratch (stream-ordered, from the pool): residue planes of op(A) and
 // op(B) for the largest count the call may use (nmod x Mpad x Kpad,
 // nmod x Npad x Kpad int8; complex 34 planes), residue planes of C (as many
@@ -2011,7 +2012,7 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   int *mu = nullptr, *nu = nullptr;
   unsigned char* pw = nullptr;  // CallWords, then the norm partials from byte 256
   auto alloc = [&](void** p, size_t n) {
-    return cudaMallocAsync(p, std::max<size_t>(n, 256), st) == cudaSuccess;
+    return scratch_alloc(p, n, st);
   };
   int* list = nullptr;  // the INT8 tiles of a masked product
   const size_t szL = a->uplo == XKB_FULL ? 0 : 4 * (1 + (size_t)(Mpad / BM) * (Npad / BN));
@@ -2019,7 +2020,6 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
             alloc((void**)&R, szR) && alloc((void**)&mu, sizeof(int) * M) &&
             alloc((void**)&nu, sizeof(int) * N) && alloc((void**)&pw, szPart);
   int err = ok ? XKB_OK : XKB_ENOMEM;
-  if (!ok) cudaGetLastError();
   CallWords* w = reinterpret_cast<CallWords*>(pw);
   double4* part = reinterpret_cast<double4*>(pw + 256);
   const OzSel* sel = w ? &w->sel : nullptr;
@@ -2036,6 +2036,11 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   if (!err)
     err = launch_norm(vb, N, K, part + (size_t)nch * std::max(M, N), nu, &w->rmax[1], st);
   if (!err) err = launch_pick(w, pl, !pl.fixed, st, cplx, exact);
+  // The device may have sent the call to the plain FP64 kernel.  Its launch
+  // comes before the recombination's (only one of the two writes C): where it
+  // finds no scratch, nothing that writes C has been queued yet, and
+  // XKB_ENOMEM leaves C as it was.
+  if (!err && (exact || !pl.fixed)) err = gemm_if(a, &w->sel.fallback, st);
   if (!err) err = launch_res(va, M, K, mu, sel, pl.chi, Ap, Arows, Kpad, st);
   if (!err && !same) err = launch_res(vb, N, K, nu, sel, pl.chi, Bp, Npad, Kpad, st);
   if (!err && !cplx && Kpad > (long)rup(K, 64)) {
@@ -2086,8 +2091,6 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
       if (cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
     }
   }
-  // the device may have sent the call to the plain FP64 kernel
-  if (!err && (exact || !pl.fixed)) err = gemm_if(a, &w->sel.fallback, st);
   if (!err && cudaPeekAtLastError() != cudaSuccess) err = XKB_ECUDA;
   trace_mark(slot, 3, st);
   if (list) cudaFreeAsync(list, st);
@@ -2113,8 +2116,8 @@ namespace xkb {
 // The exact form of a large single-precision product (S, C): FP64 work would
 // leave the INT8 tensor cores idle.  Whether the operands allow it is decided
 // on the device (k_oz_pick), else the plain kernel runs within the same call.
-// XKB_ERANGE: not taken for this shape, XKB_ENOMEM: no scratch; the caller
-// then runs the plain kernel.  Taken from M N K = 3.4e9 on (C: a quarter of
+// XKB_ERANGE: not taken for this shape, XKB_ENOMEM: no scratch, either before
+// anything that writes C; the caller then runs the plain kernel.  Taken from M N K = 3.4e9 on (C: a quarter of
 // it).  Measured (B200, us, plain -> exact): S 1024^3 76 -> 108, 1500^3 214 ->
 // 184, 2048^3 527 -> 270, 4096^3 3978 -> 1042 (error against 64 bits 2.53e-8,
 // the final rounding, on both); C 1024^3 258 -> 209, 2048^3 1976 -> 489.
@@ -2185,7 +2188,7 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
   int *mu = nullptr, *nu = nullptr;
   unsigned char* pw = nullptr;  // CallWords, then the norm partials from byte 256
   auto alloc = [&](void** p, size_t n) {
-    return cudaMallocAsync(p, std::max<size_t>(n, 256), st) == cudaSuccess;
+    return scratch_alloc(p, n, st);
   };
   bool ok = alloc((void**)&Ap, (size_t)nmod * Mpad * Kpad) &&
             alloc((void**)&Bp, (size_t)nmod * Wpad * Kpad) &&
@@ -2193,7 +2196,6 @@ extern "C" int xkb_cuda_ozaki_gemm_panels(const xkb_gemm_args* a, int nmod, void
             alloc((void**)&nu, sizeof(int) * a->N) &&
             alloc((void**)&pw, 256 + sizeof(double4) * (size_t)nch * (size_t)std::max<long>(M, wmax));
   int err = ok ? XKB_OK : XKB_ENOMEM;
-  if (!ok) cudaGetLastError();
   CallWords* w = reinterpret_cast<CallWords*>(pw);
   double4* part = reinterpret_cast<double4*>(pw + 256);
   const OzSel* sel = w ? &w->sel : nullptr;
@@ -2330,7 +2332,7 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
   int *mu = nullptr, *nu = nullptr;
   unsigned char* pw = nullptr;  // CallWords, then the norm partials from byte 256
   auto alloc = [&](void** p, size_t n) {
-    return cudaMallocAsync(p, std::max<size_t>(n, 256), st) == cudaSuccess;
+    return scratch_alloc(p, n, st);
   };
   // the largest rectangle: all rows x one panel, or one row block x all columns
   const size_t rsz = std::max((size_t)Mpad * rup((size_t)cmax, BN), rup((size_t)rmax, BM) * (size_t)Npad);
@@ -2339,7 +2341,6 @@ extern "C" int xkb_cuda_ozaki_gemm_blocks(const xkb_gemm_args* a, int nmod, void
             alloc((void**)&mu, sizeof(int) * M) && alloc((void**)&nu, sizeof(int) * N) &&
             alloc((void**)&pw, 256 + sizeof(double4) * (size_t)nch * (size_t)std::max(rmax, cmax));
   int err = ok ? XKB_OK : XKB_ENOMEM;
-  if (!ok) cudaGetLastError();
   CallWords* w = reinterpret_cast<CallWords*>(pw);
   double4* part = reinterpret_cast<double4*>(pw + 256);
   const OzSel* sel = w ? &w->sel : nullptr;

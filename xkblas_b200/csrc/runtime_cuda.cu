@@ -211,6 +211,22 @@ __global__ void k_take_errors(const ErrWords w, int* out) {
 
 void set_library_stream(cudaStream_t s) { g_lib_stream = s; }
 
+// of the calling thread (xkb_cuda_scratch_test)
+static thread_local int t_scratch_requests = 0;
+static thread_local int t_scratch_fail = 0;  // requests until the one that fails; 0: none does
+
+bool scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+  ++t_scratch_requests;
+  if (t_scratch_fail > 0 && --t_scratch_fail == 0) {
+    *p = nullptr;
+    return false;
+  }
+  if (cudaMallocAsync(p, std::max<size_t>(bytes, 256), st) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 // ---- trace ring ---------------------------------------------------------------
 struct TraceSlot {
   xkb_trace_rec rec;
@@ -328,6 +344,13 @@ extern "C" int xkb_cuda_take_device_error(void) {
 }
 
 extern "C" uint64_t xkb_cuda_kernel_count(void) { return xkb::g_launches.load(); }
+
+extern "C" int xkb_cuda_scratch_test(int fail) {
+  const int n = xkb::t_scratch_requests;
+  xkb::t_scratch_requests = 0;
+  xkb::t_scratch_fail = std::max(0, fail);
+  return n;
+}
 
 // ---------------------------------------------------------------------------
 // Tuning table: the choices the autotuner (xkblas_b200/autotune.py) measures

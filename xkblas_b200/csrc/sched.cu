@@ -961,10 +961,9 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
     e->ops.assign(ops, ops + nops);
     e->L = L;
     e->call_tasks = b.call_tasks;
-    if (cudaMallocAsync(&e->d_img, L.bytes, st) != cudaSuccess ||
-        cudaMallocAsync(&e->d_run, L.bytes, st) != cudaSuccess ||
-        cudaMallocAsync(&e->d_times, ((size_t)nops + 1) * 8, st) != cudaSuccess) {
-      cudaGetLastError();
+    if (!scratch_alloc(reinterpret_cast<void**>(&e->d_img), L.bytes, st) ||
+        !scratch_alloc(reinterpret_cast<void**>(&e->d_run), L.bytes, st) ||
+        !scratch_alloc(reinterpret_cast<void**>(&e->d_times), ((size_t)nops + 1) * 8, st)) {
       free_entry(e, st);
       return XKB_ENOMEM;
     }
@@ -990,8 +989,7 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   if (L.bytes > B.d_cap) {
     if (B.d_buf) cudaFreeAsync(B.d_buf, st);
     B.d_cap = L.bytes * 2;
-    if (cudaMallocAsync(&B.d_buf, B.d_cap, st) != cudaSuccess) {
-      B.d_buf = nullptr;
+    if (!scratch_alloc(reinterpret_cast<void**>(&B.d_buf), B.d_cap, st)) {
       B.d_cap = 0;
       return XKB_ENOMEM;
     }
@@ -999,9 +997,8 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   if ((size_t)nops + 1 > B.d_cap_times) {
     if (B.d_times) cudaFreeAsync(B.d_times, st);
     B.d_cap_times = ((size_t)nops + 1) * 2;
-    if (cudaMallocAsync(&B.d_times, B.d_cap_times * sizeof(unsigned long long), st) !=
-        cudaSuccess) {
-      B.d_times = nullptr;
+    if (!scratch_alloc(reinterpret_cast<void**>(&B.d_times),
+                       B.d_cap_times * sizeof(unsigned long long), st)) {
       B.d_cap_times = 0;
       return XKB_ENOMEM;
     }
@@ -1071,10 +1068,7 @@ extern "C" int xkb_cuda_sched_wait_test(int wait_ms, void* stream) {
   const size_t o_urq = 16, o_ndep = 32, o_left = 48, o_times = 64, o_task = 128;
   const size_t bytes = o_task + sizeof(Task);
   uint8_t* d = nullptr;
-  if (cudaMallocAsync(&d, bytes, st) != cudaSuccess) {
-    cudaGetLastError();
-    return XKB_ENOMEM;
-  }
+  if (!scratch_alloc(reinterpret_cast<void**>(&d), bytes, st)) return XKB_ENOMEM;
   uint8_t h[o_task + sizeof(Task)];
   std::memset(h, 0, sizeof h);
   const Ctl ctl{0, 0, 1, 0};  // no bulk work; one queued ticket ...

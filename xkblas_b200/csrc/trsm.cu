@@ -837,11 +837,9 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
     }
     const int nl = (int)table.size() / 3;
     const size_t wbytes = (size_t)slot * ldw * ldw * c.es;
-    if (cudaMallocAsync(&Wbuf, wbytes, st) != cudaSuccess ||
-        cudaMallocAsync(reinterpret_cast<void**>(&dtab), table.size() * sizeof(int), st) !=
-            cudaSuccess ||
-        (npairs > 0 && cudaMallocAsync(&Wtmp, (size_t)kBlk * kBlk * c.es, st) != cudaSuccess)) {
-      cudaGetLastError();
+    if (!scratch_alloc(&Wbuf, wbytes, st) ||
+        !scratch_alloc(reinterpret_cast<void**>(&dtab), table.size() * sizeof(int), st) ||
+        (npairs > 0 && !scratch_alloc(&Wtmp, (size_t)kBlk * kBlk * c.es, st))) {
       release_inv();
       return XKB_ENOMEM;
     }
@@ -926,10 +924,7 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
   auto give_tmp = [&](TrsmCtx& part) {
     if (!inv) return XKB_OK;
     void* t = nullptr;
-    if (cudaMallocAsync(&t, (size_t)c.ldw * part.nrhs * c.es, st) != cudaSuccess) {
-      cudaGetLastError();
-      return XKB_ENOMEM;
-    }
+    if (!scratch_alloc(&t, (size_t)c.ldw * part.nrhs * c.es, st)) return XKB_ENOMEM;
     tmps.push_back(t);
     part.tmp = static_cast<char*>(t);
     return XKB_OK;
@@ -1029,8 +1024,8 @@ extern "C" int xkb_cuda_trmm(int dtype, int side, int uplo, int trans, int diag,
   const long na = side == 0 ? M : N;
   const long ldt = (na + 31) / 32 * 32, ldc = ((long)M + 31) / 32 * 32;
   void *T = nullptr, *Bc = nullptr;
-  if (cudaMallocAsync(&T, (size_t)ldt * na * es, st) != cudaSuccess) return XKB_ENOMEM;
-  if (cudaMallocAsync(&Bc, (size_t)ldc * N * es, st) != cudaSuccess) {
+  if (!scratch_alloc(&T, (size_t)ldt * na * es, st)) return XKB_ENOMEM;
+  if (!scratch_alloc(&Bc, (size_t)ldc * N * es, st)) {
     cudaFreeAsync(T, st);
     return XKB_ENOMEM;
   }
@@ -1090,7 +1085,7 @@ extern "C" int xkb_cuda_symm(int dtype, int herm, int side, int uplo, int M, int
   const long na = side == 0 ? M : N;
   const long ldt = (na + 31) / 32 * 32;
   void* S = nullptr;
-  if (cudaMallocAsync(&S, (size_t)ldt * na * es, st) != cudaSuccess) return XKB_ENOMEM;
+  if (!scratch_alloc(&S, (size_t)ldt * na * es, st)) return XKB_ENOMEM;
   const unsigned nb32 = (unsigned)((na + 31) / 32);
   const dim3 g1(nb32, nb32);
   const int lower = uplo == XKB_LOWER;

@@ -197,6 +197,9 @@ int trsm_entry(int dtype, int side, int uplo, int trans, int diag, int M, int N,
 // xkb_cuda_gemm whose kernel runs only where the device word *run_if is
 // non-zero (gemm_dmma.cu): the plain fallback of a data-chosen Ozaki call.
 int gemm_if(const xkb_gemm_args* a, const int* run_if, cudaStream_t st);
+// Stream-ordered scratch from the pool (runtime_cuda.cu); false, and no CUDA
+// error left pending, where there is none.
+bool scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 // TMA operands: base and leading dimension multiples of 16 bytes.
 bool tma_ok(const void* p, long ld, int es);
 long packed_ld(long rows, int es);
@@ -226,11 +229,7 @@ struct AlignedArray {
     es = es_;
     if (tma_ok(a, lda, es)) return XKB_OK;
     const long l = packed_ld(rows, es);
-    if (cudaMallocAsync(&buf, (size_t)l * cols * es, st) != cudaSuccess) {
-      cudaGetLastError();
-      buf = nullptr;
-      return XKB_OK;
-    }
+    if (!scratch_alloc(&buf, (size_t)l * cols * es, st)) return XKB_OK;
     back = {buf, a, l, lda, rows, cols, uplo};
     const CopyArray in{a, buf, lda, l, rows, cols, uplo};
     p = buf;
@@ -244,7 +243,7 @@ struct AlignedArray {
   }
 };
 // A large single-precision product by exact INT8 arithmetic (ozaki.cu);
-// XKB_ERANGE / XKB_ENOMEM: not taken, nothing was launched.
+// XKB_ERANGE / XKB_ENOMEM: not taken, C is as it was.
 int gemm_exact(const xkb_gemm_args* a, cudaStream_t st);
 double tune(const char* key, double dflt);   // tuning table (runtime_cuda.cu)
 int tune_band(const char* prefix, long K);
