@@ -218,6 +218,21 @@ def test_cuda_abi_rejects_bad_arguments_without_device():
 
 
 
+@pytest.mark.parametrize("dtype", [0, 2])
+@pytest.mark.parametrize("bad", range(3))
+def test_gemm_refuses_misaligned_operands_before_any_work(dtype, bad):
+    """An operand that is not 4-byte aligned, at a size the exact product
+    takes: refused before scratch is asked for."""
+    lib = X.lib()
+    at = [16, 16, 16]
+    at[bad] = 18
+    g = X.GemmArgs(dtype, 0, 0, 2048, 2048, 2048, at[0], 2048, at[1], 2048, at[2], 2048)
+    g.alpha[0] = g.beta[0] = 1.0
+    lib.xkb_cuda_scratch_test(0)
+    assert lib.xkb_cuda_gemm(ctypes.byref(g), None) == -1
+    assert lib.xkb_cuda_scratch_test(0) == 0
+
+
 def test_tuning_table_load_and_lookup(tmp_path):
     """The autotuner's table: a file of "key value" lines is loaded, values
     are read back, and the moduli-count bands drive xkb_ozaki_default_moduli

@@ -187,6 +187,9 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
     return run_if ? XKB_EINVAL
                   : xkb_cuda_scale(a->dtype, a->M, a->N, a->beta, a->C, a->ldc, a->uplo,
                                    a->herm_diag, a->diag, st);
+  if (reinterpret_cast<uintptr_t>(a->A) % 4 || reinterpret_cast<uintptr_t>(a->B) % 4 ||
+      reinterpret_cast<uintptr_t>(a->C) % 4)
+    return XKB_EINVAL;
   if (!run_if && (a->dtype == XKB_S || a->dtype == XKB_C)) {
     const int e = gemm_exact(a, st);
     if (e != XKB_ERANGE && e != XKB_ENOMEM) return e;
@@ -198,9 +201,6 @@ static int gemm_impl(const xkb_gemm_args* a, cudaStream_t st, const int* run_if)
   // other operands are first copied to packed, aligned arrays (C is read and
   // written with plain loads and stores, any alignment)
   const int es = (a->dtype == XKB_S) ? 4 : (a->dtype == XKB_Z ? 16 : 8);
-  if (reinterpret_cast<uintptr_t>(a->A) % 4 || reinterpret_cast<uintptr_t>(a->B) % 4 ||
-      reinterpret_cast<uintptr_t>(a->C) % 4)
-    return XKB_EINVAL;
   xkb_gemm_args pa = *a;
   void* pack = nullptr;  // one allocation and one launch for both operands
   int r = XKB_OK;
