@@ -233,6 +233,20 @@ def test_gemm_refuses_misaligned_operands_before_any_work(dtype, bad):
     assert lib.xkb_cuda_scratch_test(0) == 0
 
 
+def test_trsm_refuses_bad_arguments_before_any_work():
+    """A solve of more than one block on operands that would be copied to
+    aligned arrays first: refused before scratch is asked for."""
+    lib = X.lib()
+    one = (ctypes.c_double * 2)(1.0, 0.0)
+    dp = ctypes.cast(one, ctypes.POINTER(ctypes.c_double))
+    lib.xkb_cuda_scratch_test(0)
+    for trans, alpha in ((5, dp), (-1, dp), (0, None)):
+        for M, N, side in ((600, 70, 0), (70, 600, 1)):
+            assert lib.xkb_cuda_trsm(1, side, 1, trans, 0, M, N, alpha, 24, 601, 24, 601, 0,
+                                     None) == -1
+    assert lib.xkb_cuda_scratch_test(0) == 0
+
+
 def test_tuning_table_load_and_lookup(tmp_path):
     """The autotuner's table: a file of "key value" lines is loaded, values
     are read back, and the moduli-count bands drive xkb_ozaki_default_moduli

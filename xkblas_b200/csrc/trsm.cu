@@ -984,7 +984,9 @@ extern "C" int xkb_cuda_trsm(int dtype, int side, int uplo, int trans, int diag,
                              int ozaki, void* stream) {
   const long n = side == 0 ? M : N;
   cudaStream_t st = resolve_stream(stream);
-  if (dtype < XKB_S || dtype > XKB_Z || M <= 0 || N <= 0 || n <= kBlk || !A || !B)
+  // arguments trsm_entry refuses go there before anything is read
+  if (dtype < XKB_S || dtype > XKB_Z || M <= 0 || N <= 0 || n <= kBlk || !A || !B || !alpha ||
+      trans < XKB_OP_N || trans > XKB_OP_C)
     return trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, A, lda, B, ldb, ozaki, st,
                       true);
   // operands TMA cannot read in place: one aligned copy each instead of one per
