@@ -86,3 +86,24 @@ def test_product(xk, t, M, N, K, pad, tensor_op):
     finally:
         lib.xkb_tune_set(b"gemm_exact_min", 3.4e9)
     assert seen >= 6  # the INT8 form ran
+
+
+@pytest.mark.parametrize("t,M,N,K", [("d", 512, 512, 4096), ("z", 300, 200, 2048),
+                                     ("s", 256, 256, 4096)])
+def test_split_product_runs_unsplit(xk, t, M, N, K):
+    """A plain product on aligned operands needs no scratch: without a
+    workspace for its slices it runs unsplit."""
+    lib = xk.lib()
+    r = np.random.default_rng(6)
+    A, B, C0 = rnd(r, t, M, K), rnd(r, t, K, N), rnd(r, t, M, N)
+    wide = np.complex128 if t in "cz" else np.float64
+    ref = (0.75 * (A.astype(wide) @ B.astype(wide)) + 0.5 * C0).T
+    dA, dB, dC = dev(A, 0), dev(B, 0), dev(C0, 0)
+
+    def call(out):
+        g = xk.GemmArgs(CODE[t], 0, 0, M, N, K, dA.data_ptr(), M, dB.data_ptr(), K,
+                        out.data_ptr(), M)
+        g.alpha[0], g.beta[0] = 0.75, 0.5
+        return lib.xkb_cuda_gemm(ctypes.byref(g), None)
+
+    assert each_refusal(xk, dC, ref, 1e-6 if t == "s" else 1e-14, call) == (1, 0)

@@ -503,7 +503,7 @@ static int launch_dmma(const xkb_gemm_args* a, cudaStream_t st, const int* run_i
   if (p.ksplit > 1 &&
       !scratch_alloc(reinterpret_cast<void**>(&p.ws),
                      (size_t)p.ksplit * ntiles * C_::NREG * C_::THREADS * 8, st))
-    return XKB_ENOMEM;
+    p.ksplit = 1;  // no workspace: every tile walks the whole k range
   const long long tv = evlog_kern_begin(st, p.ksplit > 1 ? "k_gemm_dmma+k_gemm_splitk"
                                                          : "k_gemm_dmma");
   cudaError_t le =
