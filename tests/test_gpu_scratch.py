@@ -107,3 +107,47 @@ def test_split_product_runs_unsplit(xk, t, M, N, K):
         return lib.xkb_cuda_gemm(ctypes.byref(g), None)
 
     assert each_refusal(xk, dC, ref, 1e-6 if t == "s" else 1e-14, call) == (1, 0)
+
+
+@pytest.mark.parametrize("what", ["trsm left", "trsm right", "potrf", "getrf"])
+def test_unaligned_call_gives_up_its_copy(xk, what):
+    """Solves and factorizations on operands that TMA cannot read hold an
+    aligned copy; scratch that is refused while they hold it is asked for
+    again without the copy, working in place."""
+    import torch
+    lib = xk.lib()
+    # 4600: the factorizations' first panels are solved by more than one block
+    n, m = (700 if what.startswith("trsm") else 4600), 200
+    r = np.random.default_rng(8)
+    A = rnd(r, "d", n, n)
+    A = np.asfortranarray(0.5 * (A + A.T) + n * np.eye(n))
+    dA = dev(A, 1)
+    al = (ctypes.c_double * 2)(2.0, 0.0)
+    dp = ctypes.cast(al, ctypes.POINTER(ctypes.c_double))
+    if what.startswith("trsm"):
+        left = what == "trsm left"
+        B = rnd(r, "d", *((n, m) if left else (m, n)))
+        L = np.tril(A)
+        X = 2.0 * (np.linalg.solve(L, B) if left else np.linalg.solve(L.T, B.T).T)
+        out0 = dev(B, 1)
+
+        def call(out):
+            return lib.xkb_cuda_trsm(1, 0 if left else 1, 1, 0, 0, B.shape[0], B.shape[1], dp,
+                                     dA.data_ptr(), n + 1, out.data_ptr(), B.shape[0] + 1, 0,
+                                     None)
+    else:
+        out0 = dA
+        if what == "potrf":
+            X = np.tril(np.linalg.cholesky(A)) + np.triu(A, 1)
+        else:
+            X = torch.linalg.lu_factor(torch.from_numpy(A).cuda(), pivot=False)[0].cpu().numpy()
+        info = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+        def call(out):
+            if what == "potrf":
+                return lib.xkb_cuda_potrf(1, 1, n, out.data_ptr(), n + 1, info.data_ptr(), 0, None)
+            return lib.xkb_cuda_getrf_nopiv(1, n, out.data_ptr(), n + 1, info.data_ptr(), 0, None)
+    ref = np.zeros((X.shape[1], X.shape[0] + 1))
+    ref[:, :X.shape[0]] = X.T
+    seen, refused = each_refusal(xk, out0, ref, 1e-12, call)
+    assert seen >= 2 and refused == 0

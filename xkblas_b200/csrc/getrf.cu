@@ -576,21 +576,21 @@ extern "C" int xkb_cuda_getrf_nopiv(int dtype, int N, void* A, long lda, int* d_
   // a matrix TMA cannot read in place is factored in an aligned copy
   AlignedArray w;
   int e = XKB_OK;
-  if (N > nmax && (e = w.take(A, lda, N, N, XKB_FULL, c.es, c.st))) return e;
-  if (w.buf) {
-    c.A = static_cast<char*>(w.p);
-    c.lda = w.ld;
-  }
-  auto done = [&](int r) {
-    if (!r) r = w.put_back(c.st);
-    w.release(c.st);
-    return r;
+  auto run = [&](void* M, long ldm) {
+    c.A = static_cast<char*>(M);
+    c.lda = ldm;
+    if (N > 2 * nmax && (mode == 2 || (mode == 1 && c.ozaki == 0)))
+      return factor_blocked(c, 0, N, nb);
+    if (mode == 3) {  // in plain mode too: DMMA couplings (8192: 18.3 against 18.9 ms)
+      c.blk_leaf = std::max(2 * nmax + 1, (long)tune("getrf_oz_leaf", 4096.0));
+      c.blk_nb = std::max(nmax, ((long)tune("getrf_nb", 512.0) + 63) / 64 * 64);
+    }
+    return factor(c, 0, N);
   };
-  if (N > 2 * nmax && (mode == 2 || (mode == 1 && c.ozaki == 0)))
-    return done(factor_blocked(c, 0, N, nb));
-  if (mode == 3) {  // in plain mode too: DMMA couplings (8192: 18.3 against 18.9 ms)
-    c.blk_leaf = std::max(2 * nmax + 1, (long)tune("getrf_oz_leaf", 4096.0));
-    c.blk_nb = std::max(nmax, ((long)tune("getrf_nb", 512.0) + 63) / 64 * 64);
-  }
-  return done(factor(c, 0, N));
+  if (N > nmax) e = w.take(A, lda, N, N, XKB_FULL, c.es, c.st);
+  if (!e) e = w.buf ? run(w.p, w.ld) : run(A, lda);
+  const bool again = e == XKB_ENOMEM && w.buf;
+  if (!e) e = w.put_back(c.st);
+  w.release(c.st);
+  return again ? run(A, lda) : e;
 }

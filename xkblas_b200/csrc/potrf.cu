@@ -645,21 +645,21 @@ extern "C" int xkb_cuda_potrf(int dtype, int uplo, int N, void* A, long lda, int
   // in and out instead of one per operand of every product
   AlignedArray w;
   int e = XKB_OK;
-  if (N > nmax && (e = w.take(A, lda, N, N, uplo, c.es, c.st))) return e;
-  if (w.buf) {
-    c.A = static_cast<char*>(w.p);
-    c.lda = w.ld;
-  }
-  if (N > 2 * nmax && (mode == 2 || ((mode == 1 || mode == 3) && c.ozaki == 0))) {
-    e = factor_blocked(c, 0, N, nb);
-  } else {
+  auto run = [&](void* M, long ldm) {
+    c.A = static_cast<char*>(M);
+    c.lda = ldm;
+    if (N > 2 * nmax && (mode == 2 || ((mode == 1 || mode == 3) && c.ozaki == 0)))
+      return factor_blocked(c, 0, N, nb);
     if (mode == 3 && c.ozaki > 0) {
       c.blk_leaf = std::max(2 * nmax + 1, (long)tune("potrf_oz_leaf", 4096.0));
       c.blk_nb = nb;
     }
-    e = factor(c, 0, N, true, false);
-  }
+    return factor(c, 0, N, true, false);
+  };
+  if (N > nmax) e = w.take(A, lda, N, N, uplo, c.es, c.st);
+  if (!e) e = w.buf ? run(w.p, w.ld) : run(A, lda);
+  const bool again = e == XKB_ENOMEM && w.buf;
   if (!e) e = w.put_back(c.st);
   w.release(c.st);
-  return e;
+  return again ? run(A, lda) : e;
 }

@@ -998,10 +998,15 @@ extern "C" int xkb_cuda_trsm(int dtype, int side, int uplo, int trans, int diag,
   if (!e)
     e = trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, wa.p, wa.ld, wb.p, wb.ld, ozaki,
                    st, true);
+  // again in place: B is as it was if the solve worked on its copy, and also if
+  // it worked on an aligned B (its scratch is found before it writes B)
+  const bool again = e == XKB_ENOMEM && (wb.buf || (wa.buf && tma_ok(B, ldb, es) && ozaki <= 0));
   if (!e) e = wb.put_back(st);
   wa.release(st);
   wb.release(st);
-  return e;
+  return again ? trsm_entry(dtype, side, uplo, trans, diag, M, N, alpha, A, lda, B, ldb, ozaki, st,
+                            true)
+               : e;
 }
 
 // The product on the materialised operand: Ozaki INT8 form when ozaki > 0,

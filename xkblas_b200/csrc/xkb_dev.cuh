@@ -215,8 +215,10 @@ int copy_arrays(const CopyArray* d, int n, int es, cudaStream_t st, const int* r
 // An array some of whose solves / factorization's products go through TMA, as
 // an aligned copy when its base or leading dimension is not: p, ld give the
 // array to work on; put_back() copies the uplo part of the result into the
-// array (out only) and release() frees the copy.  Without memory for a copy
-// the products repack their operands one by one instead.
+// array (out only) and release() frees the copy.  Without memory for a copy,
+// or where other scratch is refused while it is held (the array is untouched
+// until put_back), the call works in place and the products repack their
+// operands one by one instead.
 struct AlignedArray {
   void* p = nullptr;
   long ld = 0;
