@@ -151,3 +151,31 @@ def test_unaligned_call_gives_up_its_copy(xk, what):
     ref[:, :X.shape[0]] = X.T
     seen, refused = each_refusal(xk, out0, ref, 1e-12, call)
     assert seen >= 2 and refused == 0
+
+
+def test_fixed_moduli_reserve_their_planes_only():
+    """A complex tensor-op product of a fixed count takes scratch for that
+    count's residue planes (8: about half of what 16 take)."""
+    code = """
+import ctypes, torch, xkblas_b200 as X
+X.init(); lib = X.lib()
+n = 1536
+A = torch.zeros(n, n, dtype=torch.complex128, device="cuda"); C = torch.zeros_like(A)
+free = []
+for nmod in (0, 8, 16):
+    torch.cuda.synchronize()
+    if nmod:
+        g = X.GemmArgs(3, 0, 0, n, n, n, A.data_ptr(), n, A.data_ptr(), n, C.data_ptr(), n)
+        g.alpha[0] = 1.0
+        assert lib.xkb_cuda_ozaki_gemm(ctypes.byref(g), nmod, None) == 0
+        X.sync()
+    free.append(torch.cuda.mem_get_info()[0])
+print(free[0] - free[1], free[0] - free[2])
+"""
+    import subprocess
+    import sys
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    few, many = map(int, out.stdout.split()[-2:])
+    # 18 planes against 34, in the pool's 32 MiB steps
+    assert few <= 0.7 * many, (few, many)

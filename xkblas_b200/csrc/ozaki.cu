@@ -1979,8 +1979,9 @@ extern "C" int xkb_ozaki_counts(unsigned long long* out, int* last, int reset) {
 // XKB_ENOMEM, XKB_ERANGE: nothing that writes C was queued.
 // Scratch (stream-ordered, from the pool): residue planes of op(A) and
 // op(B) for the largest count the call may use (nmod x Mpad x Kpad,
-// nmod x Npad x Kpad int8; complex 34 planes), residue planes of C (as many
-// Mpad x Npad uint8), row codes, norm partials and the call's device words.
+// nmod x Npad x Kpad int8; complex two planes per modulus, 34 for 16), residue
+// planes of C (as many Mpad x Npad uint8), row codes, norm partials and the
+// call's device words.
 static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   const bool cplx = a->dtype == XKB_Z || a->dtype == XKB_C;
   const bool exact = a->dtype == XKB_S || a->dtype == XKB_C;
@@ -1988,8 +1989,8 @@ static int oz_run(const xkb_gemm_args* a, int nmod, cudaStream_t st) {
   if (Keff > 131072) return XKB_ERANGE;
   ModPlan pl;
   if (!plan_moduli(exact ? kExactHi : nmod, Keff, &pl)) return XKB_ERANGE;
-  // planes
-  const int nmax = exact ? (cplx ? 2 * kExactHiC : kExactHi) : (cplx ? kMaxPl : pl.hi);
+  // planes: of the largest count the call may use
+  const int nmax = cplx ? 2 * (exact ? kExactHiC : cplx_count(pl.chi->H)) : pl.hi;
   const Consts* c = cplx ? nullptr : pl.chi;
   const int M = a->M, N = a->N, K = a->K;
   const long Kpad = (long)rup(K, BKB);
