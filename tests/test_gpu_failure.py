@@ -73,3 +73,38 @@ def test_wait_test_rejects_bad_limits(xk):
     lib = xk.lib()
     assert lib.xkb_cuda_sched_wait_test(0, None) == -1
     assert lib.xkb_cuda_sched_wait_test(20000, None) == -1
+
+
+def test_error_word_survives_a_pending_cuda_error(xk):
+    """An older CUDA error that is still pending on the thread (a device
+    synchronisation refused while a stream is being captured) does not make
+    the read of the error words drop what it has cleared."""
+    import ctypes
+    import torch
+    lib, cu = xk.lib(), ctypes.CDLL("libcuda.so.1")
+    xk.sync()
+    st = torch.cuda.Stream()
+    h, graph = ctypes.c_void_p(st.cuda_stream), ctypes.c_void_p()
+    counts = (ctypes.c_ulonglong * 3)()
+    assert cu.cuStreamBeginCapture_v2(h, 0) == 0
+    assert lib.xkb_ozaki_counts(counts, None, 0) == -2  # leaves its error pending
+    cu.cuStreamEndCapture(h, ctypes.byref(graph))
+    if graph:
+        cu.cuGraphDestroy(graph)
+    lib.xkb_cuda_sched_wait_test(20, None)
+    torch.cuda.synchronize()
+    first, second = lib.xkb_cuda_take_device_error(), lib.xkb_cuda_take_device_error()
+    page = np.zeros(8)
+    lib.xkblas_unregister_memory(ctypes.c_void_p(page.ctypes.data), ctypes.c_size_t(64))  # clears it
+    assert (first, second) == (XKB_DEV_FULL_WAIT, 0)
+
+
+def test_error_words_are_read_after_the_default_stream(xk):
+    """The read of the error words waits for work queued on the legacy
+    default stream, as the blocking copies it replaced did."""
+    import ctypes
+    lib = xk.lib()
+    xk.sync()
+    legacy = ctypes.c_void_p(1)  # cudaStreamLegacy
+    lib.xkb_cuda_sched_wait_test(300, legacy)
+    assert lib.xkb_cuda_take_device_error() == XKB_DEV_FULL_WAIT

@@ -2501,34 +2501,6 @@ __global__ void k_oz_beta(int M, int N, double beta, double* C, long ldc, int up
   }
 }
 
-typedef CUresult (*PFN_ctxGetCurrent)(CUcontext*);
-typedef CUresult (*PFN_ctxGetId)(CUcontext, unsigned long long*);
-
-// Unique ID of the calling thread's current CUDA context (0 if unknown or
-// none is current).
-static unsigned long long current_ctx_id() {
-  static PFN_ctxGetCurrent get_cur = nullptr;
-  static PFN_ctxGetId get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_cur = reinterpret_cast<PFN_ctxGetCurrent>(p);
-    p = nullptr;
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<PFN_ctxGetId>(p);
-    cudaGetLastError();
-  });
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (!get_cur || !get_id || get_cur(&ctx) != CUDA_SUCCESS || !ctx) return 0;
-  if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-  return id;
-}
-
 // Kernels the scratch-free path launches, loaded up front (with lazy loading
 // a kernel's code is otherwise placed in device memory at its first launch).
 template <int NM>
@@ -2565,7 +2537,7 @@ static int noalloc_base(unsigned char** out) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return XKB_ECUDA;
   std::lock_guard<std::mutex> g(mu);
-  const unsigned long long id = current_ctx_id();
+  const unsigned long long id = context_id();
   if (!ptr[dev] || id == 0 || id != ctx_of[dev]) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_oz_noalloc_scratch) != cudaSuccess || !p ||
@@ -2575,7 +2547,7 @@ static int noalloc_base(unsigned char** out) {
       return XKB_ECUDA;
     }
     ptr[dev] = static_cast<unsigned char*>(p);
-    ctx_of[dev] = current_ctx_id();  // the lookup made the primary context current
+    ctx_of[dev] = context_id();  // the lookup made the primary context current
   }
   *out = ptr[dev];
   return XKB_OK;

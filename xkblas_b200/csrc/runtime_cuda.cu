@@ -184,6 +184,34 @@ int sm_count() {
   return n;
 }
 
+typedef CUresult (*PFN_ctxGetCurrent)(CUcontext*);
+typedef CUresult (*PFN_ctxGetId)(CUcontext, unsigned long long*);
+
+// Unique ID of the calling thread's current CUDA context (0 if unknown or
+// none is current).
+unsigned long long context_id() {
+  static PFN_ctxGetCurrent get_cur = nullptr;
+  static PFN_ctxGetId get_id = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_cur = reinterpret_cast<PFN_ctxGetCurrent>(p);
+    p = nullptr;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<PFN_ctxGetId>(p);
+    cudaGetLastError();
+  });
+  CUcontext ctx = nullptr;
+  unsigned long long id = 0;
+  if (!get_cur || !get_id || get_cur(&ctx) != CUDA_SUCCESS || !ctx) return 0;
+  if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
+  return id;
+}
+
 static std::vector<ErrAddr>& error_addrs() {
   static std::vector<ErrAddr> r;
   return r;
@@ -195,7 +223,7 @@ int register_error_addr(ErrAddr f) {
 
 // First error word that is set, in registration order; clears all.  One launch
 // and one wait for all units: read one by one, a blocking copy per unit made
-// up to 80 us of every xkblas_sync.
+// up to 80 us of every xkblas_sync (now 12).
 constexpr int kMaxUnits = 32;
 struct ErrWords {
   int* p[kMaxUnits];
@@ -312,8 +340,8 @@ namespace xkb {
 extern "C" int xkb_cuda_take_device_error(void) {
   using namespace xkb;
   static std::mutex mu;
-  static int* host[64] = {nullptr};  // pinned result word and stream per device
-  static cudaStream_t stream[64] = {nullptr};
+  static int* word[64] = {nullptr};  // pinned result word per device, of the context below
+  static unsigned long long ctx_of[64] = {0};
   std::lock_guard<std::mutex> g(mu);
   ErrWords w;
   w.n = 0;
@@ -321,26 +349,30 @@ extern "C" int xkb_cuda_take_device_error(void) {
     if (void* p = f())
       if (w.n < kMaxUnits) w.p[w.n++] = static_cast<int*>(p);
   int dev = 0;
-  if (w.n == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    cudaGetLastError();
-    return 0;
-  }
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if (!host[dev] &&
-        (cudaHostAlloc(reinterpret_cast<void**>(&host[dev]), sizeof(int), cudaHostAllocMapped) !=
-             cudaSuccess ||
-         cudaStreamCreateWithFlags(&stream[dev], cudaStreamNonBlocking) != cudaSuccess)) {
-      host[dev] = nullptr;
+  if (w.n == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  const unsigned long long id = context_id();
+  if (!word[dev] || id == 0 || id != ctx_of[dev]) {  // a reset context took its word along
+    word[dev] = nullptr;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&word[dev]), sizeof(int), cudaHostAllocMapped) !=
+        cudaSuccess) {
       cudaGetLastError();
+      word[dev] = nullptr;
       return 0;
     }
-    k_take_errors<<<1, 32, 0, stream[dev]>>>(w, host[dev]);
-    if (cudaPeekAtLastError() == cudaSuccess && cudaStreamSynchronize(stream[dev]) == cudaSuccess)
-      return *static_cast<volatile int*>(host[dev]);
-    cudaGetLastError();
-    host[dev] = nullptr;  // gone with a reset context: make them again
+    ctx_of[dev] = id;
   }
-  return 0;
+  volatile int* v = word[dev];
+  *v = 0;
+  // On the legacy default stream: after whatever the blocking streams hold.
+  // Only the launch's own status counts, not an older error that may be
+  // pending on the thread: once it is accepted the words are cleared, and its
+  // result is the only copy.
+  void* args[] = {&w, &word[dev]};
+  if (cudaLaunchKernel(reinterpret_cast<const void*>(k_take_errors), dim3(1), dim3(32), args, 0,
+                       nullptr) != cudaSuccess)
+    return 0;
+  cudaStreamSynchronize(nullptr);
+  return *v;
 }
 
 extern "C" uint64_t xkb_cuda_kernel_count(void) { return xkb::g_launches.load(); }

@@ -146,6 +146,9 @@ static void* unit_error_addr() {
   return cudaGetSymbolAddress(&p, g_dev_error) == cudaSuccess ? p : nullptr;
 }
 static int g_unit_error_registered = register_error_addr(&unit_error_addr);
+// Unique ID of the calling thread's current CUDA context (0: unknown, or none
+// is current); it changes with cudaDeviceReset (runtime_cuda.cu).
+unsigned long long context_id();
 // Encode a 2-D tiled tensor map: rows x cols column-major with leading
 // dimension ld (elements of `elem_bytes`), box bx (along rows) x by.
 // Returns false if the driver entry point is missing or encoding fails.
