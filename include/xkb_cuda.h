@@ -216,7 +216,9 @@ int xkb_cuda_scratch_test(int fail);
  * dtype XKB_D or XKB_Z; any leading dimension >= the row count, 8-byte
  * aligned bases (operands not 16-byte aligned are staged with 8-byte
  * copies).  Calls of one batch must not write memory another call of the
- * batch reads or writes. */
+ * batch reads or writes.  Batches may be queued on any streams; on a stream
+ * that is being captured only one that is already kept as a graph (queued
+ * twice before), XKB_ECUDA otherwise. */
 #define XKB_BATCH_GEMM 0
 #define XKB_BATCH_TRSM 1
 typedef struct xkb_batch_op {

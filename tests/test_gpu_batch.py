@@ -206,3 +206,58 @@ def test_repeated_batch_replays_a_graph(xk):
     assert all(v > 0 for v in lat)
     assert lib.xkb_cuda_batch_release() == 0
     assert lib.xkb_cuda_batch_cached() == 0
+
+
+def test_different_batches_on_two_streams(xk):
+    """Batches that differ, queued alternately on two streams without a wait
+    between them: the task lists share one staging and one device image, which
+    a later batch must not take from an earlier one that still reads it.  The
+    lists grow, so that the images are replaced as well, and more lists repeat
+    than the cache keeps, so that entries are given up in use."""
+    import torch
+    lib = xk.lib()
+    assert lib.xkb_cuda_batch_release() == 0
+    st = [torch.cuda.Stream(), torch.cuda.Stream()]
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def rnd(r, c):
+        return torch.rand(r, c, generator=g, device="cuda", dtype=torch.float64) - 0.5
+
+    A, B = rnd(300, 400), rnd(200, 300)  # column major: 400 x 300, 300 x 200
+    L = torch.tril(rnd(260, 260)) + 260 * torch.eye(260, device="cuda", dtype=torch.float64)
+    Lt, X0 = L.t().contiguous(), rnd(180, 260)
+    gemm = (A.t() @ B.t()).t()
+    solve = torch.linalg.solve_triangular(L, X0.t(), upper=False).t()
+    runs = []
+    for i in range(24):
+        ops, outs = [], []
+        for j in range(2 + i):
+            al = 1.0 + i + j / 64.0
+            o = X.BatchOp()
+            if j % 3:
+                C = torch.zeros(200, 400, device="cuda", dtype=torch.float64)
+                o.kind, o.dtype, o.M, o.N, o.K = 0, 1, 400, 200, 300
+                o.A, o.lda, o.B, o.ldb, o.C, o.ldc = (A.data_ptr(), 400, B.data_ptr(), 300,
+                                                      C.data_ptr(), 400)
+                outs.append((C, al * gemm))
+            else:
+                C = X0.clone()
+                o.kind, o.dtype, o.uplo, o.M, o.N = 1, 1, LO, 260, 180
+                o.A, o.lda, o.C, o.ldc = Lt.data_ptr(), 260, C.data_ptr(), 260
+                outs.append((C, al * solve))
+            o.alpha[0] = al
+            ops.append(o)
+        runs.append(((X.BatchOp * len(ops))(*ops), len(ops), outs))
+    for rep in range(3):  # the first uncached, then cached, then replayed where still cached
+        for i, (arr, n, outs) in enumerate(runs):
+            for k, (C, _) in enumerate(outs):
+                C.copy_(torch.zeros_like(C) if k % 3 else X0)
+        torch.cuda.synchronize()
+        for i, (arr, n, _) in enumerate(runs):
+            assert lib.xkb_cuda_batch(arr, n, 0, ctypes.c_void_p(st[i % 2].cuda_stream)) == 0
+        torch.cuda.synchronize()
+        assert lib.xkb_cuda_take_device_error() == 0
+        for i, (_, _, outs) in enumerate(runs):
+            for k, (C, ref) in enumerate(outs):
+                assert ((C - ref).norm() / ref.norm()).item() < 1e-13, (rep, i, k)
+    assert lib.xkb_cuda_batch_release() == 0

@@ -637,6 +637,7 @@ struct GraphEntry {
   cudaGraphExec_t exec = nullptr;
   std::vector<int> call_tasks;
   uint64_t last_use = 0;
+  cudaEvent_t done = nullptr;     // its last launch, on whatever stream
   size_t bytes() const { return 2 * L.bytes + ((size_t)L.nops + 1) * 8; }
 };
 
@@ -647,6 +648,9 @@ struct Batch {
   size_t d_cap = 0;
   unsigned long long* d_times = nullptr;  // call_end[ncalls], t_start
   size_t d_cap_times = 0;
+  // the staging and device images are shared by the calls of all streams: the
+  // last upload out of h_stage, and the last launch that reads d_buf / d_times
+  cudaEvent_t staged = nullptr, done = nullptr;
   // the last launch (read by xkb_cuda_batch_latency)
   int ncalls = 0;
   std::vector<int> call_tasks;
@@ -661,7 +665,23 @@ struct Batch {
 constexpr size_t kGraphMaxEntries = 8;
 constexpr size_t kGraphMaxBytes = size_t(2) << 30;
 
+static bool make_event(cudaEvent_t* e) {
+  if (*e || cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess) return true;
+  cudaGetLastError();
+  *e = nullptr;
+  return false;
+}
+
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
 static void free_entry(GraphEntry* e, cudaStream_t st) {
+  if (e->done) {
+    cudaEventSynchronize(e->done);  // it may be running on another stream
+    cudaEventDestroy(e->done);
+  }
   if (e->exec) cudaGraphExecDestroy(e->exec);
   if (e->graph) cudaGraphDestroy(e->graph);
   if (e->d_img) cudaFreeAsync(e->d_img, st);
@@ -798,6 +818,7 @@ static int launch_entry(Batch& B, GraphEntry* e, cudaStream_t st) {
   evlog_kern_end(tv, st);
   if (le != cudaSuccess) return XKB_ECUDA;
   trace_calls(tv, st, e->d_times, e->ops.data(), e->L.nops);
+  if (!capturing(st) && cudaEventRecord(e->done, st) != cudaSuccess) return XKB_ECUDA;
   count_launch();
   return XKB_OK;
 }
@@ -920,8 +941,10 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   L.set(ntasks, succ.size(), b.bulk.size(), (size_t)b.nurg, nops);
   for (int c = 0; c < nops; ++c)
     L.ztrsm = L.ztrsm || (ops[c].kind == XKB_BATCH_TRSM && ops[c].dtype == XKB_Z);
-  // the previous batch may still read the pinned staging buffer
-  if (B.h_stage) cudaStreamSynchronize(st);
+  // the shared images cannot belong to a captured graph
+  if (capturing(st) || !make_event(&B.staged) || !make_event(&B.done)) return XKB_ECUDA;
+  // the previous batch's upload may still read the pinned staging buffer
+  if (cudaEventSynchronize(B.staged) != cudaSuccess) return XKB_ECUDA;
   if (L.bytes > B.h_cap) {
     if (B.h_stage) cudaFreeHost(B.h_stage);
     B.h_cap = L.bytes * 2;
@@ -968,7 +991,8 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
       return XKB_ENOMEM;
     }
     cudaMemcpyAsync(e->d_img, h, L.bytes, cudaMemcpyHostToDevice, st);
-    if (int r = build_graph(e)) {
+    cudaEventRecord(B.staged, st);
+    if (int r = make_event(&e->done) ? build_graph(e) : XKB_ECUDA) {
       free_entry(e, st);
       return r;
     }
@@ -986,6 +1010,9 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
     return launch_entry(B, e, st);
   }
 
+  // the previous launch, perhaps on another stream, reads what is freed or
+  // overwritten below
+  if (cudaStreamWaitEvent(st, B.done, 0) != cudaSuccess) return XKB_ECUDA;
   if (L.bytes > B.d_cap) {
     if (B.d_buf) cudaFreeAsync(B.d_buf, st);
     B.d_cap = L.bytes * 2;
@@ -1005,6 +1032,7 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
   }
   uint8_t* d = B.d_buf;
   cudaMemcpyAsync(d, h, L.bytes, cudaMemcpyHostToDevice, st);
+  cudaEventRecord(B.staged, st);
   cudaMemsetAsync(B.d_times, 0, (size_t)nops * sizeof(unsigned long long), st);
   cudaMemsetAsync(B.d_times + nops, 0xff, sizeof(unsigned long long), st);
   B.cur_times = B.d_times;
@@ -1015,9 +1043,8 @@ extern "C" int xkb_cuda_batch(const xkb_batch_op* ops, int nops, int schedule, v
       a.call_end, a.t_start, a.wait_ns);
   evlog_kern_end(tv, st);
   trace_calls(tv, st, B.d_times, ops, nops);
+  cudaEventRecord(B.done, st);
   count_launch();
-  // the pinned staging buffer must outlive the copy: the copy is ordered
-  // before the kernel, and the next batch synchronises before reusing it
   return cudaPeekAtLastError() == cudaSuccess ? XKB_OK : XKB_ECUDA;
 }
 
