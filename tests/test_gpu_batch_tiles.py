@@ -94,3 +94,48 @@ def test_batch_tile_edges(xk, cplx, pad, off):
             T, B = ref, bound
             lim = 8 * (shape[0] + 4) * EPS * (np.abs(T) @ np.abs(X) + 2 * np.abs(B))
             assert (np.abs(T @ X - 2 * B) <= lim).all(), shape
+
+
+def solve_batch(xk, T, B, uplo, tr, unit):
+    """op(T) X = B by one batch of one call."""
+    import torch
+    M, N = B.shape
+    cplx = np.iscomplexobj(B)
+    dT, dB = dev(T, 0, 0), dev(B, 0, 0)
+    o = xk.BatchOp()
+    o.kind, o.dtype, o.uplo, o.trans, o.diag, o.M, o.N = 1, 3 if cplx else 1, uplo, tr, unit, M, N
+    o.A, o.lda, o.C, o.ldc = dT.data_ptr(), M, dB.data_ptr(), M
+    o.alpha[0] = 1.0
+    torch.cuda.synchronize()
+    assert xk.lib().xkb_cuda_batch(ctypes.byref(o), 1, 0, None) == 0
+    xk.sync()
+    assert xk.lib().xkb_cuda_take_device_error() == 0
+    return host(dB, B.shape, 0, 0)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("uplo,tr,unit", [(1, 0, 0), (2, 0, 0), (1, 1, 1), (2, 1, 0)])
+def test_nonfinite_right_hand_sides(xk, cplx, uplo, tr, unit):
+    """Inf and NaN in a right-hand side reach the unknowns that depend on
+    them and no others: those solved earlier, and the other columns, are what
+    they are without them."""
+    r = np.random.default_rng(4)
+    for M in (5, 20, 64, 75):
+        A = rnd(r, M, M, cplx) / M + np.eye(M)
+        B = rnd(r, M, 19, cplx)
+        clean = solve_batch(xk, A, B, uplo, tr, unit)
+        bad = B.copy()
+        at = {1: (3, np.nan), 4: (M - 2, np.inf), 17: (M // 2, -np.inf), 18: (0, np.nan)}
+        for c, (i, v) in at.items():
+            bad[i, c] = v
+        X = solve_batch(xk, A, bad, uplo, tr, unit)
+        fwd = (uplo == 1) == (tr == 0)
+        for c in range(19):
+            i = at[c][0] if c in at else None
+            # unknowns solved before unknown i
+            free = slice(0, M) if i is None else (slice(0, i) if fwd else slice(i + 1, M))
+            assert np.allclose(X[free, c], clean[free, c], rtol=0, atol=1e-13), (M, c)
+            if i is not None:
+                assert not np.isfinite(X[i, c]), (M, c)
+                dep = X[i:, c] if fwd else X[:i + 1, c]
+                assert not np.isfinite(dep).any(), (M, c)

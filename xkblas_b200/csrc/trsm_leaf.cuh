@@ -44,6 +44,43 @@ __device__ __forceinline__ size_t leaf_at(int i, int c, long ldb, bool rhs_rows)
   return rhs_rows ? (size_t)c + (size_t)i * (size_t)ldb : (size_t)i + (size_t)c * (size_t)ldb;
 }
 
+// Unknowns b .. b + 7 of a warp's right-hand sides by substitution, a lane per
+// right-hand side (Vr, Vi: the sub-block's inverse, whose diagonal is the
+// reciprocals): an unknown that is Inf or NaN reaches those after it only,
+// where a product with the inverse takes it to all eight through its zeros.
+template <class T, bool LOWER>
+__device__ __noinline__ void leaf_substitute(const double* Tr, const double* Ti, const double* Vr,
+                                             const double* Vi, int b, double* xr, double* xi) {
+  using Sh = LeafShape<T>;
+  constexpr bool CP = Sh::CP;
+  const int lane = threadIdx.x & 31;
+  if (lane < Sh::CW) {
+    double* x = xr + lane * Sh::LD + b;
+    double* z = xi + lane * Sh::LD + b;
+    for (int q = 0; q < 8; ++q) {
+      const int j = LOWER ? q : 7 - q;
+      const double dr = Vr[9 * j], di = CP ? Vi[9 * j] : 0.0;
+      double vr = x[j], vi = 0.0;
+      if (CP) {
+        const double wr = vr * dr - z[j] * di;
+        vi = vr * di + z[j] * dr;
+        vr = wr;
+        z[j] = vi;
+      } else {
+        vr *= dr;
+      }
+      x[j] = vr;
+      const double* tr = Tr + (b + j) * Sh::LD + b;
+      const double* ti = Ti + (b + j) * Sh::LD + b;
+      for (int i = LOWER ? j + 1 : 0; i < (LOWER ? 8 : j); ++i) {
+        x[i] -= CP ? tr[i] * vr - ti[i] * vi : tr[i] * vr;
+        if (CP) z[i] -= tr[i] * vi + ti[i] * vr;
+      }
+    }
+  }
+  __syncwarp();
+}
+
 // X = (ar, ai) op(T)^-1 B in place for B's nrhs columns (ldb), by 128 threads:
 // T(i,j) = A[swap ? j + i lda : i + j lda], conjugated when conj, unit: ones
 // on its diagonal.  Operands are read through L2.
@@ -191,13 +228,27 @@ __device__ __forceinline__ void leaf_solve(const typename St<T>::S* A, long lda,
           dmma_k8(yr, a_r, b_r);
         }
       }
-      __syncwarp();  // every lane has read X_s
+      // every lane has read X_s (the vote); a value that is not finite shows
+      // in this Y (the inverse's diagonal is not zero)
+      bool fin = true;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int c = g + ((v >> 1) << 3);
-        if (c < Sh::CW) {
-          xr[c * LD + b + k0 + (v & 1)] = yr[v];
-          if (CP) xi[c * LD + b + k0 + (v & 1)] = yi[v];
+      for (int v = 0; v < 4; ++v) fin = fin && isfinite(yr[v]) && (!CP || isfinite(yi[v]));
+      if (__all_sync(0xffffffffu, fin)) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int c = g + ((v >> 1) << 3);
+          if (c < Sh::CW) {
+            xr[c * LD + b + k0 + (v & 1)] = yr[v];
+            if (CP) xi[c * LD + b + k0 + (v & 1)] = yi[v];
+          }
+        }
+      } else {
+        leaf_substitute<T, LOWER>(Tr, Ti, Vr + m * 64, Vi + m * 64, b, xr, xi);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int c = g + ((v >> 1) << 3);
+          yr[v] = c < Sh::CW ? xr[c * LD + b + k0 + (v & 1)] : 0.0;
+          if (CP) yi[v] = c < Sh::CW ? xi[c * LD + b + k0 + (v & 1)] : 0.0;
         }
       }
       // rows still to solve -= T(rows, b .. b+7) Y
