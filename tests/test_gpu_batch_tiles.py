@@ -139,3 +139,23 @@ def test_nonfinite_right_hand_sides(xk, cplx, uplo, tr, unit):
                 assert not np.isfinite(X[i, c]), (M, c)
                 dep = X[i:, c] if fwd else X[:i + 1, c]
                 assert not np.isfinite(dep).any(), (M, c)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("uplo,tr", [(1, 0), (2, 0), (1, 1)])
+def test_ill_conditioned_diagonal_blocks(xk, cplx, uplo, tr):
+    """Triangles whose diagonal blocks are far from well conditioned: the
+    solve is as backward stable as substitution, componentwise
+    |op(T) X - B| <= (M + 8) eps (|op(T)| |X| + |B|), complex four times that."""
+    wide = np.clongdouble if cplx else np.longdouble
+    for seed, M in enumerate((8, 40, 64, 64, 64, 130)):
+        r = np.random.default_rng(100 + seed)
+        T = rnd(r, M, M, cplx)
+        T[np.arange(M), np.arange(M)] = 0.1j if cplx else 0.1
+        Top = OPF[tr](np.tril(T) if uplo == 1 else np.triu(T))
+        # a right-hand side whose solution stays of order one
+        B = np.asfortranarray((Top.astype(wide) @ rnd(r, M, 21, cplx)).astype(T.dtype))
+        X = solve_batch(xk, T, B, uplo, tr, 0)
+        res = np.abs(Top.astype(wide) @ X.astype(wide) - B)
+        lim = (4 if cplx else 1) * (M + 8) * EPS * (np.abs(Top) @ np.abs(X) + np.abs(B))
+        assert (res <= lim).all(), (M, seed, float((res / lim).max()))
