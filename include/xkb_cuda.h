@@ -179,6 +179,11 @@ int xkb_ozaki_default_moduli(long K);
  * Waits for the device.  No counterpart in the reference. */
 int xkb_ozaki_counts(unsigned long long* out, int* last, int reset);
 
+/* The same for the S / C products that may take the exact INT8 form: out[0]
+ * products, out[1] those the device sent to the plain kernel; *last the latest
+ * one's moduli count (0: plain kernel, -1: none yet). */
+int xkb_exact_counts(unsigned long long* out, int* last, int reset);
+
 /* Per-call trace (off by default): when enabled, contractions record CUDA
  * events around their phases on their own stream; xkb_trace_take() waits for
  * the recorded events and returns up to `max` completed records, oldest

@@ -21,7 +21,9 @@ def mat(r, t, rows, cols):
     return np.asfortranarray(v.astype(DT[t][1]))
 
 
-def call(xk, t, opA, opB, A, B, C0, beta, uplo=0, herm=0, exact=True, pad=0):
+def call(xk, t, opA, opB, A, B, C0, beta, uplo=0, herm=0, exact=True, pad=0, fits=True,
+         count=None):
+    """fits: whether the device takes the exact form; count: its moduli."""
     import torch
     code, dt = DT[t]
 
@@ -46,14 +48,17 @@ def call(xk, t, opA, opB, A, B, C0, beta, uplo=0, herm=0, exact=True, pad=0):
     lib.xkb_tune_set(b"gemm_exact_min", 0.0)
     try:
         torch.cuda.synchronize()
-        with xk.contraction_trace() as tr:
-            assert lib.xkb_cuda_gemm(ctypes.byref(g), None) == 0
-            xk.sync()
+        xk.exact_counts(reset=True)
+        assert lib.xkb_cuda_gemm(ctypes.byref(g), None) == 0
+        xk.sync()
+        calls, plain, last = xk.exact_counts()
     finally:
         lib.xkb_tune_set(b"gemm_exact", 1.0)
         lib.xkb_tune_set(b"gemm_exact_min", 3.4e9)
     assert lib.xkb_cuda_take_device_error() == 0
-    assert ("ozaki_gemm" in tr.ops()) == exact
+    assert (calls, plain) == ((1, 0 if fits else 1) if exact else (0, 0))
+    if exact:
+        assert (last > 0) == fits and (count is None or last == count), last
     return np.asfortranarray(dC.cpu().numpy()[:, :M].T)
 
 
@@ -126,10 +131,65 @@ def test_operands_that_do_and_do_not_fit(xk, t, what):
     else:
         A = np.asfortranarray(np.round(A * 8))
         B = np.asfortranarray(np.round(B * 8))
-    got = call(xk, t, "N", "N", A, B, C0, 0.5)
+    got = call(xk, t, "N", "N", A, B, C0, 0.5, fits=what in ("zero", "ints"))
     plain = call(xk, t, "N", "N", A, B, C0, 0.5, exact=False)
     if what in ("spread", "inf", "nan", "ints"):
         assert np.array_equal(got, plain, equal_nan=True)
     else:
         assert np.allclose(got, plain, rtol=0, atol=1e-5)
         assert np.array_equal(got[5, :], plain[5, :]) and np.array_equal(got[:, 4], plain[:, 4])
+
+
+# budgets of the scaled operands (bits from a row's lowest set bit up to its
+# norm) of the fewest and the most moduli a product may take, and these counts:
+# floor((log2 P - 1) / 2) - 1 of the largest pairwise coprime numbers from 256
+# down; complex floor((log2 P - 2) / 2) of those whose prime factors are 1 mod 4
+BUDGET = {"s": ((30, 8), (57, 15)), "c": ((33, 9), (57, 16))}
+
+
+@pytest.mark.parametrize("t", "sc")
+@pytest.mark.parametrize("end", [0, 1])
+def test_moduli_count_at_the_ends_of_its_range(xk, t, end):
+    """One entry far below its row's norm asks for exactly the budget of the
+    fewest and of the most moduli, then for one bit more: that takes the next
+    count, and beyond the most the plain kernel."""
+    r = np.random.default_rng(21)
+    bits, count = BUDGET[t][end]
+    A = np.asfortranarray(r.integers(0, 2, (512, 512)).astype(DT[t][1]))
+    B = np.asfortranarray(r.integers(-1, 2, (512, 520)).astype(DT[t][1]))
+    A[0, :] = 0
+    A[0, 0], A[0, 2] = 1.5, 1  # norm 1.80: exponent 1
+    C0 = mat(r, t, 512, 520)
+    for more in (0, 1):
+        A[0, 1] = 2.0 ** (1 - bits - more)
+        fits = end == 0 or more == 0
+        got = call(xk, t, "N", "N", A, B, C0, 0.0, fits=fits,
+                   count=(count + more) if fits else 0)
+        wide = np.complex128 if t == "c" else np.float64
+        ref = (0.75 - 0.5j if t == "c" else 0.75) * (A.astype(wide) @ B.astype(wide))
+        # sums of at most 512 small integers: exact in 64 bits but for row 0
+        assert np.array_equal(got[1:], ref[1:].astype(DT[t][1]))
+        assert np.allclose(got[0], ref[0], rtol=2.0 ** -23, atol=0)
+
+
+@pytest.mark.parametrize("t", "sc")
+def test_results_far_below_the_norms_are_exact(xk, t):
+    """Rows of 2^-40 to 1 (columns too), and entries whose products lie up to
+    2^16 below the norms' product: every result is a small integer times a
+    power of two and must come out exactly."""
+    r = np.random.default_rng(22)
+
+    def ints(m, n):
+        v = r.integers(-4, 5, (m, n)).astype(np.float64)
+        return v + 1j * r.integers(-4, 5, (m, n)) if t == "c" else v
+
+    M, N, K = 600, 530, 700
+    k = 2.0 ** r.integers(-8, 9, K)
+    a = 2.0 ** -r.integers(0, 41, M)[:, None]
+    b = 2.0 ** -r.integers(0, 41, N)[None, :]
+    iA, iB = ints(M, K), ints(K, N)
+    A = np.asfortranarray((a * iA * k[None, :]).astype(DT[t][1]))
+    B = np.asfortranarray((b * iB / k[:, None]).astype(DT[t][1]))
+    ref = (0.75 - 0.5j if t == "c" else 0.75) * (a * (iA @ iB) * b)
+    got = call(xk, t, "N", "N", A, B, np.zeros((M, N), DT[t][1], order="F"), 0.0)
+    assert np.array_equal(got, ref.astype(DT[t][1]))

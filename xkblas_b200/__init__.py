@@ -125,8 +125,8 @@ def lib():
         _lib.xkblas_trace_export.argtypes = [ctypes.c_char_p]
         _lib.xkblas_trace_dropped.restype = ctypes.c_uint64
         _lib.xkb_trace_take.argtypes = [ctypes.POINTER(TraceRec), c_int]
-        _lib.xkb_ozaki_counts.argtypes = [ctypes.POINTER(ctypes.c_ulonglong),
-                                          ctypes.POINTER(c_int), c_int]
+        for f in (_lib.xkb_ozaki_counts, _lib.xkb_exact_counts):
+            f.argtypes = [ctypes.POINTER(ctypes.c_ulonglong), ctypes.POINTER(c_int), c_int]
     return _lib
 
 
@@ -195,6 +195,17 @@ def ozaki_counts(reset=False):
     if r != 0:
         raise XkblasError("xkb_ozaki_counts failed: %d" % r)
     return int(out[0]), int(out[1]), int(out[2]), int(last.value)
+
+
+def exact_counts(reset=False):
+    """The same for single-precision products that may take the exact INT8
+    form: (products, sent to the plain kernel, latest one's moduli count)."""
+    out = (ctypes.c_ulonglong * 2)()
+    last = ctypes.c_int(-1)
+    r = lib().xkb_exact_counts(out, ctypes.byref(last), 1 if reset else 0)
+    if r != 0:
+        raise XkblasError("xkb_exact_counts failed: %d" % r)
+    return int(out[0]), int(out[1]), int(last.value)
 
 
 class contraction_trace:

@@ -294,6 +294,9 @@ struct OzSel {
 // Counters over all contractions of the process (xkb_ozaki_counts).
 static __device__ unsigned long long g_oz_calls, g_oz_mod_sum, g_oz_fallbacks;
 static __device__ int g_oz_last = -1;
+// and over the single-precision products (xkb_exact_counts)
+static __device__ unsigned long long g_ex_calls, g_ex_plain;
+static __device__ int g_ex_last = -1;
 
 // Exponent of the lowest set bit of a float that is not 0.
 __device__ __forceinline__ int lsb_exp(float x) {
@@ -479,6 +482,9 @@ __global__ void k_oz_pick(const unsigned* rmax, OzSel* sel, const PickP q) {
     sel->H = h;
     sel->fallback = n == 0;
     sel->np = n;
+    atomicAdd(&g_ex_calls, 1ull);
+    if (n == 0) atomicAdd(&g_ex_plain, 1ull);
+    g_ex_last = n;
     return;
   }
   if (n <= 0) {
@@ -1967,6 +1973,22 @@ extern "C" int xkb_ozaki_counts(unsigned long long* out, int* last, int reset) {
         cudaMemcpyToSymbol(g_oz_last, &none, sizeof none) != cudaSuccess)
       return XKB_ECUDA;
   }
+  return XKB_OK;
+}
+
+extern "C" int xkb_exact_counts(unsigned long long* out, int* last, int reset) {
+  if (!out) return XKB_EINVAL;
+  if (cudaDeviceSynchronize() != cudaSuccess ||
+      cudaMemcpyFromSymbol(&out[0], g_ex_calls, sizeof(out[0])) != cudaSuccess ||
+      cudaMemcpyFromSymbol(&out[1], g_ex_plain, sizeof(out[1])) != cudaSuccess ||
+      (last && cudaMemcpyFromSymbol(last, g_ex_last, sizeof(int)) != cudaSuccess))
+    return XKB_ECUDA;
+  const unsigned long long z = 0;
+  const int none = -1;
+  if (reset && (cudaMemcpyToSymbol(g_ex_calls, &z, sizeof z) != cudaSuccess ||
+                cudaMemcpyToSymbol(g_ex_plain, &z, sizeof z) != cudaSuccess ||
+                cudaMemcpyToSymbol(g_ex_last, &none, sizeof none) != cudaSuccess))
+    return XKB_ECUDA;
   return XKB_OK;
 }
 
