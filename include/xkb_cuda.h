@@ -257,9 +257,10 @@ int xkb_cuda_batch_release(void);
 /* Tuning table: choices measured on the device by the autotuner
  * (python -m xkblas_b200.autotune --out FILE; the runtime loads
  * XKBLAS_TUNE_FILE at init).  Keys (built-in default):
- *   gemm_big_min_tiles      real whole-matrix GEMM uses 64 x 64 tiles when C has
+ *   gemm_tile64_min_blocks  real whole-matrix GEMM uses 64 x 64 tiles when C has
  *                           at least this many 128 x 128 blocks, else 32 x 32
- *                           ones (unset: chosen by a model of the time)
+ *                           ones (unset: chosen by a model of the time; not
+ *                           written by the autotuner)
  *   gemm_exact              large S / C products by exact INT8 arithmetic where
  *                           the operands allow it (1); gemm_exact_min: from
  *                           this M N K on (3.4e9; C a quarter of it)

@@ -18,6 +18,8 @@ def test_quick_autotune_writes_a_loadable_table(xk, tmp_path):
     for k, (v, _) in table.items():
         assert lib.xkb_tune_get(k.encode(), -1.0) == float(v), k
     assert lib.xkb_tune_get(b"batch_schedule", -1) in (0.0, 1.0)
+    # the plain product's tiles stay the time model's
+    assert not [k for k in table if k.startswith("gemm")]
     for k, (v, note) in table.items():
         if k.startswith("ozaki_moduli_k<="):
             assert 10 <= v <= 16, (k, v)

@@ -66,7 +66,7 @@ def run(xk, t, opA, opB, M, N, K, beta, uplo=0, pad=0, off=0, seed=0):
 @pytest.mark.parametrize("tile", [0.0, 1e9])  # 64 x 64 always, 32 x 32 always (real types)
 def test_tile_edges(xk, t, tile):
     lib = xk.lib()
-    lib.xkb_tune_set(b"gemm_big_min_tiles", tile)
+    lib.xkb_tune_set(b"gemm_tile64_min_blocks", tile)
     try:
         ops = "NT" if t in "sd" else "NTC"
         seed = 0
@@ -79,7 +79,7 @@ def test_tile_edges(xk, t, tile):
                     seed += 1
                     run(xk, t, opA, opB, M, N, K, 0.5 * (seed % 2), pad=pad, off=off, seed=seed)
     finally:
-        lib.xkb_tune_set(b"gemm_big_min_tiles", -1.0)
+        lib.xkb_tune_set(b"gemm_tile64_min_blocks", -1.0)
 
 
 @pytest.mark.parametrize("t", "sdcz")

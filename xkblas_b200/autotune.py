@@ -6,10 +6,6 @@ loads at init (XKBLAS_TUNE_FILE):
     XKBLAS_TUNE_FILE=xkblas_tune.txt ./app
 
 Choices (keys of the table, see include/xkb_cuda.h):
-  gemm_big_min_tiles      whole-matrix real GEMM: 64 x 64 tiles from this many
-                          128 x 128 blocks of C on, else 32 x 32 (timed: both
-                          tile shapes on square DGEMMs; without the key the
-                          library chooses by a model of the time);
   ozaki_min_dim           tensor-op mode: Ozaki from this size on (timed:
                           plain DMMA vs Ozaki on square DGEMMs);
   ozaki_moduli_k<=<K>     moduli count per inner-size band (measured error:
@@ -143,29 +139,6 @@ class Tuner:
         return best
 
     # -- choices ---------------------------------------------------------------
-    def gemm_tiles(self):
-        lib, sizes = self.lib, ([768, 1536, 3072] if self.quick else [512, 768, 1024, 1536, 2048, 3072, 4096])
-        big_wins = []
-        for n in sizes:
-            A, B, C = self.rnd(n, n), self.rnd(n, n), self.rnd(n, n)
-            a = self.args(A, B, C, n, n, n)
-            tm = {}
-            for shape, v in (("big", 0.0), ("small", 1e12)):
-                lib.xkb_tune_set(b"gemm_big_min_tiles", v)
-                tm[shape] = self.time(lambda: lib.xkb_cuda_gemm(ctypes.byref(a), self.sp), 5)
-            tiles = math.ceil(n / 128) ** 2
-            big_wins.append((tiles, tm["big"] <= tm["small"]))
-            self.log("gemm %5d: tiles %5d big %.3f ms small %.3f ms" % (n, tiles, tm["big"], tm["small"]))
-        # smallest tile count from which the big tile wins at every larger size
-        thr = None
-        for i, (tiles, win) in enumerate(big_wins):
-            if all(w for _, w in big_wins[i:]):
-                thr = tiles
-                break
-        lib.xkb_tune_set(b"gemm_big_min_tiles", float(thr if thr is not None else 1 << 30))
-        self.table["gemm_big_min_tiles"] = (thr if thr is not None else 1 << 30,
-                                            "tiles: " + ", ".join("%d%s" % (t, "B" if w else "s") for t, w in big_wins))
-
     def ozaki_crossover(self):
         lib = self.lib
         sizes = [1024, 2048, 4096] if self.quick else [512, 768, 1024, 1536, 2048, 3072, 4096]
@@ -295,7 +268,6 @@ class Tuner:
 
     def run(self):
         self.lib.xkb_tune_clear()
-        self.gemm_tiles()
         self.ozaki_crossover()
         self.moduli()
         self.ozaki_kernel()

@@ -575,9 +575,11 @@ static TilePlan plan_tiles(const xkb_gemm_args* a) {
     return a->uplo == XKB_FULL ? tm * tn : (tm * tn + std::max(tm, tn)) / 2;
   };
   // tuning table: 64 x 64 tiles from this many 128 x 128 blocks of C on
-  // (XKBLAS_GEMM_TILE=big|small: always / never); the split stays the model's
+  // (XKBLAS_GEMM_TILE=big|small: always / never), for sweeps and tests; the
+  // split stays the model's.  Saved tables hold no such line: one threshold
+  // made 4096^2 x 128 lower 108 us (94), 1000 x 900 x 3000 203 (189)
   static const char* force = getenv("XKBLAS_GEMM_TILE");
-  const double big = force ? (force[0] == 'b' ? 0.0 : 1e18) : tune("gemm_big_min_tiles", -1.0);
+  const double big = force ? (force[0] == 'b' ? 0.0 : 1e18) : tune("gemm_tile64_min_blocks", -1.0);
   const bool fixed = !CPLX && big >= 0.0;
   const bool want_small =
       (double)((a->M + 127) / 128) * (double)((a->N + 127) / 128) < big;
