@@ -525,11 +525,11 @@ def test_trsm_pair_leaves(xk, dt):
     (np.complex128, 320, 256, 3000, C_, N_),
     (np.float64, 1000, 900, 3000, N_, N_),
 ])
-def test_gemm_stream_k(xk, case):
-    """Stream-K (tuning key gemm_sk_fill = 1: taken whenever split-K would
-    be) and split-K (gemm_streamk = 0) on the same operands: both meet the
-    reference bound, and stream-K's fixed order of the pieces makes repeated
-    calls bit-identical."""
+def test_gemm_split_k(xk, case):
+    """Split-K (two launches: the slices and their reduction) and one k range
+    per tile (gemm_splitk = 0: one launch) on the same operands: both meet the
+    reference bound, and the fixed order of the slices makes repeated calls
+    bit-identical."""
     import ctypes
     import torch
     from xkblas_b200 import GemmArgs
@@ -545,9 +545,8 @@ def test_gemm_stream_k(xk, case):
     R = O.gemm(ta, tb, al, A, B, be, C0.copy(order="F"), nb=256)
     outs = {}
     try:
-        for mode, (sk, fill) in (("sk", (1.0, 1.0)), ("sk2", (1.0, 1.0)), ("split", (0.0, 0.8))):
-            lib.xkb_tune_set(b"gemm_streamk", sk)
-            lib.xkb_tune_set(b"gemm_sk_fill", fill)
+        for mode, split in (("split", 1.0), ("again", 1.0), ("whole", 0.0)):
+            lib.xkb_tune_set(b"gemm_splitk", split)
             dC = dev(C0)
             g = GemmArgs(3 if cplx else 1, ta - N_, tb - N_, M, N, K, dA.data_ptr(), A.shape[0],
                          dB.data_ptr(), B.shape[0], dC.data_ptr(), M)
@@ -556,13 +555,12 @@ def test_gemm_stream_k(xk, case):
             torch.cuda.synchronize()
             k0 = xk.kernel_count()
             assert lib.xkb_cuda_gemm(ctypes.byref(g), None) == 0
-            assert xk.kernel_count() - k0 == 2  # the pieces and their reduction
+            assert xk.kernel_count() - k0 == (2 if split else 1)
             xk.sync()
             outs[mode] = np.asfortranarray(dC.cpu().numpy().T)
     finally:
-        lib.xkb_tune_set(b"gemm_streamk", 1.0)
-        lib.xkb_tune_set(b"gemm_sk_fill", 0.8)
+        lib.xkb_tune_set(b"gemm_splitk", 1.0)
     assert lib.xkb_cuda_take_device_error() == 0
-    assert np.array_equal(outs["sk"], outs["sk2"])
-    for mode in ("sk", "split"):
+    assert np.array_equal(outs["split"], outs["again"])
+    for mode in ("split", "whole"):
         assert checks.gemm_ratio(outs[mode], R, A, B, C0, al, be, K) <= 3.0, mode
