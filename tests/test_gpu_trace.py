@@ -19,10 +19,10 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 N_, LEFT, LO, NONUNIT = 111, 141, 122, 131
-KERNELS = {"k_gemm_dmma", "k_repack", "k_scale", "k_sched", "k_sched(graph)", "k_trsm_block",
-           "k_oz_norm+k_oz_shift", "k_oz_residues", "k_oz_gemm", "k_oz_gemm2", "k_oz_crt",
-           "k_oz_crt_store", "k_tri_fill+k_copy2d", "k_sym_fill", "k_potrf_block",
-           "k_getrf_block"}
+KERNELS = {"k_gemm_dmma", "k_gemm_dmma+k_gemm_splitk", "k_repack", "k_scale", "k_sched",
+           "k_sched(graph)", "k_trsm_block", "k_oz_norm+k_oz_stat", "k_oz_pick", "k_oz_residues",
+           "k_oz_gemm", "k_oz_gemm2", "k_oz_crt", "k_oz_beta", "k_tri_fill", "k_sym_fill",
+           "k_potrf_block", "k_getrf_block"}
 
 
 def _rows(path):

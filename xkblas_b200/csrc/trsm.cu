@@ -1039,7 +1039,7 @@ extern "C" int xkb_cuda_trmm(int dtype, int side, int uplo, int trans, int diag,
   const dim3 g1 = copy_grid(na, na);
   const int lower = uplo == XKB_LOWER, unit = diag != 0;
   const CopyArray bc{B, Bc, ldb, ldc, M, N, XKB_FULL};
-  const long long tv = evlog_kern_begin(st, "k_tri_fill+k_copy2d");
+  const long long tv = evlog_kern_begin(st, "k_tri_fill");
   switch (dtype) {
     case XKB_S: launch_pdl(k_tri_fill<float>, g1, dim3(256), 0, st, (int)na, (const float*)A, lda, lower, unit, (float*)T, ldt); break;
     case XKB_D: launch_pdl(k_tri_fill<double>, g1, dim3(256), 0, st, (int)na, (const double*)A, lda, lower, unit, (double*)T, ldt); break;

@@ -93,9 +93,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
 
 // ---- programmatic dependent launch --------------------------------------------
 // Kernels launched with launch_pdl start while the previous kernel of their
-// stream drains: they call pdl_wait before they touch global memory (every
-// thread of every block, before any early return, so that a grid never ends
-// before its predecessor has) and pdl_launch to let their own successor start.
+// stream drains: they call pdl_wait before they touch global memory and
+// pdl_launch to let their own successor start.  A grid must not end before its
+// predecessor has: every thread of at least one block calls pdl_wait on every
+// path (blocks of a masked GEMM whose tile lies outside the triangle leave
+// without it, but for block 0).
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -1,6 +1,6 @@
 """Small, self-contained cases for profiling single kernels with ncu:
 
-    python -m xkblas_b200.profcases dmma|update256|ozaki|ozaki2|ozaki8192|splitk|streamk|repack|trsm|potrf|potrf8192|getrf|getrf8192|batch|copy
+    python -m xkblas_b200.profcases dmma|update256|ozaki|ozaki2|ozaki8192|sgemm|splitk|repack|trsm|potrf|potrf8192|getrf|getrf8192|batch|copy
 
 dmma    DGEMM NN 4096^3 through xkb_cuda_gemm (k_gemm_dmma), two calls
 update256  the Cholesky's first trailing update at 8192 with 256-wide
@@ -10,10 +10,9 @@ ozaki2  the same with the CTA-pair INT8 kernel (tuning key oz_2cta = 1, k_oz_gem
 ozaki8192  DGEMM NN 8192^3, xkb_cuda_ozaki_gemm with the count chosen on the
         device (nmod = 0: 15 moduli on these inputs), two calls: the DRAM
         traffic of k_oz_gemm at a size whose residue planes exceed L2
+sgemm   SGEMM NN 4096^3 through xkb_cuda_gemm: the exact INT8 form, two calls
 splitk  DGEMM NN 512 x 512 x 4096 through xkb_cuda_gemm: 256 output tiles of
         32 x 32, split-K (k_gemm_dmma slices + k_gemm_splitk)
-streamk DGEMM TN 640 x 1280 x 2048 through xkb_cuda_gemm: few tiles and a
-        long K, tile and split by the time model, two calls
 repack  the DGEMM with lda = ldb = 4097 (k_repack, then k_gemm_dmma)
 trsm    DTRSM L/L/N/N 4096 x 4096, diagonally dominant (k_trsm_block, GEMMs)
 potrf   DPOTRF lower 4096 (k_potrf_block, k_trsm_block, GEMMs)
@@ -23,7 +22,7 @@ getrf   DGETRF without pivoting 4096, diagonally dominant (k_getrf_block,
         k_trsm_block, GEMMs)
 getrf8192  the same at 8192
 copy    beta scaling (k_scale, 8192^2) and the TRMM / SYMM materialisations
-        (k_tri_fill, k_copy2d, k_sym_fill, 4096^2)
+        (k_tri_fill, k_repack, k_sym_fill, 4096^2)
 batch   150 mixed calls (70% DGEMM, 20% DTRSM, 10% ZGEMM; M, N, K
         log-uniform in [64, 2048]) as one xkb_cuda_batch launch (k_sched)
 
@@ -63,14 +62,6 @@ def main(case):
         ga.alpha[0], ga.beta[0], ga.uplo = -1.0, 1.0, 1
         for _ in range(2):
             assert lib.xkb_cuda_gemm(ctypes.byref(ga), sp) == 0
-    elif case == "streamk":
-        m, n, k = 640, 1280, 2048
-        A, B, C = rnd(k, m), rnd(k, n), rnd(m, n)  # op(A) = A^T: A stored k x m
-        keep += [A, B, C]
-        ga = _GemmArgs(1, 1, 0, m, n, k, A.data_ptr(), k, B.data_ptr(), k, C.data_ptr(), m)
-        ga.alpha[0] = ga.beta[0] = 1.0
-        for _ in range(2):
-            assert lib.xkb_cuda_gemm(ctypes.byref(ga), sp) == 0
     elif case in ("ozaki8192", "splitk"):
         m, n, k = (8192, 8192, 8192) if case == "ozaki8192" else (512, 512, 4096)
         A, B, C = rnd(m, k), rnd(k, n), rnd(m, n)
@@ -81,6 +72,14 @@ def main(case):
             rc = (lib.xkb_cuda_ozaki_gemm(ctypes.byref(ga), 0, sp) if case == "ozaki8192"
                   else lib.xkb_cuda_gemm(ctypes.byref(ga), sp))
             assert rc == 0, rc
+    elif case == "sgemm":
+        n = 4096
+        A, B, C = (rnd(n, n).float() for _ in range(3))
+        keep += [A, B, C]
+        ga = _GemmArgs(0, 0, 0, n, n, n, A.data_ptr(), n, B.data_ptr(), n, C.data_ptr(), n)
+        ga.alpha[0] = 1.0
+        for _ in range(2):
+            assert lib.xkb_cuda_gemm(ctypes.byref(ga), sp) == 0
     elif case in ("dmma", "ozaki", "ozaki2", "repack"):
         n = 4096
         ld = n + 1 if case == "repack" else n
@@ -156,7 +155,7 @@ def main(case):
     elif case == "copy":
         # HBM-bound helpers: beta scaling of C (k_scale, 8192^2), the
         # triangle and symmetric materialisations of TRMM / SYMM
-        # (k_tri_fill, k_copy2d, k_sym_fill, 4096^2)
+        # (k_tri_fill, k_repack, k_sym_fill, 4096^2)
         n = 8192
         C = rnd(n, n)
         keep += [C]
