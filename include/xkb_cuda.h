@@ -74,7 +74,8 @@ typedef struct xkb_gemm_args {
  * tensor cores (float storage computed in double and rounded once; large S
  * and C products whose operands fit are computed exactly on the INT8 tensor
  * cores and rounded to double, then to float: the device decides, the plain
- * kernel runs otherwise). */
+ * kernel runs otherwise; their residue planes take up to 16 GiB of pool
+ * memory).  XKB_ENOMEM: C is as it was. */
 int xkb_cuda_gemm(const xkb_gemm_args* a, void* stream);
 
 /* Triangular solve, all side/uplo/trans/diag cases:

@@ -2140,10 +2140,13 @@ namespace xkb {
 // leave the INT8 tensor cores idle.  Whether the operands allow it is decided
 // on the device (k_oz_pick), else the plain kernel runs within the same call.
 // XKB_ERANGE: not taken for this shape, XKB_ENOMEM: no scratch, either before
-// anything that writes C; the caller then runs the plain kernel.  Taken from M N K = 3.4e9 on (C: a quarter of
-// it).  Measured (B200, us, plain -> exact): S 1024^3 76 -> 108, 1500^3 214 ->
-// 184, 2048^3 527 -> 270, 4096^3 3978 -> 1042 (error against 64 bits 2.53e-8,
-// the final rounding, on both); C 1024^3 258 -> 209, 2048^3 1976 -> 489.
+// anything that writes C; the caller then runs the plain kernel.  Taken from
+// M N K = 3.4e9 on (C: a quarter of it).  Measured (B200, us, plain -> exact):
+// S 1024^3 76 -> 108, 1500^3 214 -> 184, 2048^3 527 -> 270, 4096^3 3978 -> 1042
+// (error against 64 bits 2.53e-8, the final rounding, on both); C 1024^3 258 ->
+// 209, 2048^3 1976 -> 489.  Operands that do not fit pay the norm passes, the
+// allocations and the empty launches: S 1800^3 376 -> 472, 2048^3 529 -> 593,
+// 4096^3 3996 -> 4108; C 1000^3 258 -> 317, 2048^3 1980 -> 2055.
 int gemm_exact(const xkb_gemm_args* a, cudaStream_t st) {
   const bool cplx = a->dtype == XKB_C;
   const double mn = std::min(a->M, a->N);
