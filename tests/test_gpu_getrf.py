@@ -123,5 +123,5 @@ def test_getrf_nopiv_blocked_and_recursive_forms(xk, dt):
     finally:
         lib.xkb_tune_set(b"getrf_blocked", 3.0)
         lib.xkb_tune_set(b"getrf_nb", 512.0)
-        lib.xkb_tune_set(b"getrf_shrink", 12.0)
+        lib.xkb_tune_set(b"getrf_shrink", 16.0)
         lib.xkb_tune_set(b"getrf_oz_leaf", 4096.0)

@@ -152,4 +152,4 @@ def test_potrf_blocked_and_recursive_forms(xk, dt, uplo):
     finally:
         lib.xkb_tune_set(b"potrf_blocked", 3.0)
         lib.xkb_tune_set(b"potrf_nb", 512.0)
-        lib.xkb_tune_set(b"potrf_shrink", 12.0)
+        lib.xkb_tune_set(b"potrf_shrink", 8.0)
