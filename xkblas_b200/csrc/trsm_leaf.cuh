@@ -12,7 +12,8 @@
 // still to solve by DMMA, as in k_trsm_block (trsm.cu).  What bounds it is
 // latency: 8 steps of two dependent DMMAs and their shared-memory trips.  The
 // substitution it replaces (a shuffle, a product and 16 dependent updates per
-// unknown) took 40 to 60 us per block, most of a chain's time.
+// unknown) took 40 to 60 us per block, most of a chain's time; it stays for
+// ill-conditioned sub-blocks and for values that are not finite.
 #pragma once
 #include "dmma_common.cuh"
 
@@ -196,130 +197,138 @@ __device__ __forceinline__ void leaf_solve(const typename St<T>::S* A, long lda,
     if (kk == 0) cond[m] = sv * st;
   }
   leaf_sync<NT>();
+  // sub-blocks applied by their inverse (bit m)
+  const unsigned well =
+      __ballot_sync(0xffffffffu, lane < kLeafRows / 8 && cond[lane & 7] <= kLeafCond);
   // ---- this warp's right-hand sides, nothing shared with the other warps ----
   double* xr = Xr + warp * Sh::CW * LD;
   double* xi = Xi + warp * Sh::CW * LD;
 #pragma unroll 1
   for (int c0 = warp * Sh::CW; c0 < nrhs; c0 += Sh::COLS) {
+    // X by the inverses of the well-conditioned sub-blocks; where a value is not
+    // finite, which shows in that unknown's Y (an inverse's diagonal is not
+    // zero), again from B by substitution throughout
+    unsigned inv = well;
 #pragma unroll 1
-    for (int q0 = 0; q0 < Sh::CW; q0 += 4) {
-      double br[8], bi[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int i = lane + 32 * (k & 1), c = c0 + q0 + (k >> 1);
-        br[k] = bi[k] = 0.0;
-        if (i < n && c < nrhs) {
-          const size_t idx = leaf_at(i, c, ldb, false);
-          br[k] = (double)__ldcg(B + W * idx);
-          if (CP) bi[k] = (double)__ldcg(B + W * idx + W - 1);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int o = (q0 + (k >> 1)) * LD + lane + 32 * (k & 1);
-        xr[o] = ar * br[k] - ai * bi[k];
-        if (CP) xi[o] = ar * bi[k] + ai * br[k];
-      }
-    }
-    __syncwarp();
-    const int k0 = 2 * t, k1 = k0 + 1;
+    for (;;) {
+      int top = 0;  // largest exponent field of the Y (as integers: off the FP64 pipe)
 #pragma unroll 1
-    for (int s = 0; s < nsub; ++s) {
-      const int m = LOWER ? s : nsub - 1 - s, b = 8 * m;
-      // Y^T = X_s^T inv(T_ss)^T (k indices 2t, 2t + 1 on both sides)
-      double yr[4] = {0.0, 0.0, 0.0, 0.0}, yi[4] = {0.0, 0.0, 0.0, 0.0};
-      {
-        constexpr bool hi = Sh::CW > 8;  // right-hand sides g + 8 exist
-        const double* v = Vr + m * 64 + g * 8;
-        const double* x = xr + g * LD + b;
-        const double a_r[4] = {x[k0], hi ? x[8 * LD + k0] : 0.0, x[k1], hi ? x[8 * LD + k1] : 0.0};
-        const double b_r[2] = {v[k0], v[k1]};
-        if constexpr (CP) {
-          const double* w = Vi + m * 64 + g * 8;
-          const double* z = xi + g * LD + b;
-          const double a_i[4] = {z[k0], 0.0, z[k1], 0.0};
-          const double n_i[4] = {-a_i[0], 0.0, -a_i[2], 0.0};
-          const double b_i[2] = {w[k0], w[k1]};
-          dmma_k8(yr, a_r, b_r);
-          dmma_k8(yr, n_i, b_i);
-          dmma_k8(yi, a_r, b_i);
-          dmma_k8(yi, a_i, b_r);
-        } else {
-          dmma_k8(yr, a_r, b_r);
-        }
-      }
-      // by substitution instead: far from well conditioned, or not finite,
-      // which shows in this Y (the inverse's diagonal is not zero); every lane
-      // has read X_s (the vote)
-      bool fin = cond[m] <= kLeafCond;
+      for (int q0 = 0; q0 < Sh::CW; q0 += 4) {
+        double br[8], bi[8];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) fin = fin && isfinite(yr[v]) && (!CP || isfinite(yi[v]));
-      if (__all_sync(0xffffffffu, fin)) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int c = g + ((v >> 1) << 3);
-          if (c < Sh::CW) {
-            xr[c * LD + b + k0 + (v & 1)] = yr[v];
-            if (CP) xi[c * LD + b + k0 + (v & 1)] = yi[v];
+        for (int k = 0; k < 8; ++k) {
+          const int i = lane + 32 * (k & 1), c = c0 + q0 + (k >> 1);
+          br[k] = bi[k] = 0.0;
+          if (i < n && c < nrhs) {
+            const size_t idx = leaf_at(i, c, ldb, false);
+            br[k] = (double)__ldcg(B + W * idx);
+            if (CP) bi[k] = (double)__ldcg(B + W * idx + W - 1);
           }
         }
-      } else {
-        leaf_substitute<T, LOWER>(Tr, Ti, Vr + m * 64, Vi + m * 64, b, xr, xi);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int c = g + ((v >> 1) << 3);
-          yr[v] = c < Sh::CW ? xr[c * LD + b + k0 + (v & 1)] : 0.0;
-          if (CP) yi[v] = c < Sh::CW ? xi[c * LD + b + k0 + (v & 1)] : 0.0;
-        }
-      }
-      // rows still to solve -= T(rows, b .. b+7) Y
-      const int u0 = LOWER ? b + 8 : 0, u1 = LOWER ? 8 * nsub : b;
-#pragma unroll 1
-      for (int m0 = u0; m0 < u1; m0 += 16) {
-        // rows past u1 (a last half tile) are read in range and not stored
-        const int ra = m0 + g, rb = min(m0 + g + 8, kLeafRows - 1);
-        const double* t0 = Tr + (b + k0) * LD;
-        const double* t1 = t0 + LD;
-        const double a_r[4] = {-t0[ra], -t0[rb], -t1[ra], -t1[rb]};
-        double a_i[4] = {0.0, 0.0, 0.0, 0.0}, n_i[4] = {0.0, 0.0, 0.0, 0.0};
-        if constexpr (CP) {
-          const double* s0 = Ti + (b + k0) * LD;
-          const double* s1 = s0 + LD;
-          a_i[0] = -s0[ra], a_i[1] = -s0[rb], a_i[2] = -s1[ra], a_i[3] = -s1[rb];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) n_i[v] = -a_i[v];
-        }
-#pragma unroll
-        for (int n0 = 0; n0 < Sh::CW; n0 += 8) {
-          const double b_r[2] = {n0 ? yr[2] : yr[0], n0 ? yr[3] : yr[1]};
-          double cr[4], ci[4];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int o = (n0 + 2 * t + (v & 1)) * LD + (v >> 1 ? rb : ra);
-            cr[v] = xr[o];
-            ci[v] = CP ? xi[o] : 0.0;
-          }
-          if constexpr (CP) {
-            const double b_i[2] = {yi[0], yi[1]};
-            dmma_k8(cr, a_r, b_r);
-            dmma_k8(cr, n_i, b_i);
-            dmma_k8(ci, a_r, b_i);
-            dmma_k8(ci, a_i, b_r);
-          } else {
-            dmma_k8(cr, a_r, b_r);
-          }
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int row = m0 + g + ((v >> 1) << 3);
-            const int o = (n0 + 2 * t + (v & 1)) * LD + row;
-            if (row < u1) {
-              xr[o] = cr[v];
-              if (CP) xi[o] = ci[v];
-            }
-          }
+        for (int k = 0; k < 8; ++k) {
+          const int o = (q0 + (k >> 1)) * LD + lane + 32 * (k & 1);
+          xr[o] = ar * br[k] - ai * bi[k];
+          if (CP) xi[o] = ar * bi[k] + ai * br[k];
         }
       }
       __syncwarp();
+      const int k0 = 2 * t, k1 = k0 + 1;
+#pragma unroll 1
+      for (int s = 0; s < nsub; ++s) {
+        const int m = LOWER ? s : nsub - 1 - s, b = 8 * m;
+        double yr[4] = {0.0, 0.0, 0.0, 0.0}, yi[4] = {0.0, 0.0, 0.0, 0.0};
+        if (inv >> m & 1u) {
+          // Y^T = X_s^T inv(T_ss)^T (k indices 2t, 2t + 1 on both sides)
+          constexpr bool hi = Sh::CW > 8;  // right-hand sides g + 8 exist
+          const double* v = Vr + m * 64 + g * 8;
+          const double* x = xr + g * LD + b;
+          const double a_r[4] = {x[k0], hi ? x[8 * LD + k0] : 0.0, x[k1], hi ? x[8 * LD + k1] : 0.0};
+          const double b_r[2] = {v[k0], v[k1]};
+          if constexpr (CP) {
+            const double* w = Vi + m * 64 + g * 8;
+            const double* z = xi + g * LD + b;
+            const double a_i[4] = {z[k0], 0.0, z[k1], 0.0};
+            const double n_i[4] = {-a_i[0], 0.0, -a_i[2], 0.0};
+            const double b_i[2] = {w[k0], w[k1]};
+            dmma_k8(yr, a_r, b_r);
+            dmma_k8(yr, n_i, b_i);
+            dmma_k8(yi, a_r, b_i);
+            dmma_k8(yi, a_i, b_r);
+          } else {
+            dmma_k8(yr, a_r, b_r);
+          }
+          __syncwarp();  // every lane has read X_s
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int c = g + ((v >> 1) << 3);
+            if (c < Sh::CW) {
+              xr[c * LD + b + k0 + (v & 1)] = yr[v];
+              if (CP) xi[c * LD + b + k0 + (v & 1)] = yi[v];
+            }
+            top = max(top, __double2hiint(yr[v]) & 0x7fffffff);
+            if (CP) top = max(top, __double2hiint(yi[v]) & 0x7fffffff);
+          }
+        } else {
+          leaf_substitute<T, LOWER>(Tr, Ti, Vr + m * 64, Vi + m * 64, b, xr, xi);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int c = g + ((v >> 1) << 3);
+            yr[v] = c < Sh::CW ? xr[c * LD + b + k0 + (v & 1)] : 0.0;
+            if (CP) yi[v] = c < Sh::CW ? xi[c * LD + b + k0 + (v & 1)] : 0.0;
+          }
+        }
+        // rows still to solve -= T(rows, b .. b+7) Y
+        const int u0 = LOWER ? b + 8 : 0, u1 = LOWER ? 8 * nsub : b;
+#pragma unroll 1
+        for (int m0 = u0; m0 < u1; m0 += 16) {
+          // rows past u1 (a last half tile) are read in range and not stored
+          const int ra = m0 + g, rb = min(m0 + g + 8, kLeafRows - 1);
+          const double* t0 = Tr + (b + k0) * LD;
+          const double* t1 = t0 + LD;
+          const double a_r[4] = {-t0[ra], -t0[rb], -t1[ra], -t1[rb]};
+          double a_i[4] = {0.0, 0.0, 0.0, 0.0}, n_i[4] = {0.0, 0.0, 0.0, 0.0};
+          if constexpr (CP) {
+            const double* s0 = Ti + (b + k0) * LD;
+            const double* s1 = s0 + LD;
+            a_i[0] = -s0[ra], a_i[1] = -s0[rb], a_i[2] = -s1[ra], a_i[3] = -s1[rb];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) n_i[v] = -a_i[v];
+          }
+#pragma unroll
+          for (int n0 = 0; n0 < Sh::CW; n0 += 8) {
+            const double b_r[2] = {n0 ? yr[2] : yr[0], n0 ? yr[3] : yr[1]};
+            double cr[4], ci[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int o = (n0 + 2 * t + (v & 1)) * LD + (v >> 1 ? rb : ra);
+              cr[v] = xr[o];
+              ci[v] = CP ? xi[o] : 0.0;
+            }
+            if constexpr (CP) {
+              const double b_i[2] = {yi[0], yi[1]};
+              dmma_k8(cr, a_r, b_r);
+              dmma_k8(cr, n_i, b_i);
+              dmma_k8(ci, a_r, b_i);
+              dmma_k8(ci, a_i, b_r);
+            } else {
+              dmma_k8(cr, a_r, b_r);
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int row = m0 + g + ((v >> 1) << 3);
+              const int o = (n0 + 2 * t + (v & 1)) * LD + row;
+              if (row < u1) {
+                xr[o] = cr[v];
+                if (CP) xi[o] = ci[v];
+              }
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (inv == 0 || __all_sync(0xffffffffu, top < 0x7ff00000)) break;
+      inv = 0;
     }
 #pragma unroll 4
     for (int q = 0; q < 2 * Sh::CW; ++q) {
